@@ -5,9 +5,11 @@
 #include <cuda.h>
 #include <curand_kernel.h>
 
+#include <algorithm>
 #include <cmath>
 #include <cstring>
 #include <mutex>
+#include <type_traits>
 #include <vector>
 
 #include "runtime.cuh"
@@ -213,14 +215,38 @@ __global__ void k_update_noise(float *rr, float *raw, const float *__restrict__ 
 }
 
 // ------------------------------------------------------------ g(r)
-// get_gder_dev (get_gder.cu:69-127) as an exact integer histogram.  Each
-// thread owns one particle of `ra`; the partner set is staged through shared
-// memory in tiles; bins are added per warp with one shared atomic per
-// distinct bin (__match_any_sync) into a block histogram that is flushed to
-// 64-bit global counters.  SAME: unordered pairs j > i, each counted in both
-// directions; the reverse distance is recomputed whenever the minimum-image
-// rounding can differ between directions (some |d/L| >= 1/4).
-constexpr int kGderTile = 1024;
+// get_gder_dev (get_gder.cu:69-127) as an exact integer histogram over all
+// pairs.  A thread owns one particle of `ra` (256 a block); the partners
+// [j0, j1) of the block are staged in shared memory and read as broadcasts,
+// two per packed operation.  SAME: unordered pairs j > i, each counted in
+// both directions.
+//
+// Bound: issue slots (no DRAM traffic to speak of).  What keeps a pair cheap:
+//  - the minimum image is taken as fma(rint(d / L), -L, d).  When every
+//    component of the result lies within 0.4899 L of zero, d / L is within
+//    0.49 of an integer k in {-1, 0, 1}, the reference's floor equals k and
+//    L k is exact, so the rounded difference is the reference's, and that of
+//    the reverse pair is its negation.  Pairs beyond that (they matter only
+//    when the range reaches 0.489 L) and tiles with a coordinate outside
+//    [-0.2 L, 1.2 L] take the reference's arithmetic in both directions
+//    (gder_pair_exact).
+//  - the bin floor(sqrt(d2) / bin_size) comes, without a branch, from an
+//    estimate q (fused d2, rsqrtf) whose error against the reference's separately rounded
+//    operations is below eps = 1.5e-6 (nbins + 1): relative 2^-22 for rsqrtf,
+//    2^-24 for each other rounding and for half the difference of the two
+//    d2, 6e-7 in all.  Only a q closer than eps to an integer, the range
+//    among them (it is bin edge nbins), needs the reference's d2, square root
+//    and divide.
+//  - a pair out of range adds to a spare word of its lane instead of
+//    branching, and bins are added with plain shared atomics into a histogram copy per warp
+//    (fewer copies when they would pass 32 KB).
+// Blocks are cut over the partners until the grid has several per SM.
+// Measured at 4095 + 4099 particles, 200 bins to L / 2: 25 us for equal
+// species and 35 us for mixed ones, 43 thread instructions a pair, 46-59% of
+// issue slots (3.49 and 1.74 ms with 16 to 128 blocks of 8192 partners, a
+// square root and a divide per pair and a __match_any_sync histogram).
+constexpr int kGderThreads = 256, kGderTile = 1024, kGderMaxCopies = kGderThreads / 32;
+constexpr float kRintMagic = 12582912.f;  // 1.5 2^23: adding it rounds |x| < 2^22 to an integer
 __device__ __forceinline__ int gder_bin(float dx, float dy, float dz, float side, float side_inv, float range,
                                         float range2_hi, float bin_size, int nbins) {
     dx = min_image_gder(dx, side, side_inv);
@@ -234,57 +260,154 @@ __device__ __forceinline__ int gder_bin(float dx, float dy, float dz, float side
     if (bin == nbins) bin--;
     return bin;
 }
-__device__ __forceinline__ void hist_add(unsigned *hist, int bin, unsigned lane_mask_all) {
-    unsigned same = __match_any_sync(lane_mask_all, bin);
-    int lane = threadIdx.x & 31;
-    if (bin >= 0 && lane == __ffs(same) - 1) atomicAdd(&hist[bin], (unsigned)__popc(same));
-}
+struct GderArgs {
+    const float *ra, *rb;
+    int na, nb;
+    float side, side_inv, range, range2_hi, bin_size;
+    float thr;      // smallest squared distance at or beyond the range
+    float inv_bin;  // estimate only
+    int nbins, jchunk, copies;
+    unsigned long long *counts;
+};
+// one pair in the reference's arithmetic, both directions when SAME
 template <bool SAME>
-__global__ void __launch_bounds__(256) k_gder(const float *__restrict__ ra, int na, const float *__restrict__ rb,
-                                              int nb, float side, float side_inv, float range, float range2_hi,
-                                              float bin_size, int nbins, int jchunk,
-                                              unsigned long long *counts) {
-    extern __shared__ unsigned char smem[];
+__device__ __noinline__ void gder_pair_exact(const GderArgs &a, float dx, float dy, float dz, unsigned *hist) {
+    const int bf = gder_bin(dx, dy, dz, a.side, a.side_inv, a.range, a.range2_hi, a.bin_size, a.nbins);
+    if (bf >= 0) atomicAdd(&hist[bf], 1u);
+    if (SAME) {
+        const int br = gder_bin(-dx, -dy, -dz, a.side, a.side_inv, a.range, a.range2_hi, a.bin_size, a.nbins);
+        if (br >= 0) atomicAdd(&hist[br], 1u);
+    }
+}
+template <bool SAME, bool CHECK>
+__global__ void __launch_bounds__(kGderThreads) k_gder(const GderArgs a) {
+    extern __shared__ __align__(16) unsigned char smem[];
     float *tx = reinterpret_cast<float *>(smem);
     float *ty = tx + kGderTile, *tz = ty + kGderTile;
-    unsigned *hist = reinterpret_cast<unsigned *>(tz + kGderTile);
-    for (int b = threadIdx.x; b < nbins; b += blockDim.x) hist[b] = 0;
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    const bool vi = i < na;
-    float xi = 0, yi = 0, zi = 0;
-    if (vi) { xi = ra[3 * i]; yi = ra[3 * i + 1]; zi = ra[3 * i + 2]; }
-    int j0 = blockIdx.y * jchunk, j1 = min(nb, j0 + jchunk);
-    if (SAME) j0 = max(j0, (int)(blockIdx.x * blockDim.x) + 1);
-    __syncthreads();
+    unsigned *hist0 = reinterpret_cast<unsigned *>(tz + kGderTile);  // [copies][nbins + 32]
+    const int i0 = blockIdx.x * kGderThreads, i = i0 + threadIdx.x;
+    int j0 = blockIdx.y * a.jchunk;
+    const int j1 = min(a.nb, j0 + a.jchunk);
+    if (SAME) j0 = max(j0, i0 + 1);  // partners before the block's first particle: other blocks count them
+    if (j0 >= j1) return;
+    const int nbins = a.nbins;
+    // a copy ends with a spare word per lane, where uncounted pairs add
+    const int stride = nbins + 32, spare = nbins + (threadIdx.x & 31);
+    unsigned *hist = hist0 + ((threadIdx.x >> 5) * a.copies / kGderMaxCopies) * stride;
+    for (int b = threadIdx.x; b < a.copies * stride; b += kGderThreads) hist0[b] = 0;
+    const float wild_lo = -0.2f * a.side, wild_hi = 1.2f * a.side;
+    auto wild_at = [&](float v) { return !(v >= wild_lo && v <= wild_hi); };
+    const float nan = __int_as_float(0x7fffffff);  // a distance from it is never within range
+    float xi = nan, yi = nan, zi = nan;
+    bool wild = false;
+    if (i < a.na) {
+        xi = a.ra[3 * (size_t)i], yi = a.ra[3 * (size_t)i + 1], zi = a.ra[3 * (size_t)i + 2];
+        wild = wild_at(xi) || wild_at(yi) || wild_at(zi);
+    }
+    const f2 XI = f2_bcast(xi), YI = f2_bcast(yi), ZI = f2_bcast(zi);
+    const f2 SINV = f2_bcast(a.side_inv), NSIDE = f2_bcast(-a.side), MAGIC = f2_bcast(kRintMagic);
+    const float edge = 0.4899f * a.side;
+    const float near = a.thr * 1.000001f, lim = CHECK ? a.thr * 1.0001f : near;
+    const float half_eps = 0.5f - 1.5e-6f * (float)(nbins + 1);
+    const f2 INVB = f2_bcast(a.inv_bin), NHALF = f2_bcast(-0.5f);
     for (int t0 = j0; t0 < j1; t0 += kGderTile) {
-        int tn = min(kGderTile, j1 - t0);
+        const int tn = min(kGderTile, j1 - t0), tp = (tn + 3) & ~3;
         __syncthreads();
-        for (int t = threadIdx.x; t < tn; t += blockDim.x) {
-            tx[t] = rb[3 * (t0 + t)];
-            ty[t] = rb[3 * (t0 + t) + 1];
-            tz[t] = rb[3 * (t0 + t) + 2];
+        for (int t = threadIdx.x; t < tp; t += kGderThreads) {
+            float x = nan, y = nan, z = nan;  // padding
+            if (t < tn) {
+                const size_t j = 3 * (size_t)(t0 + t);
+                x = a.rb[j], y = a.rb[j + 1], z = a.rb[j + 2];
+                wild = wild || wild_at(x) || wild_at(y) || wild_at(z);
+            }
+            tx[t] = x, ty[t] = y, tz[t] = z;
         }
-        __syncthreads();
-        for (int t = 0; t < tn; t++) {
-            int j = t0 + t;
-            bool ok = vi && (!SAME || j > i);
-            int bf = -1, br = -1;
-            if (ok) {
-                float dx = __fsub_rn(xi, tx[t]), dy = __fsub_rn(yi, ty[t]), dz = __fsub_rn(zi, tz[t]);
-                bf = gder_bin(dx, dy, dz, side, side_inv, range, range2_hi, bin_size, nbins);
-                if (SAME) {
-                    bool sym = fabsf(__fmul_rn(side_inv, dx)) < 0.25f && fabsf(__fmul_rn(side_inv, dy)) < 0.25f &&
-                               fabsf(__fmul_rn(side_inv, dz)) < 0.25f;
-                    br = sym ? bf : gder_bin(-dx, -dy, -dz, side, side_inv, range, range2_hi, bin_size, nbins);
+        if (__syncthreads_or(wild)) {
+            if (i < a.na)
+                for (int t = 0; t < tn; t++)
+                    if (!SAME || t0 + t > i)
+                        gder_pair_exact<SAME>(a, __fsub_rn(xi, tx[t]), __fsub_rn(yi, ty[t]), __fsub_rn(zi, tz[t]),
+                                              hist);
+            continue;
+        }
+        auto image = [&](f2 d) {
+            return f2_fma(f2_sub(f2_fma(d, SINV, MAGIC), MAGIC), NSIDE, d);
+        };
+        // a pair whose estimate does not settle its bin
+        auto settle = [&](float d2, float dx, float dy, float dz, int t) {
+            if (CHECK) {
+                if (fmaxf(fmaxf(fabsf(dx), fabsf(dy)), fabsf(dz)) > edge) {
+                    gder_pair_exact<SAME>(a, __fsub_rn(xi, tx[t]), __fsub_rn(yi, ty[t]), __fsub_rn(zi, tz[t]), hist);
+                    return;
+                }
+                if (!(d2 < near)) return;
+            }
+            const float e2 = dist2_rn(dx, dy, dz);
+            if (!(e2 < a.thr)) return;
+            int bin = (int)__fdiv_rn(__fsqrt_rn(e2), a.bin_size);
+            if (bin == nbins) bin--;
+            atomicAdd(&hist[bin], SAME ? 2u : 1u);
+        };
+        auto pairs = [&](auto diagonal) {  // diagonal: some partner of the tile may not come after i
+            constexpr bool kDiag = decltype(diagonal)::value;
+            for (int t = 0; t < tp; t += 4) {
+                const float4 x = *reinterpret_cast<const float4 *>(tx + t),
+                             y = *reinterpret_cast<const float4 *>(ty + t),
+                             z = *reinterpret_cast<const float4 *>(tz + t);
+                float d2[4], dx[4], dy[4], dz[4], qm[4];
+                bool open[4];
+                int slot[4];
+#pragma unroll
+                for (int u = 0; u < 4; u += 2) {
+                    const f2 DX = image(f2_sub(XI, u ? f2_make(x.z, x.w) : f2_make(x.x, x.y)));
+                    const f2 DY = image(f2_sub(YI, u ? f2_make(y.z, y.w) : f2_make(y.x, y.y)));
+                    const f2 DZ = image(f2_sub(ZI, u ? f2_make(z.z, z.w) : f2_make(z.x, z.y)));
+                    const f2 D2 = f2_fma(DZ, DZ, f2_fma(DY, DY, f2_mul(DX, DX)));
+                    f2_split(D2, d2[u], d2[u + 1]);
+                    f2_split(DX, dx[u], dx[u + 1]);
+                    f2_split(DY, dy[u], dy[u + 1]);
+                    f2_split(DZ, dz[u], dz[u + 1]);
+                    // q - 1/2 rounded to the nearest integer: floor(q) unless q is next to one
+                    const f2 Q = f2_fma(f2_mul(D2, f2_make(rsqrtf(d2[u]), rsqrtf(d2[u + 1]))), INVB, NHALF);
+                    const f2 QM = f2_add(Q, MAGIC), R = f2_sub(Q, f2_sub(QM, MAGIC));
+                    float r[2];
+                    f2_split(QM, qm[u], qm[u + 1]);
+                    f2_split(R, r[0], r[1]);
+#pragma unroll
+                    for (int h = 0; h < 2; h++) {
+                        const int v = u + h;
+                        bool in = d2[v] < lim;
+                        if (kDiag) in = in & (t0 + t + v > i);
+                        bool far = !(fabsf(r[h]) <= half_eps);
+                        if (CHECK) {
+                            far = far | (fmaxf(fmaxf(fabsf(dx[v]), fabsf(dy[v])), fabsf(dz[v])) > edge);
+                            open[v] = in & far;
+                            in = in & (d2[v] < near);
+                        } else {
+                            open[v] = in & far;
+                        }
+                        slot[v] = in & !far ? __float_as_int(qm[v]) - __float_as_int(kRintMagic) : spare;
+                    }
+                }
+#pragma unroll
+                for (int u = 0; u < 4; u++) atomicAdd(&hist[slot[u]], SAME ? 2u : 1u);
+                const bool any = open[0] | open[1] | open[2] | open[3];
+                if (any) {
+#pragma unroll
+                    for (int u = 0; u < 4; u++)
+                        if (open[u]) settle(d2[u], dx[u], dy[u], dz[u], t + u);
                 }
             }
-            hist_add(hist, bf, 0xffffffffu);
-            if (SAME) hist_add(hist, br, 0xffffffffu);
-        }
+        };
+        if (SAME && t0 <= i0 + kGderThreads - 1) pairs(std::true_type{});
+        else pairs(std::false_type{});
     }
     __syncthreads();
-    for (int b = threadIdx.x; b < nbins; b += blockDim.x)
-        if (hist[b]) atomicAdd(&counts[b], (unsigned long long)hist[b]);
+    for (int b = threadIdx.x; b < nbins; b += kGderThreads) {
+        unsigned long long v = 0;
+        for (int c = 0; c < a.copies; c++) v += hist0[c * stride + b];
+        if (v) atomicAdd(&a.counts[b], v);
+    }
 }
 
 // ------------------------------------------------------------ F_s, MSD
@@ -599,6 +722,22 @@ float bd_calculate_temp_sine(float T0, float Tf, float t0, float tf, float perio
     return a + bs;
 }
 
+// smallest float x >= 0 whose square root is not below `range` (bisection over
+// the bit patterns of the non-negative floats)
+static float sqrt_threshold(float range) {
+    unsigned lo = 0u, hi = 0x7f800000u;  // +0 .. +inf
+    while (lo < hi) {
+        const unsigned mid = lo + ((hi - lo) >> 1);
+        float x;
+        std::memcpy(&x, &mid, 4);
+        if (!(std::sqrt(x) < range)) hi = mid;
+        else lo = mid + 1;
+    }
+    float x;
+    std::memcpy(&x, &lo, 4);
+    return x;
+}
+
 int bd_get_gder(char type, char type_other, const float *rr, const float *rr_other, unsigned long long *counts,
                 const bd_parametros *p, void *stream) {
     if (!p || (type != 'b' && type != 's') || (type_other != 'b' && type_other != 's') || !counts) return BD_ERR_ARG;
@@ -608,23 +747,40 @@ int bd_get_gder(char type, char type_other, const float *rr, const float *rr_oth
     if (nbins < 1 || nbins > 8192 || !(p->range_gder > 0)) return BD_ERR_ARG;
     if (na == 0 || nb == 0) return BD_OK;
     if (!rr || !rr_other) return BD_ERR_ARG;
-    const float side = p->side, side_inv = (float)(1.0 / side), range = p->range_gder;
-    const float bin_size = range / ((float)nbins);
-    const float range2_hi = range * range * 1.00001f;
+    GderArgs a;
+    a.ra = rr;
+    a.rb = rr_other;
+    a.na = na;
+    a.nb = nb;
+    a.side = p->side;
+    a.side_inv = (float)(1.0 / a.side);
+    a.range = p->range_gder;
+    a.range2_hi = a.range * a.range * 1.00001f;
+    a.bin_size = a.range / ((float)nbins);
+    a.inv_bin = 1.0f / a.bin_size;
+    a.thr = sqrt_threshold(a.range);
+    a.nbins = nbins;
+    a.counts = counts;
     const bool same = type == type_other;
-    const int jchunk = 8192;
-    dim3 grid(div_up(na, 256), div_up(nb, jchunk));
-    size_t sm = 3 * kGderTile * sizeof(float) + (size_t)nbins * sizeof(unsigned);
+    // partners per block: enough blocks for 8 of 256 threads on each SM (half
+    // of the grid of equal species is empty), in tiles of at least 64 so that
+    // the histogram's clear and flush stay a small part
+    const int rows = div_up(na, kGderThreads);
+    const long want = (long)148 * 8 * (same ? 2 : 1);
+    const long per = ((long)rows * nb / want + 63) / 64 * 64;
+    a.jchunk = (int)std::min(8192L, std::max(64L, per));
+    a.copies = kGderMaxCopies;  // a power of two
+    while (a.copies > 1 && (size_t)a.copies * (nbins + 32) * sizeof(unsigned) > 32 * 1024) a.copies /= 2;
+    const dim3 grid(rows, div_up(nb, a.jchunk));
+    const size_t sm = 3 * kGderTile * sizeof(float) + (size_t)a.copies * (nbins + 32) * sizeof(unsigned);
     cudaStream_t s = as_stream(stream);
-    if (same) {
-        BD_CUDA_TRY(cudaFuncSetAttribute(k_gder<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
-        k_gder<true><<<grid, 256, sm, s>>>(rr, na, rr_other, nb, side, side_inv, range, range2_hi, bin_size, nbins,
-                                           jchunk, counts);
-    } else {
-        BD_CUDA_TRY(cudaFuncSetAttribute(k_gder<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
-        k_gder<false><<<grid, 256, sm, s>>>(rr, na, rr_other, nb, side, side_inv, range, range2_hi, bin_size, nbins,
-                                            jchunk, counts);
-    }
+    // pairs at the edge of the minimum image may be within range
+    const float edge = 0.489f * a.side;
+    const bool check = !(a.thr <= edge * edge);
+    auto kern = same ? (check ? k_gder<true, true> : k_gder<true, false>)
+                     : (check ? k_gder<false, true> : k_gder<false, false>);
+    if (sm > 48 * 1024) BD_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+    kern<<<grid, kGderThreads, sm, s>>>(a);
     BD_LAUNCH_CHECK();
     return BD_OK;
 }

@@ -25,41 +25,6 @@ namespace bd {
 constexpr int kQueue = 72;            // queue length per thread; >= one row (3 cells x 24 slots)
 constexpr unsigned kNoShift = 0x15u;  // shift code of a halo cell that did not wrap
 
-typedef unsigned long long f2;  // two floats in one 64-bit register (lo, hi)
-__device__ __forceinline__ f2 f2_bcast(float v) {
-    f2 r;
-    asm("mov.b64 %0, {%1, %1};" : "=l"(r) : "f"(v));
-    return r;
-}
-__device__ __forceinline__ void f2_split(f2 v, float &lo, float &hi) {
-    asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
-}
-__device__ __forceinline__ f2 f2_add(f2 a, f2 b) {
-    f2 d;
-    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
-    return d;
-}
-__device__ __forceinline__ f2 f2_sub(f2 a, f2 b) {
-    f2 d;
-    asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
-    return d;
-}
-__device__ __forceinline__ f2 f2_mul(f2 a, f2 b) {
-    f2 d;
-    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
-    return d;
-}
-__device__ __forceinline__ f2 f2_make(float lo, float hi) {
-    f2 r;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
-    return r;
-}
-__device__ __forceinline__ f2 f2_fma(f2 a, f2 b, f2 c) {
-    f2 d;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
-    return d;
-}
-
 struct BrickSmem {
     int *start;             // [nh+1] staged-particle prefix over halo cells
     int *hstart;            // [nh+1] home-particle prefix over halo cells

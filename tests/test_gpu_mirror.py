@@ -112,6 +112,37 @@ def test_gder_counts_exact_larger_system():
         np.testing.assert_array_equal(host(counts).astype(np.uint64), ref[k])
 
 
+@pytest.mark.parametrize("nb,ns,nbins,reach,where", [
+    (1, 1, 7, 0.5, "fluid"), (255, 257, 200, 0.5, "fluid"), (256, 65, 8192, 0.49, "fluid"),
+    (513, 511, 1, 0.87, "fluid"), (700, 343, 64, 0.8, "lattice"), (512, 512, 300, 0.5, "lattice"),
+    (300, 200, 90, 0.6, "outside")])
+def test_gder_counts_exact_edges(nb, ns, nbins, reach, where):
+    """Sizes around a block of particles and a partner tile, one bin and the
+    most bins, ranges below, at and beyond L / 2, a lattice whose separations
+    are exact fractions of L (ties of the minimum image, distances on bin
+    edges, coincident points), and coordinates outside the box."""
+    import torch
+    rng = np.random.default_rng(nb + nbins)
+    side = 8.0 if where == "lattice" else CF.side_from_phi(nb + 60, ns + 60, 0.4)
+    n = nb + ns
+    if where == "lattice":
+        pos = rng.integers(0, 9, (n, 3)).astype(np.float32)
+    else:
+        pos = rng.uniform(0, side, (n, 3)).astype(np.float32)
+    if where == "outside":
+        pos[::7] += np.float32(1.5 * side)
+        pos[::11, 0] -= np.float32(3 * side)
+    p = O.setup_params(side, nb, ns, float(CF.SIGMA_BIG), float(CF.SIGMA_SML), nbins=nbins, rng=reach * side)
+    ref = O.gder_counts(p, pos[:nb].copy(), pos[nb:].copy())
+    pp = B.Parametros.from_buffer_copy(bytes(p))
+    rb, rs = dev(pos[:nb]), dev(pos[nb:])
+    for k, (a, b, ra, rbb) in enumerate((("b", "b", rb, rb), ("b", "s", rb, rs), ("s", "b", rs, rb),
+                                         ("s", "s", rs, rs))):
+        counts = torch.zeros(nbins, dtype=torch.int64, device="cuda:0")
+        B.get_gder(a, b, ra, rbb, counts, pp)
+        np.testing.assert_array_equal(host(counts).astype(np.uint64), ref[k], err_msg=a + b)
+
+
 def test_fself_and_msd(golden):
     raw, r0 = golden["g1_fself_raw_b"], golden["g1_rb"]
     fs = np.zeros(4, np.float32)
