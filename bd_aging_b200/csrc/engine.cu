@@ -1,115 +1,8 @@
 // engine.cu -- host driver of the batched replica engine (bd_engine_* ABI):
-// geometry, buffers, initial load, CUDA-graph stepping, observation passes,
-// export, and the batch g(r) kernel.
+// geometry, buffers, initial load, CUDA-graph stepping, observation passes and
+// export.
 #include "engine_kernels.cuh"
 #include "engine_state.cuh"
-
-namespace bd {
-
-// ------------------------------------------------------------- batch g(r)
-// get_gder_dev (get_gder.cu:69-127) for all four species pairs of one
-// replica in one pass over unordered pairs i < j: the forward distance
-// (r_i - r_j) counts for (type_i, type_j), the reverse one for (type_j,
-// type_i), recomputed when the minimum-image rounding can differ.  Big
-// particles come first, so i < j gives bb, bs and ss forward and bb, sb, ss
-// in reverse.
-// g(r) bin thresholds (gr_bin_thr): thr[k], k = 0 .. nbins + 1
-__global__ void k_gr_thresholds(float range, int nbins, float *thr) {
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k > nbins + 1) return;
-    if (k == 0) { thr[0] = 0.f; return; }
-    const float bin_size = __fdiv_rn(range, (float)nbins);
-    unsigned lo = 0u, hi = 0x7f800000u;  // +0 .. +inf
-    while (lo < hi) {
-        const unsigned mid = lo + ((hi - lo) >> 1);
-        const float x = __uint_as_float(mid);
-        const bool reach = k <= nbins ? gr_bin_exact(x, bin_size) >= k : !(__fsqrt_rn(x) < range);
-        if (reach) hi = mid;
-        else lo = mid + 1;
-    }
-    thr[k] = __uint_as_float(lo);
-}
-constexpr int kGrTile = 1024;
-__device__ __forceinline__ int gr_bin(float dx, float dy, float dz, float side, float side_inv, const float *thr,
-                                      float inv_bin_size, int nbins) {
-    dx = min_image_gder_fast(dx, side, side_inv);
-    dy = min_image_gder_fast(dy, side, side_inv);
-    dz = min_image_gder_fast(dz, side, side_inv);
-    return gr_bin_thr(dist2_rn(dx, dy, dz), thr, inv_bin_size, nbins);
-}
-// One launch for every replica that needs all pairs (blockIdx.z indexes
-// `reps`).  Histogram: with `copies` > 1 each pair of warps adds into its own
-// copy in shared memory with plain atomics (bins spread over the lanes rarely
-// collide), and the copies are summed at the end; with one copy, lanes of
-// equal bins are combined by __match_any_sync first.
-__global__ void __launch_bounds__(256) k_gr_batch(const float4 *__restrict__ snap_all, const SysDev *__restrict__ sys,
-                                                  const int *__restrict__ reps, float range,
-                                                  const float *__restrict__ thr_g, int nbins, int jchunk, int copies,
-                                                  unsigned long long *counts_all) {
-    extern __shared__ __align__(16) unsigned char smem[];
-    const int r = reps[blockIdx.z];
-    const SysDev &S = sys[r];
-    const int n = S.n, n_big = S.n_big;
-    const int j0 = max(blockIdx.y * jchunk, (int)(blockIdx.x * blockDim.x) + 1), j1 = min(n, (int)(blockIdx.y + 1) * jchunk);
-    if (j0 >= j1) return;  // uniform over the block: no pair of this replica here
-    const float4 *snap = snap_all + S.part_base;
-    unsigned long long *counts = counts_all + (size_t)r * 4 * nbins;
-    const float side = S.L;
-    float4 *tile = reinterpret_cast<float4 *>(smem);
-    float *thr = reinterpret_cast<float *>(tile + kGrTile);          // [nbins + 2] bin thresholds
-    unsigned *hist0 = reinterpret_cast<unsigned *>(thr + nbins + 2);  // [copies][4][nbins]
-    for (int b = threadIdx.x; b < copies * 4 * nbins; b += blockDim.x) hist0[b] = 0;
-    for (int b = threadIdx.x; b < nbins + 2; b += blockDim.x) thr[b] = thr_g[b];
-    const int per_copy = (blockDim.x / 32 + copies - 1) / copies;  // warps per copy
-    unsigned *hist = hist0 + ((threadIdx.x >> 5) / per_copy) * 4 * nbins;
-    const float side_inv = __double2float_rn(1.0 / (double)side);
-    const float inv_bin_size = 1.0f / __fdiv_rn(range, (float)nbins);  // estimate only (gr_bin_thr)
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    const bool vi = i < n;
-    float4 pi = vi ? snap[i] : make_float4(0, 0, 0, 0);
-    const int ti = i < n_big ? 0 : 1;
-    __syncthreads();
-    for (int t0 = j0; t0 < j1; t0 += kGrTile) {
-        const int tn = min(kGrTile, j1 - t0);
-        __syncthreads();
-        for (int t = threadIdx.x; t < tn; t += blockDim.x) tile[t] = snap[t0 + t];
-        __syncthreads();
-        for (int t = 0; t < tn; t++) {
-            const int j = t0 + t;
-            const int tj = j < n_big ? 0 : 1;
-            int kf = -1, kr = -1;
-            if (vi && j > i) {
-                float4 pj = tile[t];
-                float dx = __fsub_rn(pi.x, pj.x), dy = __fsub_rn(pi.y, pj.y), dz = __fsub_rn(pi.z, pj.z);
-                int bf = gr_bin(dx, dy, dz, side, side_inv, thr, inv_bin_size, nbins);
-                // below 0.49 the minimum image returns d itself for both signs
-                // (min_image_gder_fast), so the reverse distance is the same
-                bool sym = fabsf(__fmul_rn(side_inv, dx)) < 0.49f && fabsf(__fmul_rn(side_inv, dy)) < 0.49f &&
-                           fabsf(__fmul_rn(side_inv, dz)) < 0.49f;
-                int bb = sym ? bf : gr_bin(-dx, -dy, -dz, side, side_inv, thr, inv_bin_size, nbins);
-                if (bf >= 0) kf = (ti * 2 + tj) * nbins + bf;
-                if (bb >= 0) kr = (tj * 2 + ti) * nbins + bb;
-            }
-            if (copies > 1) {
-                if (kf >= 0) atomicAdd(&hist[kf], 1u);
-                if (kr >= 0) atomicAdd(&hist[kr], 1u);
-            } else {
-                unsigned s1 = __match_any_sync(0xffffffffu, kf);
-                if (kf >= 0 && (threadIdx.x & 31) == __ffs(s1) - 1) atomicAdd(&hist[kf], (unsigned)__popc(s1));
-                unsigned s2 = __match_any_sync(0xffffffffu, kr);
-                if (kr >= 0 && (threadIdx.x & 31) == __ffs(s2) - 1) atomicAdd(&hist[kr], (unsigned)__popc(s2));
-            }
-        }
-    }
-    __syncthreads();
-    for (int b = threadIdx.x; b < 4 * nbins; b += blockDim.x) {
-        unsigned long long v = 0;
-        for (int c = 0; c < copies; c++) v += hist0[c * 4 * nbins + b];
-        if (v) atomicAdd(&counts[b], v);
-    }
-}
-
-}  // namespace bd
 
 using namespace bd;
 
@@ -402,6 +295,15 @@ int bd::sync_dsp(bd_engine *e) {
     return BD_OK;
 }
 
+int bd::export_snap(bd_engine *e) {
+    const int b = obs_buf(e);
+    k_export<<<div_up(e->C, 128), 128, 0, e->stream>>>(e->cnt[b], e->pos[b], (int)e->C, e->cap, (int)e->P, e->gid_of,
+                                                       e->x0, e->dsp[0], e->dsp[1], e->dsp[2], nullptr, nullptr,
+                                                       e->snap);
+    BD_LAUNCH_CHECK();
+    return BD_OK;
+}
+
 namespace {
 // observation passes read cell buckets and displacements: rebuild them from
 // the by-id state
@@ -488,7 +390,7 @@ void free_engine(bd_engine *e) {
                     e->snaps, e->d_segs, e->d_seg_first, e->corr_part, e->corr_out, e->lpos[0], e->lpos[1],
                     e->pbuild, e->nbr, e->nnb, e->lflag, e->d_one, e->d_builds, e->ld_in, e->ld_staged,
                     e->ld_slot, e->ld_bucket, e->ld_cnt, e->ld_start, e->ld_bsum, e->ld_bad, e->img, e->amp_tab,
-                    e->d_rep_order, e->d_step_rebuilt};
+                    e->d_rep_order, e->d_step_rebuilt, e->gr_buf, e->gr_bricks};
     for (void *p : ptrs)
         if (p) cudaFree(p);
     if (e->stream) cudaStreamDestroy(e->stream);
@@ -1187,64 +1089,14 @@ int bd_engine_gder_method(bd_engine *e, int nbins, float range, int method, unsi
     if (!e->loaded) return BD_ERR_STATE;
     if (int rcb = sync_buckets(e)) return rcb;
     // per replica: cell-bounded whenever the stencil applies (it skips cells
-    // beyond the range and evaluates each unordered pair once; on the aging
-    // boxes, a region as large as the box, it measured 90 ms against 220 ms
-    // of all pairs for 64 x 32768 particles, 400 bins to 15)
+    // beyond the range)
     std::vector<int> m_of(e->R, -1);
-    bool any_all = false;
     for (int r = 0; r < e->R; r++) {
-        const SysDev &S = e->sysh[r];
-        const int m = gder_cell_reach(S, range);
+        const int m = gder_cell_reach(e->sysh[r], range);
         if (method == BD_GDER_CELLS && m < 0) return BD_ERR_ARG;
-        const bool cells = m >= 0 && (method == BD_GDER_CELLS || method == BD_GDER_AUTO);
-        m_of[r] = cells ? m : -1;
-        any_all |= !cells;
+        if (method != BD_GDER_ALL_PAIRS) m_of[r] = m;
     }
-    unsigned long long *d_counts = nullptr;
-    const size_t per = (size_t)4 * nbins;
-    // counts, then the nbins + 2 bin thresholds (gr_bin_thr)
-    BD_CUDA_TRY(cudaMalloc(&d_counts, sizeof(unsigned long long) * per * e->R + sizeof(float) * (nbins + 2)));
-    float *d_thr = reinterpret_cast<float *>(d_counts + per * e->R);
-    cudaMemsetAsync(d_counts, 0, sizeof(unsigned long long) * per * e->R, e->stream);
-    k_gr_thresholds<<<div_up(nbins + 2, 128), 128, 0, e->stream>>>(range, nbins, d_thr);
-    int rc = launch_gder_cells(e, m_of, nbins, range, d_thr, d_counts);  // may hand replicas back
-    for (int r = 0; r < e->R; r++) any_all |= m_of[r] < 0;
-    cudaError_t le = cudaSuccess;
-    if (rc == BD_OK && any_all) {
-        k_export<<<div_up(e->C, 128), 128, 0, e->stream>>>(e->cnt[obs_buf(e)], e->pos[obs_buf(e)], (int)e->C, e->cap, (int)e->P,
-                                                           e->gid_of, e->x0, e->dsp[0], e->dsp[1], e->dsp[2], nullptr,
-                                                           nullptr, e->snap);
-        // one histogram copy per two warps when 4 of them fit beside the tile
-        const int copies = (size_t)4 * per * sizeof(unsigned) <= 96 * 1024 ? 4 : 1;
-        const size_t sm = kGrTile * sizeof(float4) + sizeof(float) * (nbins + 2) + copies * per * sizeof(unsigned);
-        cudaFuncSetAttribute(k_gr_batch, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-        const int jchunk = 8192;
-        std::vector<int> reps;
-        int nmax = 0;
-        for (int r = 0; r < e->R; r++)
-            if (m_of[r] < 0) {
-                reps.push_back(r);
-                nmax = std::max(nmax, e->sysh[r].n);
-            }
-        int *d_reps = nullptr;
-        le = cudaMalloc(&d_reps, sizeof(int) * reps.size());
-        if (le == cudaSuccess)
-            le = cudaMemcpyAsync(d_reps, reps.data(), sizeof(int) * reps.size(), cudaMemcpyHostToDevice, e->stream);
-        if (le == cudaSuccess && nmax > 0) {
-            dim3 grid(div_up(nmax, 256), div_up(nmax, jchunk), (unsigned)reps.size());
-            k_gr_batch<<<grid, 256, sm, e->stream>>>(e->snap, e->d_sys, d_reps, range, d_thr, nbins, jchunk, copies,
-                                                     d_counts);
-        }
-        if (le == cudaSuccess) le = cudaStreamSynchronize(e->stream);
-        if (d_reps) cudaFree(d_reps);
-        if (le != cudaSuccess) rc = BD_ERR_CUDA;
-        le = cudaGetLastError();
-        if (le != cudaSuccess) rc = BD_ERR_CUDA;
-    }
-    cudaMemcpyAsync(counts_host, d_counts, sizeof(unsigned long long) * per * e->R, cudaMemcpyDeviceToHost, e->stream);
-    cudaStreamSynchronize(e->stream);
-    cudaFree(d_counts);
-    if (rc) return rc;
+    if (int rc = run_gder(e, m_of, nbins, range, counts_host)) return rc;
     return engine_status(e);
 }
 

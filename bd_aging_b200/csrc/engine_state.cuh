@@ -93,17 +93,22 @@ struct bd_engine {
     int *ld_bsum = nullptr;                         // [slots / kScanBlock + 1]
     unsigned *ld_bad = nullptr;
     long long ld_slots = 0;        // capacity of ld_cnt
+    // g(r): counts and per-replica words; brick table of the cell stencil (geometry only)
+    void *gr_buf = nullptr;
+    size_t gr_cap = 0;
+    int4 *gr_bricks = nullptr;
+    int gr_nbricks = 0;
 };
 
 
 namespace bd {
 
-// cell-bounded g(r) (gder.cu): stencil reach of a replica (-1: region would
-// wrap) and the launch over the replicas with m_of[r] >= 0; replicas it
-// cannot count come back with m_of[r] = -1
+// g(r) (gder.cu): stencil reach of a replica (-1: the region would wrap) and
+// the counts of every replica, by cells where m_of[r] >= 0
 int gder_cell_reach(const SysDev &S, float range);
-int launch_gder_cells(bd_engine *e, std::vector<int> &m_of, int nbins, float range, const float *d_thr,
-                      unsigned long long *d_counts);
+int run_gder(bd_engine *e, std::vector<int> &m_of, int nbins, float range, unsigned long long *counts_host);
+// positions by global index (e->snap) from the cell buckets
+int export_snap(bd_engine *e);
 
 // cell-bucket buffer holding the current state (list mode rebuilds buffer 0
 // before every observation pass)

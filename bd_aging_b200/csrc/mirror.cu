@@ -12,6 +12,7 @@
 #include <type_traits>
 #include <vector>
 
+#include "gr_bins.cuh"
 #include "runtime.cuh"
 
 namespace bd {
@@ -223,30 +224,22 @@ __global__ void k_update_noise(float *rr, float *raw, const float *__restrict__ 
 //
 // Bound: issue slots (no DRAM traffic to speak of).  What keeps a pair cheap:
 //  - the minimum image is taken as fma(rint(d / L), -L, d).  When every
-//    component of the result lies within 0.4899 L of zero, d / L is within
-//    0.49 of an integer k in {-1, 0, 1}, the reference's floor equals k and
-//    L k is exact, so the rounded difference is the reference's, and that of
-//    the reverse pair is its negation.  Pairs beyond that (they matter only
-//    when the range reaches 0.489 L) and tiles with a coordinate outside
-//    [-0.2 L, 1.2 L] take the reference's arithmetic in both directions
-//    (gder_pair_exact).
-//  - the bin floor(sqrt(d2) / bin_size) comes, without a branch, from an
-//    estimate q (fused d2, rsqrtf) whose error against the reference's separately rounded
-//    operations is below eps = 1.5e-6 (nbins + 1): relative 2^-22 for rsqrtf,
-//    2^-24 for each other rounding and for half the difference of the two
-//    d2, 6e-7 in all.  Only a q closer than eps to an integer, the range
-//    among them (it is bin edge nbins), needs the reference's d2, square root
-//    and divide.
-//  - a pair out of range adds to a spare word of its lane instead of
-//    branching, and bins are added with plain shared atomics into a histogram copy per warp
-//    (fewer copies when they would pass 32 KB).
+//    component of the result lies within 0.49999 L of zero, d / L is within
+//    0.499995 of an integer k in {-1, 0, 1} (its rounding errors are below
+//    4e-7), the reference's floor equals k and L k is exact, so the rounded
+//    difference is the reference's, and that of the reverse pair is its
+//    negation.  Pairs beyond that (they matter only when the range reaches
+//    L / 2) and tiles with a coordinate outside [-0.2 L, 1.2 L] take the
+//    reference's arithmetic in both directions (gder_pair_exact);
+//  - the bin comes from an estimate (gr_bins.cuh), without a branch;
+//  - every pair adds to its estimated slot with a plain shared atomic, into a
+//    histogram copy per warp (fewer copies when they would pass 32 KB); an
+//    open pair takes that count back.
 // Blocks are cut over the partners until the grid has several per SM.
-// Measured at 4095 + 4099 particles, 200 bins to L / 2: 25 us for equal
-// species and 35 us for mixed ones, 43 thread instructions a pair, 46-59% of
-// issue slots (3.49 and 1.74 ms with 16 to 128 blocks of 8192 partners, a
-// square root and a divide per pair and a __match_any_sync histogram).
+// Measured at 4095 + 4099 particles, 200 bins to L / 2, the four species
+// pairs: 10.46 -> 0.11 ms (before: 16 to 128 blocks of 8192 partners, a square
+// root and a divide per pair, a __match_any_sync histogram).
 constexpr int kGderThreads = 256, kGderTile = 1024, kGderMaxCopies = kGderThreads / 32;
-constexpr float kRintMagic = 12582912.f;  // 1.5 2^23: adding it rounds |x| < 2^22 to an integer
 __device__ __forceinline__ int gder_bin(float dx, float dy, float dz, float side, float side_inv, float range,
                                         float range2_hi, float bin_size, int nbins) {
     dx = min_image_gder(dx, side, side_inv);
@@ -263,19 +256,20 @@ __device__ __forceinline__ int gder_bin(float dx, float dy, float dz, float side
 struct GderArgs {
     const float *ra, *rb;
     int na, nb;
-    float side, side_inv, range, range2_hi, bin_size;
-    float thr;      // smallest squared distance at or beyond the range
-    float inv_bin;  // estimate only
-    int nbins, jchunk, copies;
+    float side, side_inv, range, range2_hi;
+    GrBins bins;
+    int jchunk, copies;
     unsigned long long *counts;
 };
 // one pair in the reference's arithmetic, both directions when SAME
 template <bool SAME>
 __device__ __noinline__ void gder_pair_exact(const GderArgs &a, float dx, float dy, float dz, unsigned *hist) {
-    const int bf = gder_bin(dx, dy, dz, a.side, a.side_inv, a.range, a.range2_hi, a.bin_size, a.nbins);
+    const int bf = gder_bin(dx, dy, dz, a.side, a.side_inv, a.range, a.range2_hi, a.bins.bin_size,
+                            a.bins.nbins);
     if (bf >= 0) atomicAdd(&hist[bf], 1u);
     if (SAME) {
-        const int br = gder_bin(-dx, -dy, -dz, a.side, a.side_inv, a.range, a.range2_hi, a.bin_size, a.nbins);
+        const int br = gder_bin(-dx, -dy, -dz, a.side, a.side_inv, a.range, a.range2_hi, a.bins.bin_size,
+                            a.bins.nbins);
         if (br >= 0) atomicAdd(&hist[br], 1u);
     }
 }
@@ -284,16 +278,16 @@ __global__ void __launch_bounds__(kGderThreads) k_gder(const GderArgs a) {
     extern __shared__ __align__(16) unsigned char smem[];
     float *tx = reinterpret_cast<float *>(smem);
     float *ty = tx + kGderTile, *tz = ty + kGderTile;
-    unsigned *hist0 = reinterpret_cast<unsigned *>(tz + kGderTile);  // [copies][nbins + 32]
+    unsigned *hist0 = reinterpret_cast<unsigned *>(tz + kGderTile);  // [copies][nbins + kGrSpare]
     const int i0 = blockIdx.x * kGderThreads, i = i0 + threadIdx.x;
     int j0 = blockIdx.y * a.jchunk;
     const int j1 = min(a.nb, j0 + a.jchunk);
     if (SAME) j0 = max(j0, i0 + 1);  // partners before the block's first particle: other blocks count them
     if (j0 >= j1) return;
-    const int nbins = a.nbins;
-    // a copy ends with a spare word per lane, where uncounted pairs add
-    const int stride = nbins + 32, spare = nbins + (threadIdx.x & 31);
+    const int nbins = a.bins.nbins;
+    const int stride = nbins + kGrSpare;
     unsigned *hist = hist0 + ((threadIdx.x >> 5) * a.copies / kGderMaxCopies) * stride;
+    const unsigned row = gr_row(hist), top = gr_top(nbins, threadIdx.x & 31);
     for (int b = threadIdx.x; b < a.copies * stride; b += kGderThreads) hist0[b] = 0;
     const float wild_lo = -0.2f * a.side, wild_hi = 1.2f * a.side;
     auto wild_at = [&](float v) { return !(v >= wild_lo && v <= wild_hi); };
@@ -306,10 +300,9 @@ __global__ void __launch_bounds__(kGderThreads) k_gder(const GderArgs a) {
     }
     const f2 XI = f2_bcast(xi), YI = f2_bcast(yi), ZI = f2_bcast(zi);
     const f2 SINV = f2_bcast(a.side_inv), NSIDE = f2_bcast(-a.side), MAGIC = f2_bcast(kRintMagic);
-    const float edge = 0.4899f * a.side;
-    const float near = a.thr * 1.000001f, lim = CHECK ? a.thr * 1.0001f : near;
-    const float half_eps = 0.5f - 1.5e-6f * (float)(nbins + 1);
-    const f2 INVB = f2_bcast(a.inv_bin), NHALF = f2_bcast(-0.5f);
+    const float edge = 0.49999f * a.side;
+    const float lim = a.bins.near * (CHECK ? 1.0001f : 1.0f);
+    constexpr unsigned kWeight = SAME ? 2u : 1u;
     for (int t0 = j0; t0 < j1; t0 += kGderTile) {
         const int tn = min(kGderTile, j1 - t0), tp = (tn + 3) & ~3;
         __syncthreads();
@@ -334,19 +327,14 @@ __global__ void __launch_bounds__(kGderThreads) k_gder(const GderArgs a) {
             return f2_fma(f2_sub(f2_fma(d, SINV, MAGIC), MAGIC), NSIDE, d);
         };
         // a pair whose estimate does not settle its bin
-        auto settle = [&](float d2, float dx, float dy, float dz, int t) {
-            if (CHECK) {
-                if (fmaxf(fmaxf(fabsf(dx), fabsf(dy)), fabsf(dz)) > edge) {
-                    gder_pair_exact<SAME>(a, __fsub_rn(xi, tx[t]), __fsub_rn(yi, ty[t]), __fsub_rn(zi, tz[t]), hist);
-                    return;
-                }
-                if (!(d2 < near)) return;
+        auto settle = [&](unsigned slot, float dx, float dy, float dz, int t) {
+            gr_uncount(row, slot, kWeight, nbins);
+            if (CHECK && fmaxf(fmaxf(fabsf(dx), fabsf(dy)), fabsf(dz)) > edge) {
+                gder_pair_exact<SAME>(a, __fsub_rn(xi, tx[t]), __fsub_rn(yi, ty[t]), __fsub_rn(zi, tz[t]), hist);
+                return;
             }
             const float e2 = dist2_rn(dx, dy, dz);
-            if (!(e2 < a.thr)) return;
-            int bin = (int)__fdiv_rn(__fsqrt_rn(e2), a.bin_size);
-            if (bin == nbins) bin--;
-            atomicAdd(&hist[bin], SAME ? 2u : 1u);
+            if (e2 < a.bins.thr) atomicAdd(&hist[gr_bin_settled(e2, a.bins)], kWeight);
         };
         auto pairs = [&](auto diagonal) {  // diagonal: some partner of the tile may not come after i
             constexpr bool kDiag = decltype(diagonal)::value;
@@ -354,9 +342,9 @@ __global__ void __launch_bounds__(kGderThreads) k_gder(const GderArgs a) {
                 const float4 x = *reinterpret_cast<const float4 *>(tx + t),
                              y = *reinterpret_cast<const float4 *>(ty + t),
                              z = *reinterpret_cast<const float4 *>(tz + t);
-                float d2[4], dx[4], dy[4], dz[4], qm[4];
+                float d2[4], dx[4], dy[4], dz[4];
+                unsigned slot[4];
                 bool open[4];
-                int slot[4];
 #pragma unroll
                 for (int u = 0; u < 4; u += 2) {
                     const f2 DX = image(f2_sub(XI, u ? f2_make(x.z, x.w) : f2_make(x.x, x.y)));
@@ -367,35 +355,25 @@ __global__ void __launch_bounds__(kGderThreads) k_gder(const GderArgs a) {
                     f2_split(DX, dx[u], dx[u + 1]);
                     f2_split(DY, dy[u], dy[u + 1]);
                     f2_split(DZ, dz[u], dz[u + 1]);
-                    // q - 1/2 rounded to the nearest integer: floor(q) unless q is next to one
-                    const f2 Q = f2_fma(f2_mul(D2, f2_make(rsqrtf(d2[u]), rsqrtf(d2[u + 1]))), INVB, NHALF);
-                    const f2 QM = f2_add(Q, MAGIC), R = f2_sub(Q, f2_sub(QM, MAGIC));
-                    float r[2];
-                    f2_split(QM, qm[u], qm[u + 1]);
-                    f2_split(R, r[0], r[1]);
+                    unsigned sl[2];
+                    bool far[2];
+                    gr_estimate(D2, a.bins, top, sl, far);
 #pragma unroll
                     for (int h = 0; h < 2; h++) {
                         const int v = u + h;
                         bool in = d2[v] < lim;
-                        if (kDiag) in = in & (t0 + t + v > i);
-                        bool far = !(fabsf(r[h]) <= half_eps);
-                        if (CHECK) {
-                            far = far | (fmaxf(fmaxf(fabsf(dx[v]), fabsf(dy[v])), fabsf(dz[v])) > edge);
-                            open[v] = in & far;
-                            in = in & (d2[v] < near);
-                        } else {
-                            open[v] = in & far;
-                        }
-                        slot[v] = in & !far ? __float_as_int(qm[v]) - __float_as_int(kRintMagic) : spare;
+                        if (kDiag && t0 + t + v <= i) in = false, sl[h] = top;
+                        if (CHECK) far[h] = far[h] | (fmaxf(fmaxf(fabsf(dx[v]), fabsf(dy[v])), fabsf(dz[v])) > edge);
+                        open[v] = in & far[h];
+                        slot[v] = sl[h];
+                        gr_count(row + 4u * sl[h], kWeight);
                     }
                 }
-#pragma unroll
-                for (int u = 0; u < 4; u++) atomicAdd(&hist[slot[u]], SAME ? 2u : 1u);
                 const bool any = open[0] | open[1] | open[2] | open[3];
                 if (any) {
 #pragma unroll
                     for (int u = 0; u < 4; u++)
-                        if (open[u]) settle(d2[u], dx[u], dy[u], dz[u], t + u);
+                        if (open[u]) settle(slot[u], dx[u], dy[u], dz[u], t + u);
                 }
             }
         };
@@ -722,22 +700,6 @@ float bd_calculate_temp_sine(float T0, float Tf, float t0, float tf, float perio
     return a + bs;
 }
 
-// smallest float x >= 0 whose square root is not below `range` (bisection over
-// the bit patterns of the non-negative floats)
-static float sqrt_threshold(float range) {
-    unsigned lo = 0u, hi = 0x7f800000u;  // +0 .. +inf
-    while (lo < hi) {
-        const unsigned mid = lo + ((hi - lo) >> 1);
-        float x;
-        std::memcpy(&x, &mid, 4);
-        if (!(std::sqrt(x) < range)) hi = mid;
-        else lo = mid + 1;
-    }
-    float x;
-    std::memcpy(&x, &lo, 4);
-    return x;
-}
-
 int bd_get_gder(char type, char type_other, const float *rr, const float *rr_other, unsigned long long *counts,
                 const bd_parametros *p, void *stream) {
     if (!p || (type != 'b' && type != 's') || (type_other != 'b' && type_other != 's') || !counts) return BD_ERR_ARG;
@@ -756,10 +718,7 @@ int bd_get_gder(char type, char type_other, const float *rr, const float *rr_oth
     a.side_inv = (float)(1.0 / a.side);
     a.range = p->range_gder;
     a.range2_hi = a.range * a.range * 1.00001f;
-    a.bin_size = a.range / ((float)nbins);
-    a.inv_bin = 1.0f / a.bin_size;
-    a.thr = sqrt_threshold(a.range);
-    a.nbins = nbins;
+    a.bins = gr_bins(a.range, nbins, 0.0);
     a.counts = counts;
     const bool same = type == type_other;
     // partners per block: enough blocks for 8 of 256 threads on each SM (half
@@ -770,13 +729,13 @@ int bd_get_gder(char type, char type_other, const float *rr, const float *rr_oth
     const long per = ((long)rows * nb / want + 63) / 64 * 64;
     a.jchunk = (int)std::min(8192L, std::max(64L, per));
     a.copies = kGderMaxCopies;  // a power of two
-    while (a.copies > 1 && (size_t)a.copies * (nbins + 32) * sizeof(unsigned) > 32 * 1024) a.copies /= 2;
+    while (a.copies > 1 && (size_t)a.copies * (nbins + kGrSpare) * sizeof(unsigned) > 32 * 1024) a.copies /= 2;
     const dim3 grid(rows, div_up(nb, a.jchunk));
-    const size_t sm = 3 * kGderTile * sizeof(float) + (size_t)a.copies * (nbins + 32) * sizeof(unsigned);
+    const size_t sm = 3 * kGderTile * sizeof(float) + (size_t)a.copies * (nbins + kGrSpare) * sizeof(unsigned);
     cudaStream_t s = as_stream(stream);
     // pairs at the edge of the minimum image may be within range
-    const float edge = 0.489f * a.side;
-    const bool check = !(a.thr <= edge * edge);
+    const float edge = 0.49998f * a.side;
+    const bool check = !(a.bins.near <= edge * edge);
     auto kern = same ? (check ? k_gder<true, true> : k_gder<true, false>)
                      : (check ? k_gder<false, true> : k_gder<false, false>);
     if (sm > 48 * 1024) BD_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));

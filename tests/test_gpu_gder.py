@@ -98,3 +98,21 @@ def test_bin_edges_on_a_lattice_match_oracle(method):
     ref = O.gder_counts(p, snap[: s.n_big], snap[s.n_big:])
     np.testing.assert_array_equal(got, ref)
     assert got.sum() > 0
+
+
+@pytest.mark.parametrize("nb,ns,phi,nbins,range_,method", [
+    (600, 600, 0.5, 1, 1.8, "cells"), (600, 600, 0.5, 4096, 1.8, "cells"), (0, 1500, 0.45, 33, 1.5, "cells"),
+    (7000, 7001, 0.58, 150, 8.0, "cells"), (1, 1, 0.0005, 5, 2.0, "all_pairs"), (257, 255, 0.5, 90, 9.0, "all_pairs"),
+    (300, 213, 0.4, 4096, 4.99, "all_pairs"), (1000, 0, 0.5, 64, 7.0, "all_pairs")])
+def test_counts_at_the_edges_of_the_kernels_match_oracle(nb, ns, phi, nbins, range_, method):
+    # stencils of partial bricks and of the whole box, one species, one bin and
+    # the most bins; all pairs at and beyond L / 2 (ties of the minimum image)
+    # and around a block of particles
+    s, pos = system(nb, ns, phi, 5, force_cap=100.0)
+    e = B.Engine([s])
+    e.set_positions(pos)
+    e.run(3)
+    snap, _ = e.get_positions()
+    got = e.gder(nbins, range_, method=method)[0]
+    p = O.setup_params(s.side, s.n_big, s.n_sml, SB, SS, nbins=nbins, rng=range_)
+    np.testing.assert_array_equal(got, O.gder_counts(p, snap[: s.n_big], snap[s.n_big:]))
