@@ -17,6 +17,8 @@ namespace bd {
 constexpr float kRefPi = 3.14159266f;
 constexpr float kEps = 1.0f;
 
+constexpr float kRintMagic = 12582912.f;  // 1.5 2^23: adding it rounds |x| < 2^22 to an integer
+
 // device status word bits (OR-ed by kernels, read by the host after a call)
 enum : unsigned {
     kStatCellOverflow = 1u,   // a cell or staging buffer exceeded its capacity
@@ -262,7 +264,10 @@ __device__ __forceinline__ float advance_wrap(float &hi, float &lo, float d, flo
     float c = __fadd_rn(lo, e);
     float h2 = __fadd_rn(s, c);
     c = __fsub_rn(c, __fsub_rn(h2, s));
-    float kw = floorf(__fmul_rn(side_inv, h2));
+    // inside the box (nearly always) without the conversion pipe's floor
+    const float t = __fmul_rn(side_inv, h2);
+    float kw = 0.0f;
+    if (!(t >= 0.0f && t < 1.0f)) kw = floorf(t);
     if (kw != 0.0f) {
         float s2, e2;
         two_sum(h2, -__fmul_rn(side, kw), s2, e2);

@@ -117,6 +117,11 @@ int max_active_clusters(bd_engine *e) {
     return n;
 }
 
+auto grid_kernel(const bd_engine *e) {
+    return e->lgr_help ? (e->extra_pot ? k_list_grid<true, true> : k_list_grid<false, true>)
+                       : (e->extra_pot ? k_list_grid<true, false> : k_list_grid<false, false>);
+}
+
 int configure_kernels(bd_engine *e) {
     StepArgs a;
     std::memset(&a, 0, sizeof(a));
@@ -136,6 +141,16 @@ int configure_kernels(bd_engine *e) {
 #undef BD_ATTR
     if (cudaFuncSetAttribute(k_list_build, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)e->lsmem) != cudaSuccess)
         rc = 1;
+    if (e->lgr_blocks > 0 && cudaFuncSetAttribute(grid_kernel(e), cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                  (int)grid_smem_bytes(e->lgr_owners)) != cudaSuccess)
+        rc = 1;
+    if (e->lcl_ctas > 0) {
+        if (cudaFuncSetAttribute(k_list_cluster<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)e->lcl_smem) != cudaSuccess ||
+            cudaFuncSetAttribute(k_list_cluster<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)e->lcl_smem) != cudaSuccess)
+            rc = 1;
+    }
     if (e->lrep_smem > 0) {  // variant 5 rebuilds from shared memory
         if (cudaFuncSetAttribute(k_list_replica<false, 5>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)e->lrep_smem) != cudaSuccess ||
@@ -253,6 +268,8 @@ int launch_list_step(bd_engine *e, const ListArgs &a, int ni_off) {
 bool list_per_replica(const bd_engine *e) {
     return e->list && e->lvar >= kListFirstPersistent && e->rng == BD_RNG_PHILOX;
 }
+// words of the grid barrier, beside the build counters
+unsigned long long *grid_word(bd_engine *e) { return reinterpret_cast<unsigned long long *>(e->d_builds + 3); }
 template <int V>
 int launch_list_replica_v(bd_engine *e, int cur, int nsteps) {
     constexpr int T = ListVariant<V>::kThreads;
@@ -264,12 +281,67 @@ int launch_list_replica_v(bd_engine *e, int cur, int nsteps) {
     if (e->extra_pot) k_list_replica<true, V><<<e->R, T, sm, e->stream>>>(a, lp, e->d_ni, nsteps);
     else k_list_replica<false, V><<<e->R, T, sm, e->stream>>>(a, lp, e->d_ni, nsteps);
     BD_LAUNCH_CHECK();
-    k_list_replica_done<<<1, 256, 0, e->stream>>>(e->lflag, e->R, e->d_step_rebuilt, nsteps, e->d_builds);
+    k_list_replica_done<<<1, 256, 0, e->stream>>>(e->lflag, e->R, e->d_step_rebuilt, nsteps, e->d_builds,
+                                                grid_word(e));
     BD_LAUNCH_CHECK();
     return BD_OK;
 }
-int list_replica_steps(bd_engine *e, int cur, int nsteps) {
+// Variant 0 of small replicas: a cluster per replica runs `nsteps` steps.
+bool list_cluster(const bd_engine *e) {
+    return e->list && e->lvar == 0 && e->lcl_ctas > 0 && e->rng == BD_RNG_PHILOX;
+}
+int launch_list_cluster(bd_engine *e, int cur, int nsteps) {
+    const ListPersist lp{{e->lpos[0], e->lpos[1]}, cur & 1, e->cnt[0], e->pos[0], e->cap, e->nbr, e->nnb,
+                         e->pbuild, e->d_rep_order, e->d_builds, e->d_step_rebuilt, 0};
+    cudaLaunchConfig_t cfg;
+    std::memset(&cfg, 0, sizeof(cfg));
+    cfg.gridDim = dim3(e->R * e->lcl_ctas);
+    cfg.blockDim = dim3(2 * e->lcl_owners);
+    cfg.dynamicSmemBytes = e->lcl_smem;
+    cfg.stream = e->stream;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = e->lcl_ctas;
+    at[0].val.clusterDim.y = 1;
+    at[0].val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    BD_CUDA_TRY(cudaLaunchKernelEx(&cfg, e->extra_pot ? k_list_cluster<true> : k_list_cluster<false>,
+                                   make_largs(e, cur), lp, (const long long *)e->d_ni, nsteps, e->lcl_nmax, e->lcl_cells,
+                                   e->lcl_ctas));
+    k_list_replica_done<<<1, 256, 0, e->stream>>>(e->lflag, e->R, e->d_step_rebuilt, nsteps, e->d_builds,
+                                                grid_word(e));
+    BD_LAUNCH_CHECK();
+    return BD_OK;
+}
+// Variant 0 of mid-size batches: the whole grid runs `nsteps` steps.
+bool list_grid(const bd_engine *e) { return e->list && e->lvar == 0 && e->lgr_blocks > 0 && e->rng == BD_RNG_PHILOX; }
+int launch_list_grid(bd_engine *e, int cur, int nsteps) {
+    const ListPersist lp{{e->lpos[0], e->lpos[1]}, cur & 1, e->cnt[0], e->pos[0], e->cap, e->nbr, e->nnb,
+                         e->pbuild, e->d_rep_order, e->d_builds, e->d_step_rebuilt, 0};
+    cudaLaunchConfig_t cfg;
+    std::memset(&cfg, 0, sizeof(cfg));
+    cfg.gridDim = dim3(e->lgr_blocks);
+    cfg.blockDim = dim3(e->lgr_help ? 2 * e->lgr_owners : e->lgr_owners);
+    cfg.dynamicSmemBytes = grid_smem_bytes(e->lgr_owners);
+    cfg.stream = e->stream;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeCooperative;  // the blocks wait for one another
+    at[0].val.cooperative = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    BD_CUDA_TRY(cudaLaunchKernelEx(&cfg, grid_kernel(e), make_largs(e, cur), lp, (const long long *)e->d_ni, nsteps,
+                                   grid_word(e)));
+    k_list_replica_done<<<1, 256, 0, e->stream>>>(e->lflag, e->R, e->d_step_rebuilt, nsteps, e->d_builds, grid_word(e));
+    BD_LAUNCH_CHECK();
+    return BD_OK;
+}
+// launches of a whole batch of steps
+bool list_batched(const bd_engine *e) { return list_per_replica(e) || list_cluster(e) || list_grid(e); }
+int list_batch_steps(bd_engine *e, int cur, int nsteps) {
     if (nsteps > e->graph_steps) return BD_ERR_ARG;  // the amplitude table holds one batch
+    if (list_cluster(e)) return launch_list_cluster(e, cur, nsteps);
+    if (list_grid(e)) return launch_list_grid(e, cur, nsteps);
     switch (e->lvar) {
         case 3: return launch_list_replica_v<3>(e, cur, nsteps);
         case 4: return launch_list_replica_v<4>(e, cur, nsteps);
@@ -326,8 +398,8 @@ int direct_steps(bd_engine *e, int k) {
     if (e->list) {
         if (k > e->graph_steps) return BD_ERR_ARG;  // the amplitude table holds one batch
         if (int rc = list_amplitudes(e, k)) return rc;
-        if (list_per_replica(e)) {
-            if (int rc = list_replica_steps(e, e->cur, k)) return rc;
+        if (list_batched(e)) {
+            if (int rc = list_batch_steps(e, e->cur, k)) return rc;
         } else {
             for (int i = 0; i < k; i++) {
                 int rc = list_step(e, e->cur + i, i);
@@ -359,7 +431,7 @@ int build_graph(bd_engine *e) {
     int rc = BD_OK;
     if (e->list) {
         rc = list_amplitudes(e, e->graph_steps);
-        if (rc == BD_OK && list_per_replica(e)) rc = list_replica_steps(e, e->cur, e->graph_steps);
+        if (rc == BD_OK && list_batched(e)) rc = list_batch_steps(e, e->cur, e->graph_steps);
         else
             for (int j = 0; j < e->graph_steps && rc == BD_OK; j++) rc = list_step(e, e->cur + j, j);
     } else if (e->mode == BD_MODE_PERSISTENT) {
@@ -457,6 +529,39 @@ int rebuild_bricks(bd_engine *e) {
         e->nclusters = G;
     }
     return BD_OK;
+}
+
+// Variant 0 runs small replicas in clusters (nlist_cluster.cuh): the most CTAs
+// per replica (up to 8) that leave every replica resident at once, one thread
+// per particle; and other batches of up to 512 particles per SM on the whole
+// grid (nlist_grid.cuh).  Larger ones keep the per-step kernels.
+void choose_resident(bd_engine *e) {
+    int nmax = 0, cmax = 0;
+    for (const SysDev &S : e->sysh) {
+        nmax = std::max(nmax, S.n);
+        cmax = std::max(cmax, S.ncell * S.ncell * S.ncell);
+    }
+    for (int C = kClusterMaxCtas; C >= 1; C /= 2) {
+        const int T = std::max(32, (div_up(nmax, C) + 31) / 32 * 32);
+        const size_t sm = cluster_smem_bytes(nmax, cmax, T);
+        if ((long long)e->R * C > 148 || T > kClusterMaxOwners || sm > (size_t)226 * 1024) continue;
+        e->lcl_ctas = C;
+        e->lcl_owners = T;
+        e->lcl_smem = sm;
+        e->lcl_nmax = nmax;
+        e->lcl_cells = cmax;
+        return;
+    }
+    // Batches of up to 512 particles per SM: the whole grid resident, 128
+    // particles per block until every SM has one
+    int sms = 0, coop = 0;
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, e->dev);
+    cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, e->dev);
+    if (!coop || e->P > (long long)sms * kGridMaxOwners) return;
+    const int G = std::min(sms, div_up(e->P, 128));
+    e->lgr_owners = (div_up(e->P, G) + 31) / 32 * 32;
+    e->lgr_help = 2 * e->lgr_owners <= kGridMaxOwners;
+    e->lgr_blocks = G;
 }
 
 // Upload the brick layout (after rebuild_bricks) and drop graphs recorded
@@ -665,8 +770,8 @@ int bd_engine_create(const bd_system_desc *systems, int nsys, const bd_engine_op
         ALLOC(e->amp_tab, sizeof(float) * 2 * (size_t)e->R * e->graph_steps);
         ALLOC(e->lflag, sizeof(int) * (e->R + 1));
         ALLOC(e->d_one, sizeof(int));
-        ALLOC(e->d_builds, 3 * sizeof(long long));  // + the build's finished-block counter
-        cudaMemsetAsync(e->d_builds, 0, 3 * sizeof(long long), e->stream);
+        ALLOC(e->d_builds, 5 * sizeof(long long));  // + the build's finished-block counter, the grid barrier's words
+        cudaMemsetAsync(e->d_builds, 0, 5 * sizeof(long long), e->stream);
         ALLOC(e->d_step_rebuilt, sizeof(int) * e->graph_steps);
         cudaMemsetAsync(e->d_step_rebuilt, 0, sizeof(int) * e->graph_steps, e->stream);
         ALLOC(e->d_rep_order, sizeof(int) * e->R);
@@ -682,6 +787,7 @@ int bd_engine_create(const bd_system_desc *systems, int nsys, const bd_engine_op
                 need = std::max(need, replica_shared_build_bytes(S.n, S.ncell * S.ncell * S.ncell));
             }
             e->lrep_smem = need <= (size_t)227 * 1024 ? need : 0;
+            choose_resident(e);
             cudaStreamSynchronize(e->stream);  // the host vector goes out of scope
         }
         const int one = 1;
@@ -845,7 +951,7 @@ namespace {
 // Steps issued directly (no graph): one persistent launch, or k plain launches.
 int run_direct(bd_engine *e, int k) {
     if (k <= 0) return BD_OK;
-    if (e->mode == BD_MODE_PERSISTENT) return direct_steps(e, k);
+    if (e->mode == BD_MODE_PERSISTENT || list_batched(e)) return direct_steps(e, k);
     for (int i = 0; i < k; i++) {
         int rc = direct_steps(e, 1);
         if (rc) return rc;
@@ -860,7 +966,8 @@ int run_direct(bd_engine *e, int k) {
 // List mode, in two stages, on the live batch with rebuilds as they come:
 // 1. the list-build brick shape and the per-step launch variant (0-2), each
 //    pair over 2 + 12 steps launched one by one;
-// 2. the winner of stage 1 against the per-replica variants (3-5), each over
+// 2. the winner of stage 1 against the variants that run a whole batch in one
+//    launch (3-5, and 0 where it does), each over
 //    one whole graph batch (graph_steps steps, graph instantiated before the
 //    timer starts) after 2 warm-up steps: a per-replica launch pays each
 //    block's cold start and in-block rebuilds once per launch, so a
@@ -876,6 +983,10 @@ int autotune_list(bd_engine *e, long long &nsteps) {
         if (!(e->tune_lvar || v == e->lvar)) continue;
         if (v >= kListFirstPersistent) {  // builds its lists in the block: no brick shape to choose
             if (e->rng == BD_RNG_PHILOX) stage2.push_back({e->bx, e->by, e->bz, v});
+            continue;
+        }
+        if (v == 0 && (e->lcl_ctas > 0 || e->lgr_blocks > 0)) {
+            stage2.push_back({e->bx, e->by, e->bz, v});
             continue;
         }
         for (auto &sh : shapes) stage1.push_back({sh[0], sh[1], sh[2], v});

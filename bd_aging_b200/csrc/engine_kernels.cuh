@@ -108,6 +108,8 @@ __device__ __forceinline__ double block_sum(double v, double *red) {
 }  // namespace bd
 #include "step.cuh"
 #include "nlist.cuh"
+#include "nlist_cluster.cuh"
+#include "nlist_grid.cuh"
 namespace bd {
 
 __global__ void k_advance_counter(long long *ni_base, int k) { *ni_base += k; }

@@ -84,6 +84,13 @@ struct bd_engine {
     float *amp_tab = nullptr;       // [graph_steps][R][2] noise amplitudes of a launch batch
     int *d_rep_order = nullptr;     // per-replica launch (variants 3-5): replica of each block
     size_t lrep_smem = 0;           // variant 5: shared memory of an in-block rebuild (0: from global memory)
+    // variant 0 in clusters (0 CTAs: the per-step kernels): CTAs per replica, the particles each owns at
+    // most, their shared memory, the largest replica's particles and cells
+    int lcl_ctas = 0, lcl_owners = 0, lcl_nmax = 0, lcl_cells = 0;
+    size_t lcl_smem = 0;
+    // variant 0 on the whole grid (0 blocks: not used): blocks, particles each owns at most, helper threads
+    int lgr_blocks = 0, lgr_owners = 0;
+    bool lgr_help = false;
     int *d_step_rebuilt = nullptr;  // [graph_steps] steps of such a launch that rebuilt a replica
     // set_positions scratch (storage order computed on the device)
     float *ld_in = nullptr;        // [P][3] positions as given

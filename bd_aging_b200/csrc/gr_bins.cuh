@@ -21,7 +21,6 @@
 
 namespace bd {
 
-constexpr float kRintMagic = 12582912.f;  // 1.5 2^23: adding it rounds |x| < 2^22 to an integer
 constexpr float kGrC1 = 1e-6f;
 
 struct GrBins {

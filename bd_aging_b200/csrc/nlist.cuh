@@ -25,6 +25,7 @@
 // (cnt / pos of buffer 0) are rebuilt from the by-id positions for list
 // builds and observation passes.
 #pragma once
+#include <type_traits>
 
 namespace bd {
 
@@ -331,26 +332,30 @@ __device__ __forceinline__ T ld_state(const T *p) {
     else return *p;
 }
 
-// list words k0 .. k0 + kGather - 1 (k0 < kMaxNbr)
-template <bool NC = true>
-__device__ __forceinline__ void list_words(const ListArgs &a, int sid, int k0, int (&jn)[kGather]) {
-    const int4 w = ld_state<NC>(reinterpret_cast<const int4 *>(a.nbr) + (size_t)(k0 >> 2) * a.np + sid);
-    jn[0] = w.x;
-    jn[1] = w.y;
-    jn[2] = w.z;
-    jn[3] = w.w;
-}
-// positions of the chunk's partners: an entry outside [0, np) reads the zero
-// position at np and counts as absent (jj = np)
-template <bool NC = true>
-__device__ __forceinline__ void gather_chunk(const ListArgs &a, const int (&jn)[kGather], int (&jj)[kGather],
-                                             float4 (&pj)[kGather]) {
-#pragma unroll
-    for (int u = 0; u < kGather; u++) {
-        jj[u] = (int)min((unsigned)jn[u], (unsigned)a.np);
-        pj[u] = ld_state<NC>(a.pos_in + jj[u]);
+// Where a particle's list and its partners' positions are read.  words():
+// list words k0 .. k0 + kGather - 1 (k0 < kMaxNbr); gather(): the positions of
+// those partners, an entry outside [0, none) reading the zero position at
+// `none` and counting as absent (jj = none).
+template <bool NC>
+struct ListGlobal {  // lists and by-id positions in global memory; entries are storage ids
+    const ListArgs &a;
+    int sid, none;
+    __device__ __forceinline__ ListGlobal(const ListArgs &a_, int sid_) : a(a_), sid(sid_), none(a_.np) {}
+    __device__ __forceinline__ void words(int k0, int (&jn)[kGather]) const {
+        const int4 w = ld_state<NC>(reinterpret_cast<const int4 *>(a.nbr) + (size_t)(k0 >> 2) * a.np + sid);
+        jn[0] = w.x;
+        jn[1] = w.y;
+        jn[2] = w.z;
+        jn[3] = w.w;
     }
-}
+    __device__ __forceinline__ void gather(const int (&jn)[kGather], int (&jj)[kGather], float4 (&pj)[kGather]) const {
+#pragma unroll
+        for (int u = 0; u < kGather; u++) {
+            jj[u] = (int)min((unsigned)jn[u], (unsigned)a.np);
+            pj[u] = ld_state<NC>(a.pos_in + jj[u]);
+        }
+    }
+};
 
 // The reference's minimum image d - L floor(d / L + 1/2) (get_forces.cu)
 // of two list partners at once.  A list partner lies within cut + 2 skin of
@@ -361,10 +366,11 @@ __device__ __forceinline__ void gather_chunk(const ListArgs &a, const int (&jn)[
 // fma(k, -L, d) is the reference's rounded difference.  (A pair whose
 // quotient lay near a half integer would sit near L / 2, beyond every cut
 // distance, and fail the cut test with either rounding.)
+// rint of |x| < 2^22 by adding and subtracting 1.5 2^23: two additions on the
+// FMA pipe, where rintf takes the conversion pipe (a quarter of its rate).
 __device__ __forceinline__ f2 min_image_pair(f2 d, f2 linv, f2 neg_l) {
-    float ta, tb;
-    f2_split(f2_mul(d, linv), ta, tb);
-    return f2_fma(f2_make(rintf(ta), rintf(tb)), neg_l, d);
+    const f2 magic = f2_bcast(kRintMagic);
+    return f2_fma(f2_sub(f2_add(f2_mul(d, linv), magic), magic), neg_l, d);
 }
 
 // Modified-WCA force on one particle from its list, two partners per f32x2
@@ -374,22 +380,21 @@ __device__ __forceinline__ f2 min_image_pair(f2 d, f2 linv, f2 neg_l) {
 // around the particle and the minimum image would return the plain
 // difference.  The force is summed in two interleaved partial sums (even and
 // odd list positions) that are added at the end.
-template <bool WRAP, bool NC = true>
-__device__ __forceinline__ void list_forces_wca(const ListArgs &a, int sid, int n, float4 pi, float L, float Linv,
-                                                float sg0, float sg1, float c0, float c1, float &fx, float &fy,
-                                                float &fz) {
+template <bool WRAP, class SRC>
+__device__ __forceinline__ void list_forces_wca(const SRC &src, int n, float4 pi, float L, float Linv, float sg0,
+                                                float sg1, float c0, float c1, float &fx, float &fy, float &fz) {
     const f2 PX = f2_bcast(pi.x), PY = f2_bcast(pi.y), PZ = f2_bcast(pi.z), M12 = f2_bcast(-12.0f);
     const float sq0 = sg0 * sg0, sq1 = sg1 * sg1;
     const f2 LINV = f2_bcast(Linv), NEGL = f2_bcast(-L);
     f2 FX = 0ull, FY = 0ull, FZ = 0ull;  // (0.f, 0.f)
-    const int np = a.np;
+    const int np = src.none;
     int jn[kGather];
-    if (n > 0) list_words<NC>(a, sid, 0, jn);
+    if (n > 0) src.words(0, jn);
     for (int k0 = 0; k0 < n; k0 += kGather) {
         int jj[kGather];
         float4 pj[kGather];
-        gather_chunk<NC>(a, jn, jj, pj);
-        if (k0 + kGather < n) list_words<NC>(a, sid, k0 + kGather, jn);
+        src.gather(jn, jj, pj);
+        if (k0 + kGather < n) src.words(k0 + kGather, jn);
 #pragma unroll
         for (int u = 0; u < kGather; u += 2) {
             const float4 qa = pj[u], qb = pj[u + 1];
@@ -401,8 +406,9 @@ __device__ __forceinline__ void list_forces_wca(const ListArgs &a, int sid, int 
                 dY = min_image_pair(dY, LINV, NEGL);
                 dZ = min_image_pair(dZ, LINV, NEGL);
             }
-            // dist2_rn in each lane
-            const f2 D2 = f2_add(f2_add(f2_mul(dX, dX), f2_mul(dY, dY)), f2_mul(dZ, dZ));
+            // squared distances with fused sums, written out: the compiler fuses
+            // packed products and sums on its own, and every kernel has to round alike
+            const f2 D2 = f2_fma(dZ, dZ, f2_fma(dX, dX, f2_mul(dY, dY)));
             float d2a, d2b;
             f2_split(D2, d2a, d2b);
             const bool ta = (__float_as_uint(qa.w) >> 31) != 0u, tb = (__float_as_uint(qb.w) >> 31) != 0u;
@@ -441,23 +447,23 @@ __device__ __forceinline__ void list_forces_wca(const ListArgs &a, int sid, int 
 
 // Force from the list for a replica with another potential of PotKind
 // (scalar, list order).
-template <bool NC = true>
-__device__ __forceinline__ void list_forces_extra(const ListArgs &a, const SysDev &S, int sid, int n, float4 pi, int tm,
-                                               float &fx, float &fy, float &fz) {
+template <class SRC>
+__device__ __forceinline__ void list_forces_extra(const SRC &src, const SysDev &S, int n, float4 pi, int tm, float &fx,
+                                                  float &fy, float &fz) {
     const float L = S.L, Linv = S.Linv;
     const float sg0 = tm ? S.sig[1] : S.sig[0], sg1 = tm ? S.sig[2] : S.sig[1];
     const float c0 = tm ? S.cut2[1] : S.cut2[0], c1 = tm ? S.cut2[2] : S.cut2[1];
     fx = fy = fz = 0.f;
     int jn[kGather];
-    if (n > 0) list_words<NC>(a, sid, 0, jn);
+    if (n > 0) src.words(0, jn);
     for (int k0 = 0; k0 < n; k0 += kGather) {
         int jj[kGather];
         float4 pj[kGather];
-        gather_chunk<NC>(a, jn, jj, pj);
-        if (k0 + kGather < n) list_words<NC>(a, sid, k0 + kGather, jn);
+        src.gather(jn, jj, pj);
+        if (k0 + kGather < n) src.words(k0 + kGather, jn);
 #pragma unroll
         for (int u = 0; u < kGather; u++) {
-            if (jj[u] == a.np) continue;
+            if (jj[u] == src.none) continue;
             const float dx = min_image_fast(__fsub_rn(pj[u].x, pi.x), L, Linv);
             const float dy = min_image_fast(__fsub_rn(pj[u].y, pi.y), L, Linv);
             const float dz = min_image_fast(__fsub_rn(pj[u].z, pi.z), L, Linv);
@@ -476,35 +482,18 @@ __device__ __forceinline__ void list_forces_extra(const ListArgs &a, const SysDe
     }
 }
 
-// One time step of particle sid from its list: force sum in list order;
-// update, compensated position and FP64 displacement exactly as
-// process_brick.  Returns true when the particle has moved more than half
-// the skin since the last build (its replica's lists must be rebuilt).
-// EXTRA: some replica of the batch uses a potential other than the modified
-// WCA (instantiated separately so the default kernel keeps its registers).
-// LATE: the particle's own state is loaded after the force loop.  NC: loads
-// through the read-only path (ld_state).
-template <int RNG, bool EXTRA, bool LATE, bool NC>
-__device__ __forceinline__ bool list_particle_step(const ListArgs &a, int sid, int rep, long long ni, int ni_off) {
-    const SysDev &S = a.sys[rep];
+// Force on a particle from its list of n partners, capped for the initial
+// relaxation.  EXTRA: some replica of the batch uses a potential other than
+// the modified WCA (instantiated separately so the default kernel keeps its
+// registers).  Called by whole warps less those past the last particle.
+template <bool EXTRA, class SRC>
+__device__ __forceinline__ void list_force(const SRC &src, const SysDev &S, int n, float4 pi, int tm, float &fx,
+                                           float &fy, float &fz) {
     const float L = S.L, Linv = S.Linv;
-    const float4 pi = a.pos_in[sid];
-    const unsigned wi = __float_as_uint(pi.w);
-    const int tm = (int)(wi >> 31);
     const float sg0 = tm ? S.sig[1] : S.sig[0], sg1 = tm ? S.sig[2] : S.sig[1];
     const float c0 = tm ? S.cut2[1] : S.cut2[0], c1 = tm ? S.cut2[2] : S.cut2[1];
-    int gid;
-    float lx, ly, lz;
-    float4 pb;
-    if constexpr (!LATE) {  // own state early: its latency overlaps the force loop
-        gid = __ldg(a.gid_of + sid);
-        lx = a.lo_x[sid], ly = a.lo_y[sid], lz = a.lo_z[sid];
-        pb = ld_state<NC>(a.pbuild + sid);
-    }
-    float fx, fy, fz;
-    const int n = min(ld_state<NC>(a.nnb + sid), kMaxNbr);
     if (EXTRA && S.pot != kPotWcaModified) {
-        list_forces_extra<NC>(a, S, sid, n, pi, tm, fx, fy, fz);
+        list_forces_extra(src, S, n, pi, tm, fx, fy, fz);
     } else {  // the same arithmetic in either instantiation: a replica's result does not depend on its batch
         // a warp whose particles all sit away from the faces needs no
         // minimum image for any partner
@@ -512,9 +501,9 @@ __device__ __forceinline__ bool list_particle_step(const ListArgs &a, int sid, i
         const bool inner = pi.x >= lo_edge && pi.x <= hi_edge && pi.y >= lo_edge && pi.y <= hi_edge &&
                            pi.z >= lo_edge && pi.z <= hi_edge;
         if (__all_sync(__activemask(), inner))
-            list_forces_wca<false, NC>(a, sid, n, pi, L, Linv, sg0, sg1, c0, c1, fx, fy, fz);
+            list_forces_wca<false>(src, n, pi, L, Linv, sg0, sg1, c0, c1, fx, fy, fz);
         else
-            list_forces_wca<true, NC>(a, sid, n, pi, L, Linv, sg0, sg1, c0, c1, fx, fy, fz);
+            list_forces_wca<true>(src, n, pi, L, Linv, sg0, sg1, c0, c1, fx, fy, fz);
     }
     if (S.fcap > 0.f) {  // capped forces for the initial relaxation
         const float fmx = fmaxf(fabsf(fx), fmaxf(fabsf(fy), fabsf(fz)));
@@ -529,6 +518,45 @@ __device__ __forceinline__ bool list_particle_step(const ListArgs &a, int sid, i
             fx = fy = fz = 0.f;
         }
     }
+}
+
+// Whether a particle at (x, y, z) has left half the skin around its build
+// position pb: the minimum image as in min_image_pair (a displacement near
+// L / 2 raises the flag with either rounding of the image).
+__device__ __forceinline__ bool list_beyond(float x, float y, float z, float4 pb, float L, float Linv,
+                                            float skin_half2) {
+    const float dbx = __fsub_rn(x, pb.x), dby = __fsub_rn(y, pb.y), dbz = __fsub_rn(z, pb.z);
+    auto image = [&](float d) {
+        return fmaf(__fsub_rn(__fadd_rn(__fmul_rn(Linv, d), kRintMagic), kRintMagic), -L, d);
+    };
+    const float bx = image(dbx), by = image(dby), bz = image(dbz);
+    return !(dist2_rn(bx, by, bz) <= skin_half2);
+}
+
+// One time step of particle sid from its list: force sum in list order;
+// update, compensated position and FP64 displacement exactly as
+// process_brick.  Returns true when the particle has moved more than half
+// the skin since the last build (its replica's lists must be rebuilt).
+// LATE: the particle's own state is loaded after the force loop.  NC: loads
+// through the read-only path (ld_state).
+template <int RNG, bool EXTRA, bool LATE, bool NC>
+__device__ __forceinline__ bool list_particle_step(const ListArgs &a, int sid, int rep, long long ni, int ni_off) {
+    const SysDev &S = a.sys[rep];
+    const float L = S.L, Linv = S.Linv;
+    const float4 pi = a.pos_in[sid];
+    const unsigned wi = __float_as_uint(pi.w);
+    const int tm = (int)(wi >> 31);
+    int gid;
+    float lx, ly, lz;
+    float4 pb;
+    if constexpr (!LATE) {  // own state early: its latency overlaps the force loop
+        gid = __ldg(a.gid_of + sid);
+        lx = a.lo_x[sid], ly = a.lo_y[sid], lz = a.lo_z[sid];
+        pb = ld_state<NC>(a.pbuild + sid);
+    }
+    float fx, fy, fz;
+    const int n = min(ld_state<NC>(a.nnb + sid), kMaxNbr);
+    list_force<EXTRA>(ListGlobal<NC>(a, sid), S, n, pi, tm, fx, fy, fz);
     if constexpr (LATE) {
         gid = __ldg(a.gid_of + sid);
         lx = a.lo_x[sid], ly = a.lo_y[sid], lz = a.lo_z[sid];
@@ -576,14 +604,7 @@ __device__ __forceinline__ bool list_particle_step(const ListArgs &a, int sid, i
     a.lo_z[sid] = lz;
     if (!(isfinite(x) && isfinite(y) && isfinite(z))) set_status(a.status, kStatNumeric);
     a.pos_out[sid] = make_float4(x, y, z, pi.w);
-    // skin check against the positions at the last build: the minimum image
-    // as in min_image_pair (a displacement near L / 2 raises the flag with
-    // either rounding of the image)
-    const float dbx = __fsub_rn(x, pb.x), dby = __fsub_rn(y, pb.y), dbz = __fsub_rn(z, pb.z);
-    const float bx = fmaf(rintf(__fmul_rn(Linv, dbx)), -L, dbx);
-    const float by = fmaf(rintf(__fmul_rn(Linv, dby)), -L, dby);
-    const float bz = fmaf(rintf(__fmul_rn(Linv, dbz)), -L, dbz);
-    return !(dist2_rn(bx, by, bz) <= S.skin_half2);
+    return list_beyond(x, y, z, pb, L, Linv, S.skin_half2);
 }
 
 // One time step of every particle (thread per storage id); a particle beyond
@@ -633,6 +654,12 @@ __device__ __forceinline__ int3 list_cell_of(const float4 v, const SysDev &S) {
     int ix = (int)__fmul_rn(v.x, S.cinv), iy = (int)__fmul_rn(v.y, S.cinv), iz = (int)__fmul_rn(v.z, S.cinv);
     return make_int3(min(max(ix, 0), nc - 1), min(max(iy, 0), nc - 1), min(max(iz, 0), nc - 1));
 }
+// Squared distance of a list build as the staged sweep rounds it (sweep_row):
+// fused in rows of cells away from the faces, every operation rounded in rows
+// that cross one.
+__device__ __forceinline__ float list_build_d2(float ex, float ey, float ez, bool wrap) {
+    return wrap ? dist2_rn(ex, ey, ez) : __fmaf_rn(ez, ez, __fmaf_rn(ex, ex, __fmul_rn(ey, ey)));
+}
 // neighbour cell index along one axis (periodic) and the staged sweep's
 // shift of its particles (+L when the cell wrapped below 0, -L above nc - 1)
 __device__ __forceinline__ int wrap_cell(int g, int nc, float L, float &shift) {
@@ -658,18 +685,14 @@ struct CellsGlobal {
 struct CellsShared {
     const int *start;  // [cells + 1]
     const float4 *pos;
-    __device__ __forceinline__ const float4 *cell(int c, int &m) const {
-        m = start[c + 1] - start[c];
-        return pos + start[c];
-    }
 };
 
-// List of particle sid from the sorted cells of its replica.
-template <class CELLS>
-__device__ __forceinline__ void replica_list(const ListArgs &a, const ListPersist &lp, const SysDev &S, int sid,
-                                             const CELLS &cells) {
-    const float4 v = a.pos_in[sid];
-    const int np = a.np, nc = S.ncell;
+// Partners of the particle at v from the sorted cells of its replica:
+// emit(k, storage id) for the k-th; returns their number.
+template <class EMIT>
+__device__ __forceinline__ int replica_partners(const SysDev &S, float4 v, const CellsGlobal &cells, EMIT emit) {
+    const int nc = S.ncell;
+    const int sid = (int)(__float_as_uint(v.w) & 0x7fffffffu);
     const int tm = (int)(__float_as_uint(v.w) >> 31);
     const float cut_b = S.lcut2[tm], cut_s = S.lcut2[tm + 1];  // towards a big / a small partner
     const float L = S.L;
@@ -681,6 +704,7 @@ __device__ __forceinline__ void replica_list(const ListArgs &a, const ListPersis
         for (int dy = -1; dy <= 1; dy++) {
             float shy;
             const int gy = wrap_cell(c.y + dy, nc, L, shy);
+            const bool wrap = c.x == 0 || c.x == nc - 1 || shy != 0.f || shz != 0.f;
             for (int dx = -1; dx <= 1; dx++) {
                 float shx;
                 const int gx = wrap_cell(c.x + dx, nc, L, shx);
@@ -694,15 +718,85 @@ __device__ __forceinline__ void replica_list(const ListArgs &a, const ListPersis
                     const float ex = __fsub_rn(__fsub_rn(q.x, v.x), shx);
                     const float ey = __fsub_rn(__fsub_rn(q.y, v.y), shy);
                     const float ez = __fsub_rn(__fsub_rn(q.z, v.z), shz);
-                    if (dist2_rn(ex, ey, ez) < ((wq >> 31) ? cut_s : cut_b)) {
-                        if (cnt < kMaxNbr) lp.nbr[list_slot(cnt, sid, np)] = sj;
-                        else set_status(a.status, kStatCellOverflow);
+                    if (list_build_d2(ex, ey, ez, wrap) < ((wq >> 31) ? cut_s : cut_b)) {
+                        emit(cnt, sj);
                         cnt++;
                     }
                 }
             }
         }
     }
+    return cnt;
+}
+// The same from the cell-sorted copy in shared memory, rows row0 .. row1 - 1 of
+// its nine (dz, dy), where the three cells
+// of a row are one run of positions (two where the row crosses a face).  A
+// row's candidates are tested four at a time into a bit mask, and the hits
+// written after it: with a branch and a store per candidate a block of 128
+// particles took 50000 cycles (each lane waiting for the others' cells and
+// hits), now 22000, and 11000 with its rows shared by two threads.
+template <class EMIT>
+__device__ __forceinline__ int replica_partners(const SysDev &S, float4 v, const CellsShared &cells, int row0, int row1,
+                                                EMIT emit) {
+    const int nc = S.ncell;
+    const unsigned self = __float_as_uint(v.w) & 0x7fffffffu;
+    const int tm = (int)(__float_as_uint(v.w) >> 31);
+    const float cut_b = S.lcut2[tm], cut_s = S.lcut2[tm + 1];  // towards a big / a small partner
+    const float L = S.L;
+    const int3 c = list_cell_of(v, S);
+    const bool low = c.x == 0, high = c.x == nc - 1;
+    int cnt = 0;
+#pragma unroll 1
+    for (int row = row0; row < row1; row++) {
+        float shy, shz;
+        const int gz = wrap_cell(c.z + row / 3 - 1, nc, L, shz), gy = wrap_cell(c.y + row % 3 - 1, nc, L, shy);
+        const int *start = cells.start + nc * (gy + nc * gz);
+        // runs [a0, a0 + n0) at shift s0, then [a1, ..) at shift s1
+        const int a0 = start[low ? nc - 1 : c.x - 1], e0 = start[low ? nc : min(c.x + 2, nc)];
+        const int a1 = start[0], e1 = low ? start[2] : high ? start[1] : a1;
+        const float s0 = low ? L : 0.f, s1 = high ? -L : 0.f;
+        const int n0 = e0 - a0, total = n0 + (e1 - a1);
+        const bool wrap = low || high || shy != 0.f || shz != 0.f;
+        for (int t0 = 0; t0 < total; t0 += 32) {
+            unsigned hits = 0;
+            const int stop = min(32, total - t0);
+            for (int t = 0; t < stop; t += 4) {
+#pragma unroll
+                for (int u = 0; u < 4; u++) {
+                    const int k = min(t0 + t + u, total - 1);
+                    const bool first = k < n0;
+                    const float4 q = cells.pos[first ? a0 + k : a1 + k - n0];
+                    const unsigned w = __float_as_uint(q.w);
+                    const float ex = __fsub_rn(__fsub_rn(q.x, v.x), first ? s0 : s1);
+                    const float ey = __fsub_rn(__fsub_rn(q.y, v.y), shy);
+                    const float ez = __fsub_rn(__fsub_rn(q.z, v.z), shz);
+                    const bool hit = (list_build_d2(ex, ey, ez, wrap) < ((w >> 31) ? cut_s : cut_b)) & (t + u < stop) &
+                                     ((w & 0x7fffffffu) != self);
+                    hits |= (hit ? 1u : 0u) << (t + u);
+                }
+            }
+            for (; hits; hits &= hits - 1u) {
+                const int k = t0 + __ffs(hits) - 1;
+                emit(cnt, (int)(__float_as_uint(cells.pos[k < n0 ? a0 + k : a1 + k - n0].w) & 0x7fffffffu));
+                cnt++;
+            }
+        }
+    }
+    return cnt;
+}
+// List of particle sid from the sorted cells of its replica.
+template <class CELLS>
+__device__ __forceinline__ void replica_list(const ListArgs &a, const ListPersist &lp, const SysDev &S, int sid,
+                                             const CELLS &cells) {
+    const float4 v = a.pos_in[sid];
+    const int np = a.np;
+    auto emit = [&](int k, int sj) {
+        if (k < kMaxNbr) lp.nbr[list_slot(k, sid, np)] = sj;
+        else set_status(a.status, kStatCellOverflow);
+    };
+    int cnt;
+    if constexpr (std::is_same_v<CELLS, CellsShared>) cnt = replica_partners(S, v, cells, 0, 9, emit);
+    else cnt = replica_partners(S, v, cells, emit);
     const int nl = min(cnt, kMaxNbr);
     for (int k = nl; k < kMaxNbr && (k % kGather) != 0; k++) lp.nbr[list_slot(k, sid, np)] = np;
     lp.nnb[sid] = nl;
@@ -753,24 +847,21 @@ __host__ __device__ inline size_t replica_shared_build_bytes(int n, int c) {
     return (((size_t)(2 * c + 1) * 4 + 15) & ~(size_t)15) + (size_t)n * 16;
 }
 
-// The same lists as replica_rebuild, from a compact copy of the replica
-// sorted by cell (a counting sort, then each cell by storage id) in the
-// block's dynamic shared memory `dsm` (replica_shared_build_bytes).  Cells
-// above the bucket capacity raise the overflow status as the bucket build
-// does.
-__device__ __forceinline__ void replica_rebuild_shared(const ListArgs &a, const ListPersist &lp, const SysDev &S,
-                                                       unsigned char *dsm) {
+// Positions at(0 .. n - 1) of replica S sorted by cell (a counting sort, then
+// each cell by storage id) into s_pos by the whole block: s_start [cells + 1],
+// s_fill [cells].  Cells above the bucket capacity `cap` raise the overflow
+// status as the bucket build does.  Ends with a block barrier.
+template <class AT>
+__device__ __forceinline__ void replica_sort(const SysDev &S, AT at, int cap, unsigned *status, int *s_start,
+                                             int *s_fill, float4 *s_pos) {
     const int tid = threadIdx.x, T = blockDim.x, lane = tid & 31, warp = tid >> 5;
     const int nc = S.ncell, ncell = nc * nc * nc;
-    const int base = S.part_base, n = S.n;
-    int *s_start = reinterpret_cast<int *>(dsm);  // [ncell + 1]
-    int *s_fill = s_start + ncell + 1;            // [ncell]
-    float4 *s_pos = reinterpret_cast<float4 *>(dsm + (((size_t)(2 * ncell + 1) * 4 + 15) & ~(size_t)15));
+    const int n = S.n;
     __shared__ int s_warp[32];
     for (int c = tid; c < ncell; c += T) s_fill[c] = 0;
     __syncthreads();
     for (int i = tid; i < n; i += T) {
-        const int3 c = list_cell_of(a.pos_in[base + i], S);
+        const int3 c = list_cell_of(at(i), S);
         atomicAdd(&s_fill[c.x + nc * (c.y + nc * c.z)], 1);
     }
     __syncthreads();
@@ -799,7 +890,7 @@ __device__ __forceinline__ void replica_rebuild_shared(const ListArgs &a, const 
     int run = incl - local + (warp > 0 ? s_warp[warp - 1] : 0);
     for (int c = c0; c < c1; c++) {
         const int k = s_fill[c];
-        if (k > lp.cap) set_status(a.status, kStatCellOverflow);
+        if (k > cap) set_status(status, kStatCellOverflow);
         s_start[c] = run;
         s_fill[c] = run;
         run += k;
@@ -807,7 +898,7 @@ __device__ __forceinline__ void replica_rebuild_shared(const ListArgs &a, const 
     if (tid == 0) s_start[ncell] = n;
     __syncthreads();
     for (int i = tid; i < n; i += T) {
-        const float4 v = a.pos_in[base + i];
+        const float4 v = at(i);
         const int3 c = list_cell_of(v, S);
         s_pos[atomicAdd(&s_fill[c.x + nc * (c.y + nc * c.z)], 1)] = v;
     }
@@ -828,8 +919,19 @@ __device__ __forceinline__ void replica_rebuild_shared(const ListArgs &a, const 
         }
     }
     __syncthreads();
+}
+
+// The same lists as replica_rebuild, from a compact sorted copy of the replica
+// in the block's dynamic shared memory `dsm` (replica_shared_build_bytes).
+__device__ __forceinline__ void replica_rebuild_shared(const ListArgs &a, const ListPersist &lp, const SysDev &S,
+                                                       unsigned char *dsm) {
+    const int ncell = S.ncell * S.ncell * S.ncell, base = S.part_base;
+    int *s_start = reinterpret_cast<int *>(dsm);  // [ncell + 1]
+    int *s_fill = s_start + ncell + 1;            // [ncell]
+    float4 *s_pos = reinterpret_cast<float4 *>(dsm + (((size_t)(2 * ncell + 1) * 4 + 15) & ~(size_t)15));
+    replica_sort(S, [&](int i) { return a.pos_in[base + i]; }, lp.cap, a.status, s_start, s_fill, s_pos);
     const CellsShared cells{s_start, s_pos};
-    for (int sid = base + tid; sid < base + n; sid += T) replica_list(a, lp, S, sid, cells);
+    for (int sid = base + (int)threadIdx.x; sid < base + S.n; sid += blockDim.x) replica_list(a, lp, S, sid, cells);
     __syncthreads();
 }
 
@@ -874,7 +976,9 @@ __global__ void __launch_bounds__(ListVariant<V>::kThreads, ListVariant<V>::kMin
 
 // After a per-replica launch: the any-replica flag from the per-replica
 // flags, and the launch's steps that rebuilt some replica counted.
-__global__ void k_list_replica_done(int *flag, int nrep, int *step_rebuilt, int nsteps, long long *builds) {
+// The grid barrier's words (nlist_grid.cuh) are zero between launches.
+__global__ void k_list_replica_done(int *flag, int nrep, int *step_rebuilt, int nsteps, long long *builds,
+                                    unsigned long long *bar_word) {
     __shared__ int s_any, s_steps;
     if (threadIdx.x == 0) s_any = s_steps = 0;
     __syncthreads();
@@ -889,6 +993,7 @@ __global__ void k_list_replica_done(int *flag, int nrep, int *step_rebuilt, int 
     __syncthreads();
     if (threadIdx.x == 0) {
         flag[nrep] = s_any;
+        bar_word[0] = bar_word[1] = 0ull;
         if (s_steps) atomicAdd((unsigned long long *)(builds + 1), (unsigned long long)s_steps);
     }
 }

@@ -168,7 +168,9 @@ __device__ __forceinline__ void sweep_row(const BrickSmem &sm, const float *view
         const f2 dx = f2_sub(*reinterpret_cast<const f2 *>(sm.xs + j), mxx);
         const f2 dy = f2_sub(*reinterpret_cast<const f2 *>(sm.ys + j), myy);
         const f2 dz = f2_sub(*reinterpret_cast<const f2 *>(sm.zs + j), mzz);
-        const f2 d2 = f2_add(f2_add(f2_mul(dx, dx), f2_mul(dy, dy)), f2_mul(dz, dz));
+        // fused sums, written out: the compiler fuses packed products and sums on
+        // its own, and the other list builds have to round alike (list_build_d2)
+        const f2 d2 = f2_fma(dz, dz, f2_fma(dx, dx, f2_mul(dy, dy)));
         float d2a, d2b, ca, cb;
         f2_split(d2, d2a, d2b);
         f2_split(*reinterpret_cast<const f2 *>(view + j), ca, cb);

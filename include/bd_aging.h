@@ -291,7 +291,10 @@ typedef struct bd_engine_opts {
                                   cut distance (BD_ERR_ARG otherwise) */
     int list_variant;          /* list-step launch variant 0 .. BD_LIST_VARIANTS-1, same
                                   results in every variant: 0-2 launch each step (CTA size,
-                                  registers, load placement) with separate rebuild kernels;
+                                  registers, load placement) with separate rebuild kernels,
+                                  except that 0 runs small and mid-size batches (Philox
+                                  noise, up to 512 particles per SM) in one launch per batch
+                                  of steps, a cluster per replica or the whole grid;
                                   3-5 run a whole batch of steps in one launch, one block
                                   of 256 / 512 / 1024 threads per replica that rebuilds its
                                   replica's lists itself (Philox noise; the other noise

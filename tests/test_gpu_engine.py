@@ -253,6 +253,41 @@ def test_list_autotuner_and_launch_variants_change_speed_not_results():
         B.Engine(list(systems), list_variant=6)
 
 
+@pytest.mark.parametrize("sizes,kw", [
+    ([(40, 41)], {}), ([(2048, 2040)], {}), ([(500, 500)], {"potential": "wca"}),
+    ([(60 + 7 * k, 71 + 3 * k) for k in range(20)], {}), ([(300, 30 + k) for k in range(60)], {}),
+    ([(100 + k % 5, 150) for k in range(140)], {}),
+    ([(1100, 1001)], {}), ([(1500, 2900), (90, 41), (3000, 500)], {"potential": "wca"}),
+    ([(2500 + 100 * k, 2000) for k in range(6)], {}), ([(18000, 22003)], {})])
+def test_resident_launches_match_the_per_step_kernels(sizes, kw):
+    """Small replicas run in clusters of 8, 4, 2 and 1 CTAs (by their number),
+    mid-size batches on the whole grid with and without helper threads: the
+    same bits, rebuild counts and neighbour sets as the per-step launches, over
+    whole batches and odd remainders, hot enough to rebuild often."""
+    systems, poss = [], []
+    for k, (nb, ns) in enumerate(sizes):
+        s, p = system(nb, ns, 0.4, 11 + k, T0=3.0, force_cap=100.0, **kw)
+        systems.append(s)
+        poss.append(p)
+    pos = np.concatenate(poss)
+    want = None
+    for v in (1, None):
+        e = B.Engine(list(systems), list_variant=v)
+        assert e.info().neighbor_skin > 0
+        e.set_positions(pos)
+        for k in (1, 230, 96, 33):
+            e.run(k)
+        info = e.info()
+        got = (*e.get_positions(), e.get_displacements(), *e.census(),
+               np.array([info.list_builds, info.list_rebuild_steps]))
+        e.close()
+        if want is None:
+            want = got
+            assert info.list_builds > 2 * len(sizes)
+        for a, b in zip(got, want):
+            np.testing.assert_array_equal(a, b)
+
+
 def test_first_step_temperature_carried_over():
     """A replica given T_first takes its first update at that temperature and
     then follows its protocol (the drop-in executable uses this for
