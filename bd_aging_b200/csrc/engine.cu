@@ -1,6 +1,8 @@
 // engine.cu -- host driver of the batched replica engine (bd_engine_* ABI):
 // geometry, buffers, initial load, CUDA-graph stepping, observation passes and
 // export.
+#include <functional>
+
 #include "engine_kernels.cuh"
 #include "engine_state.cuh"
 
@@ -151,7 +153,7 @@ int configure_kernels(bd_engine *e) {
                                  (int)e->lcl_smem) != cudaSuccess)
             rc = 1;
     }
-    if (e->lrep_smem > 0) {  // variant 5 rebuilds from shared memory
+    if (e->lrep_smem > 0) {  // variant 5: resident positions or rebuilds in shared memory
         if (cudaFuncSetAttribute(k_list_replica<false, 5>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)e->lrep_smem) != cudaSuccess ||
             cudaFuncSetAttribute(k_list_replica<true, 5>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -266,7 +268,8 @@ int launch_list_step(bd_engine *e, const ListArgs &a, int ni_off) {
 // Launch variants 3-5: one block per replica runs `nsteps` steps (the
 // Philox noise only; other noise streams take variant 0).
 bool list_per_replica(const bd_engine *e) {
-    return e->list && e->lvar >= kListFirstPersistent && e->rng == BD_RNG_PHILOX;
+    return e->list && (e->lvar >= kListFirstPersistent || (e->lvar == 0 && e->lrep_default)) &&
+           e->rng == BD_RNG_PHILOX;
 }
 // words of the grid barrier, beside the build counters
 unsigned long long *grid_word(bd_engine *e) { return reinterpret_cast<unsigned long long *>(e->d_builds + 3); }
@@ -274,10 +277,9 @@ template <int V>
 int launch_list_replica_v(bd_engine *e, int cur, int nsteps) {
     constexpr int T = ListVariant<V>::kThreads;
     const ListArgs a = make_largs(e, cur);
-    const bool shared_build = V == 5 && e->lrep_smem > 0;
+    const size_t sm = V == 5 ? e->lrep_smem : 0;
     const ListPersist lp{{e->lpos[0], e->lpos[1]}, cur & 1, e->cnt[0], e->pos[0], e->cap, e->nbr, e->nnb,
-                         e->pbuild, e->d_rep_order, e->d_builds, e->d_step_rebuilt, shared_build ? 1 : 0};
-    const size_t sm = shared_build ? e->lrep_smem : 0;
+                         e->pbuild, e->d_rep_order, e->d_builds, e->d_step_rebuilt, sm, V == 5 && e->lrep_resident ? 1 : 0};
     if (e->extra_pot) k_list_replica<true, V><<<e->R, T, sm, e->stream>>>(a, lp, e->d_ni, nsteps);
     else k_list_replica<false, V><<<e->R, T, sm, e->stream>>>(a, lp, e->d_ni, nsteps);
     BD_LAUNCH_CHECK();
@@ -292,7 +294,7 @@ bool list_cluster(const bd_engine *e) {
 }
 int launch_list_cluster(bd_engine *e, int cur, int nsteps) {
     const ListPersist lp{{e->lpos[0], e->lpos[1]}, cur & 1, e->cnt[0], e->pos[0], e->cap, e->nbr, e->nnb,
-                         e->pbuild, e->d_rep_order, e->d_builds, e->d_step_rebuilt, 0};
+                         e->pbuild, e->d_rep_order, e->d_builds, e->d_step_rebuilt, 0, 0};
     cudaLaunchConfig_t cfg;
     std::memset(&cfg, 0, sizeof(cfg));
     cfg.gridDim = dim3(e->R * e->lcl_ctas);
@@ -318,7 +320,7 @@ int launch_list_cluster(bd_engine *e, int cur, int nsteps) {
 bool list_grid(const bd_engine *e) { return e->list && e->lvar == 0 && e->lgr_blocks > 0 && e->rng == BD_RNG_PHILOX; }
 int launch_list_grid(bd_engine *e, int cur, int nsteps) {
     const ListPersist lp{{e->lpos[0], e->lpos[1]}, cur & 1, e->cnt[0], e->pos[0], e->cap, e->nbr, e->nnb,
-                         e->pbuild, e->d_rep_order, e->d_builds, e->d_step_rebuilt, 0};
+                         e->pbuild, e->d_rep_order, e->d_builds, e->d_step_rebuilt, 0, 0};
     cudaLaunchConfig_t cfg;
     std::memset(&cfg, 0, sizeof(cfg));
     cfg.gridDim = dim3(e->lgr_blocks);
@@ -533,8 +535,9 @@ int rebuild_bricks(bd_engine *e) {
 
 // Variant 0 runs small replicas in clusters (nlist_cluster.cuh): the most CTAs
 // per replica (up to 8) that leave every replica resident at once, one thread
-// per particle; and other batches of up to 512 particles per SM on the whole
-// grid (nlist_grid.cuh).  Larger ones keep the per-step kernels.
+// per particle; other batches of up to 512 particles per SM on the whole grid
+// (nlist_grid.cuh); larger batches of many replicas one block per replica.
+// The others keep the per-step kernels.
 void choose_resident(bd_engine *e) {
     int nmax = 0, cmax = 0;
     for (const SysDev &S : e->sysh) {
@@ -557,11 +560,34 @@ void choose_resident(bd_engine *e) {
     int sms = 0, coop = 0;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, e->dev);
     cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, e->dev);
-    if (!coop || e->P > (long long)sms * kGridMaxOwners) return;
-    const int G = std::min(sms, div_up(e->P, 128));
-    e->lgr_owners = (div_up(e->P, G) + 31) / 32 * 32;
-    e->lgr_help = 2 * e->lgr_owners <= kGridMaxOwners;
-    e->lgr_blocks = G;
+    if (coop && e->P <= (long long)sms * kGridMaxOwners) {
+        const int G = std::min(sms, div_up(e->P, 128));
+        e->lgr_owners = (div_up(e->P, G) + 31) / 32 * 32;
+        e->lgr_help = 2 * e->lgr_owners <= kGridMaxOwners;
+        e->lgr_blocks = G;
+        return;
+    }
+    // Many replicas, none much larger than an SM's share: variant 5's launch.
+    // Its step takes 5.5 us per 1000 particles of the most loaded SM (blocks go
+    // to SMs largest replica first) with resident positions, 6.2 without; the
+    // per-step kernels' 6 us, 43 us per million particles and, since some
+    // replica rebuilds in most steps of a large batch, up to 20 us of rebuild
+    // passes.  Measured, us a step, this launch / per-step: 256 replicas of 500
+    // to 8000 50 / 79, 148 x 6000 33 / 63, 60 x 3000 17 / 25, 1000 x 500 24 / 62,
+    // 250 x 8000 97 / 110; 64 x 32768 (183 by this rule) / 93.
+    std::vector<long long> load(std::max(1, sms), 0);
+    std::vector<int> sizes;
+    for (const SysDev &S : e->sysh) sizes.push_back(S.n);
+    std::sort(sizes.begin(), sizes.end(), std::greater<int>());
+    std::make_heap(load.begin(), load.end(), std::greater<long long>());
+    for (int n : sizes) {
+        std::pop_heap(load.begin(), load.end(), std::greater<long long>());
+        load.back() += n;
+        std::push_heap(load.begin(), load.end(), std::greater<long long>());
+    }
+    const double most = (double)*std::max_element(load.begin(), load.end());
+    e->lrep_default = (e->lrep_resident ? 5.5e-3 : 6.2e-3) * most <
+                      6.0 + 4.3e-5 * (double)e->P + std::min(20.0, 0.08 * e->R);
 }
 
 // Upload the brick layout (after rebuild_bricks) and drop graphs recorded
@@ -781,12 +807,20 @@ int bd_engine_create(const bd_system_desc *systems, int nsys, const bd_engine_op
             std::stable_sort(order.begin(), order.end(),
                              [&](int a, int b) { return e->sysh[a].n > e->sysh[b].n; });
             cudaMemcpyAsync(e->d_rep_order, order.data(), sizeof(int) * e->R, cudaMemcpyHostToDevice, e->stream);
-            size_t need = 0;  // the largest in-block rebuild from shared memory
+            // variant 5: positions resident in shared memory where every replica's
+            // fit (the memory is taken from L1, which the others' gathers need:
+            // with replicas of 7000 to 8000 among smaller ones 51.5 us a step
+            // became 59.4), else in-block rebuilds in shared memory
+            size_t resident = 0, build = 0;
             for (int r = 0; r < e->R; r++) {
                 const SysDev &S = e->sysh[r];
-                need = std::max(need, replica_shared_build_bytes(S.n, S.ncell * S.ncell * S.ncell));
+                const int cells = S.ncell * S.ncell * S.ncell;
+                resident = std::max(resident, replica_resident_bytes(S.n, cells));
+                build = std::max(build, replica_shared_build_bytes(S.n, cells));
             }
-            e->lrep_smem = need <= (size_t)227 * 1024 ? need : 0;
+            const size_t most = (size_t)226 * 1024;
+            e->lrep_smem = resident <= most ? resident : build <= most ? build : 0;
+            e->lrep_resident = resident <= most;
             choose_resident(e);
             cudaStreamSynchronize(e->stream);  // the host vector goes out of scope
         }
@@ -985,7 +1019,7 @@ int autotune_list(bd_engine *e, long long &nsteps) {
             if (e->rng == BD_RNG_PHILOX) stage2.push_back({e->bx, e->by, e->bz, v});
             continue;
         }
-        if (v == 0 && (e->lcl_ctas > 0 || e->lgr_blocks > 0)) {
+        if (v == 0 && (e->lcl_ctas > 0 || e->lgr_blocks > 0 || e->lrep_default)) {
             stage2.push_back({e->bx, e->by, e->bz, v});
             continue;
         }

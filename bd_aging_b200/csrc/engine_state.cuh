@@ -83,7 +83,9 @@ struct bd_engine {
     int *img = nullptr;             // [3][P] face crossings since the origin (displacement on demand)
     float *amp_tab = nullptr;       // [graph_steps][R][2] noise amplitudes of a launch batch
     int *d_rep_order = nullptr;     // per-replica launch (variants 3-5): replica of each block
-    size_t lrep_smem = 0;           // variant 5: shared memory of an in-block rebuild (0: from global memory)
+    bool lrep_resident = false;     // variant 5: positions resident in shared memory
+    bool lrep_default = false;      // variant 0 takes variant 5's launch
+    size_t lrep_smem = 0;           // variant 5: dynamic shared memory (resident positions, in-block rebuilds)
     // variant 0 in clusters (0 CTAs: the per-step kernels): CTAs per replica, the particles each owns at
     // most, their shared memory, the largest replica's particles and cells
     int lcl_ctas = 0, lcl_owners = 0, lcl_nmax = 0, lcl_cells = 0;

@@ -25,7 +25,6 @@
 // (cnt / pos of buffer 0) are rebuilt from the by-id positions for list
 // builds and observation passes.
 #pragma once
-#include <type_traits>
 
 namespace bd {
 
@@ -381,15 +380,13 @@ __device__ __forceinline__ f2 min_image_pair(f2 d, f2 linv, f2 neg_l) {
 // difference.  The force is summed in two interleaved partial sums (even and
 // odd list positions) that are added at the end.
 template <bool WRAP, class SRC>
-__device__ __forceinline__ void list_forces_wca(const SRC &src, int n, float4 pi, float L, float Linv, float sg0,
+__device__ __forceinline__ void list_forces_wca(const SRC &src, int n, int (&jn)[kGather], float4 pi, float L, float Linv, float sg0,
                                                 float sg1, float c0, float c1, float &fx, float &fy, float &fz) {
     const f2 PX = f2_bcast(pi.x), PY = f2_bcast(pi.y), PZ = f2_bcast(pi.z), M12 = f2_bcast(-12.0f);
     const float sq0 = sg0 * sg0, sq1 = sg1 * sg1;
     const f2 LINV = f2_bcast(Linv), NEGL = f2_bcast(-L);
     f2 FX = 0ull, FY = 0ull, FZ = 0ull;  // (0.f, 0.f)
     const int np = src.none;
-    int jn[kGather];
-    if (n > 0) src.words(0, jn);
     for (int k0 = 0; k0 < n; k0 += kGather) {
         int jj[kGather];
         float4 pj[kGather];
@@ -448,14 +445,12 @@ __device__ __forceinline__ void list_forces_wca(const SRC &src, int n, float4 pi
 // Force from the list for a replica with another potential of PotKind
 // (scalar, list order).
 template <class SRC>
-__device__ __forceinline__ void list_forces_extra(const SRC &src, const SysDev &S, int n, float4 pi, int tm, float &fx,
-                                                  float &fy, float &fz) {
+__device__ __forceinline__ void list_forces_extra(const SRC &src, const SysDev &S, int n, int (&jn)[kGather], float4 pi,
+                                                  int tm, float &fx, float &fy, float &fz) {
     const float L = S.L, Linv = S.Linv;
     const float sg0 = tm ? S.sig[1] : S.sig[0], sg1 = tm ? S.sig[2] : S.sig[1];
     const float c0 = tm ? S.cut2[1] : S.cut2[0], c1 = tm ? S.cut2[2] : S.cut2[1];
     fx = fy = fz = 0.f;
-    int jn[kGather];
-    if (n > 0) src.words(0, jn);
     for (int k0 = 0; k0 < n; k0 += kGather) {
         int jj[kGather];
         float4 pj[kGather];
@@ -485,15 +480,16 @@ __device__ __forceinline__ void list_forces_extra(const SRC &src, const SysDev &
 // Force on a particle from its list of n partners, capped for the initial
 // relaxation.  EXTRA: some replica of the batch uses a potential other than
 // the modified WCA (instantiated separately so the default kernel keeps its
-// registers).  Called by whole warps less those past the last particle.
+// registers).  jn: the list's first words, loaded by the caller beside its
+// length.  Called by whole warps less those past the last particle.
 template <bool EXTRA, class SRC>
-__device__ __forceinline__ void list_force(const SRC &src, const SysDev &S, int n, float4 pi, int tm, float &fx,
-                                           float &fy, float &fz) {
+__device__ __forceinline__ void list_force(const SRC &src, const SysDev &S, int n, int (&jn)[kGather], float4 pi, int tm,
+                                           float &fx, float &fy, float &fz) {
     const float L = S.L, Linv = S.Linv;
     const float sg0 = tm ? S.sig[1] : S.sig[0], sg1 = tm ? S.sig[2] : S.sig[1];
     const float c0 = tm ? S.cut2[1] : S.cut2[0], c1 = tm ? S.cut2[2] : S.cut2[1];
     if (EXTRA && S.pot != kPotWcaModified) {
-        list_forces_extra(src, S, n, pi, tm, fx, fy, fz);
+        list_forces_extra(src, S, n, jn, pi, tm, fx, fy, fz);
     } else {  // the same arithmetic in either instantiation: a replica's result does not depend on its batch
         // a warp whose particles all sit away from the faces needs no
         // minimum image for any partner
@@ -501,9 +497,9 @@ __device__ __forceinline__ void list_force(const SRC &src, const SysDev &S, int 
         const bool inner = pi.x >= lo_edge && pi.x <= hi_edge && pi.y >= lo_edge && pi.y <= hi_edge &&
                            pi.z >= lo_edge && pi.z <= hi_edge;
         if (__all_sync(__activemask(), inner))
-            list_forces_wca<false>(src, n, pi, L, Linv, sg0, sg1, c0, c1, fx, fy, fz);
+            list_forces_wca<false>(src, n, jn, pi, L, Linv, sg0, sg1, c0, c1, fx, fy, fz);
         else
-            list_forces_wca<true>(src, n, pi, L, Linv, sg0, sg1, c0, c1, fx, fy, fz);
+            list_forces_wca<true>(src, n, jn, pi, L, Linv, sg0, sg1, c0, c1, fx, fy, fz);
     }
     if (S.fcap > 0.f) {  // capped forces for the initial relaxation
         const float fmx = fmaxf(fabsf(fx), fmaxf(fabsf(fy), fabsf(fz)));
@@ -538,12 +534,13 @@ __device__ __forceinline__ bool list_beyond(float x, float y, float z, float4 pb
 // process_brick.  Returns true when the particle has moved more than half
 // the skin since the last build (its replica's lists must be rebuilt).
 // LATE: the particle's own state is loaded after the force loop.  NC: loads
-// through the read-only path (ld_state).
-template <int RNG, bool EXTRA, bool LATE, bool NC>
-__device__ __forceinline__ bool list_particle_step(const ListArgs &a, int sid, int rep, long long ni, int ni_off) {
+// through the read-only path (ld_state).  The positions of this step come
+// from `src` and the particle's own, pi; the new one goes to *out.
+template <int RNG, bool EXTRA, bool LATE, bool NC, class SRC>
+__device__ __forceinline__ bool list_particle_step(const ListArgs &a, const SRC &src, float4 pi, float4 *out, int sid,
+                                                   int rep, long long ni, int ni_off) {
     const SysDev &S = a.sys[rep];
     const float L = S.L, Linv = S.Linv;
-    const float4 pi = a.pos_in[sid];
     const unsigned wi = __float_as_uint(pi.w);
     const int tm = (int)(wi >> 31);
     int gid;
@@ -554,9 +551,13 @@ __device__ __forceinline__ bool list_particle_step(const ListArgs &a, int sid, i
         lx = a.lo_x[sid], ly = a.lo_y[sid], lz = a.lo_z[sid];
         pb = ld_state<NC>(a.pbuild + sid);
     }
-    float fx, fy, fz;
+    // the first list words are loaded whatever the list's length, so that their
+    // latency runs beside its own (aging batch: 96.1 -> 92.6 us a step)
+    int jn[kGather];
+    src.words(0, jn);
     const int n = min(ld_state<NC>(a.nnb + sid), kMaxNbr);
-    list_force<EXTRA>(ListGlobal<NC>(a, sid), S, n, pi, tm, fx, fy, fz);
+    float fx, fy, fz;
+    list_force<EXTRA>(src, S, n, jn, pi, tm, fx, fy, fz);
     if constexpr (LATE) {
         gid = __ldg(a.gid_of + sid);
         lx = a.lo_x[sid], ly = a.lo_y[sid], lz = a.lo_z[sid];
@@ -603,7 +604,7 @@ __device__ __forceinline__ bool list_particle_step(const ListArgs &a, int sid, i
     a.lo_y[sid] = ly;
     a.lo_z[sid] = lz;
     if (!(isfinite(x) && isfinite(y) && isfinite(z))) set_status(a.status, kStatNumeric);
-    a.pos_out[sid] = make_float4(x, y, z, pi.w);
+    *out = make_float4(x, y, z, pi.w);
     return list_beyond(x, y, z, pb, L, Linv, S.skin_half2);
 }
 
@@ -615,7 +616,9 @@ __global__ void __launch_bounds__(ListVariant<V>::kThreads, ListVariant<V>::kMin
     const int sid = blockIdx.x * blockDim.x + threadIdx.x;
     if (sid >= a.np) return;
     const int rep = a.rep_of_sid[sid];
-    if (list_particle_step<RNG, EXTRA, ListVariant<V>::kLate, true>(a, sid, rep, *ni_base + ni_off, ni_off)) {
+    if (list_particle_step<RNG, EXTRA, ListVariant<V>::kLate, true>(a, ListGlobal<true>(a, sid), a.pos_in[sid],
+                                                                    a.pos_out + sid, sid, rep, *ni_base + ni_off,
+                                                                    ni_off)) {
         a.flag[rep] = 1;
         a.flag[a.nrep] = 1;
     }
@@ -645,7 +648,8 @@ struct ListPersist {
     const int *order;      // replica of each block, most particles first
     long long *builds;     // [0] replica list builds, [1] steps that rebuilt
     int *step_rebuilt;     // [step of the launch]: some replica rebuilt before it
-    int shared_build;      // variant 5: rebuild from shared memory (replica_rebuild_shared)
+    size_t smem;           // variant 5: dynamic shared memory, for resident positions (replica_resident_bytes)
+    int resident;          //   or a rebuild (replica_shared_build_bytes; 0: rebuilds from global memory)
 };
 
 // cell of a by-id position, as bin_particle and the step kernels bin it
@@ -685,12 +689,16 @@ struct CellsGlobal {
 struct CellsShared {
     const int *start;  // [cells + 1]
     const float4 *pos;
+    __device__ __forceinline__ const float4 *cell(int c, int &m) const {
+        m = start[c + 1] - start[c];
+        return pos + start[c];
+    }
 };
 
 // Partners of the particle at v from the sorted cells of its replica:
 // emit(k, storage id) for the k-th; returns their number.
-template <class EMIT>
-__device__ __forceinline__ int replica_partners(const SysDev &S, float4 v, const CellsGlobal &cells, EMIT emit) {
+template <class CELLS, class EMIT>
+__device__ __forceinline__ int replica_partners(const SysDev &S, float4 v, const CELLS &cells, EMIT emit) {
     const int nc = S.ncell;
     const int sid = (int)(__float_as_uint(v.w) & 0x7fffffffu);
     const int tm = (int)(__float_as_uint(v.w) >> 31);
@@ -728,16 +736,18 @@ __device__ __forceinline__ int replica_partners(const SysDev &S, float4 v, const
     }
     return cnt;
 }
-// The same from the cell-sorted copy in shared memory, rows row0 .. row1 - 1 of
-// its nine (dz, dy), where the three cells
-// of a row are one run of positions (two where the row crosses a face).  A
-// row's candidates are tested four at a time into a bit mask, and the hits
-// written after it: with a branch and a store per candidate a block of 128
-// particles took 50000 cycles (each lane waiting for the others' cells and
-// hits), now 22000, and 11000 with its rows shared by two threads.
+// The same for few warps (nlist_cluster.cuh): rows row0 .. row1 - 1 of the nine
+// (dz, dy), where the three cells of the cell-sorted copy are one run of
+// positions (two where the row crosses a face).  A row's candidates are tested
+// four at a time into a bit mask, and the hits written after it.  With a branch
+// and a store per candidate a block of 128 particles took 50000 cycles, each
+// lane waiting for the others' cells and hits, and now 22000 (11000 with its
+// rows shared by two threads); with 32 warps on the SM to hide those waits the
+// fewer instructions of the plain loop win (51.4 against 54.4 us a step of the
+// ragged batch, a rebuild in every 40th).
 template <class EMIT>
-__device__ __forceinline__ int replica_partners(const SysDev &S, float4 v, const CellsShared &cells, int row0, int row1,
-                                                EMIT emit) {
+__device__ __forceinline__ int replica_partners_rows(const SysDev &S, float4 v, const CellsShared &cells, int row0,
+                                                     int row1, EMIT emit) {
     const int nc = S.ncell;
     const unsigned self = __float_as_uint(v.w) & 0x7fffffffu;
     const int tm = (int)(__float_as_uint(v.w) >> 31);
@@ -787,16 +797,12 @@ __device__ __forceinline__ int replica_partners(const SysDev &S, float4 v, const
 // List of particle sid from the sorted cells of its replica.
 template <class CELLS>
 __device__ __forceinline__ void replica_list(const ListArgs &a, const ListPersist &lp, const SysDev &S, int sid,
-                                             const CELLS &cells) {
-    const float4 v = a.pos_in[sid];
+                                             float4 v, const CELLS &cells) {
     const int np = a.np;
-    auto emit = [&](int k, int sj) {
+    const int cnt = replica_partners(S, v, cells, [&](int k, int sj) {
         if (k < kMaxNbr) lp.nbr[list_slot(k, sid, np)] = sj;
         else set_status(a.status, kStatCellOverflow);
-    };
-    int cnt;
-    if constexpr (std::is_same_v<CELLS, CellsShared>) cnt = replica_partners(S, v, cells, 0, 9, emit);
-    else cnt = replica_partners(S, v, cells, emit);
+    });
     const int nl = min(cnt, kMaxNbr);
     for (int k = nl; k < kMaxNbr && (k % kGather) != 0; k++) lp.nbr[list_slot(k, sid, np)] = np;
     lp.nnb[sid] = nl;
@@ -836,7 +842,7 @@ __device__ __forceinline__ void replica_rebuild(const ListArgs &a, const ListPer
     }
     __syncthreads();
     const CellsGlobal cells{lp.cnt, lp.bucket, cap, cb};
-    for (int sid = base + tid; sid < end; sid += T) replica_list(a, lp, S, sid, cells);
+    for (int sid = base + tid; sid < end; sid += T) replica_list(a, lp, S, sid, a.pos_in[sid], cells);
     __syncthreads();
 }
 
@@ -931,8 +937,68 @@ __device__ __forceinline__ void replica_rebuild_shared(const ListArgs &a, const 
     float4 *s_pos = reinterpret_cast<float4 *>(dsm + (((size_t)(2 * ncell + 1) * 4 + 15) & ~(size_t)15));
     replica_sort(S, [&](int i) { return a.pos_in[base + i]; }, lp.cap, a.status, s_start, s_fill, s_pos);
     const CellsShared cells{s_start, s_pos};
-    for (int sid = base + (int)threadIdx.x; sid < base + S.n; sid += blockDim.x) replica_list(a, lp, S, sid, cells);
+    for (int sid = base + (int)threadIdx.x; sid < base + S.n; sid += blockDim.x) replica_list(a, lp, S, sid, a.pos_in[sid], cells);
     __syncthreads();
+}
+
+// Variant 5, shared memory of a replica whose positions stay in it for the
+// launch: two position buffers (with the zero position), the second of which
+// is a rebuild's sorted copy, then its cell starts and counters.
+__host__ __device__ inline size_t replica_resident_bytes(int n, int c) {
+    return 2 * (size_t)(n + 1) * 16 + (size_t)(2 * c + 1) * 4;
+}
+struct ListBlock {  // lists in global memory (storage ids), positions of the replica in shared memory
+    const ListArgs &a;
+    const float4 *pos;
+    int sid, base, none;
+    __device__ __forceinline__ void words(int k0, int (&jn)[kGather]) const {
+        ListGlobal<false>(a, sid).words(k0, jn);
+    }
+    __device__ __forceinline__ void gather(const int (&jn)[kGather], int (&jj)[kGather], float4 (&pj)[kGather]) const {
+#pragma unroll
+        for (int u = 0; u < kGather; u++) {
+            jj[u] = (int)min((unsigned)(jn[u] - base), (unsigned)none);
+            pj[u] = pos[jj[u]];
+        }
+    }
+};
+// The steps of k_list_replica with the positions resident in shared memory:
+// a partner gather is a shared load instead of one from L1 (70%) or L2, and a
+// step needs no more barriers than before (the buffers alternate): 32.6 us a
+// step against 40.5 with 148 replicas of 6000 particles.
+template <bool EXTRA>
+__device__ __forceinline__ bool replica_steps_resident(const ListArgs &a, const ListPersist &lp, const SysDev &S, int rep,
+                                                       long long ni0, int nsteps, bool need, unsigned char *dsm) {
+    const int tid = threadIdx.x, T = blockDim.x, n = S.n, base = S.part_base;
+    const int ncell = S.ncell * S.ncell * S.ncell;
+    float4 *s_pos = reinterpret_cast<float4 *>(dsm);  // [2][n + 1]
+    int *s_start = reinterpret_cast<int *>(s_pos + 2 * (n + 1)), *s_fill = s_start + ncell + 1;
+    const float4 *in = (lp.cur0 & 1) ? lp.pos[1] : lp.pos[0];
+    float4 *out = ((lp.cur0 + nsteps) & 1) ? lp.pos[1] : lp.pos[0];
+    for (int i = tid; i < n; i += T) s_pos[i] = in[base + i];
+    if (tid < 2) s_pos[tid * (n + 1) + n] = make_float4(0.f, 0.f, 0.f, 0.f);
+    __syncthreads();
+    for (int s = 0; s < nsteps; s++) {
+        float4 *cur = s_pos + (s & 1) * (n + 1), *nxt = s_pos + ((s & 1) ^ 1) * (n + 1);
+        if (need) {
+            replica_sort(S, [&](int i) { return cur[i]; }, lp.cap, a.status, s_start, s_fill, nxt);
+            const CellsShared cells{s_start, nxt};
+            for (int i = tid; i < n; i += T) replica_list(a, lp, S, base + i, cur[i], cells);
+            __syncthreads();
+            if (tid == 0) {
+                atomicAdd((unsigned long long *)lp.builds, 1ull);
+                lp.step_rebuilt[s] = 1;
+            }
+        }
+        bool beyond = false;
+        for (int i = tid; i < n; i += T)
+            beyond |= list_particle_step<kRngPhilox, EXTRA, true, false>(a, ListBlock{a, cur, base + i, base, n}, cur[i],
+                                                                         nxt + i, base + i, rep, ni0 + s, s);
+        need = __syncthreads_or(beyond) != 0;
+    }
+    const float4 *last = s_pos + (nsteps & 1) * (n + 1);
+    for (int i = tid; i < n; i += T) out[base + i] = last[i];
+    return need;
 }
 
 // nsteps steps of replica order[blockIdx.x] (Philox noise; nsteps at most the
@@ -947,6 +1013,13 @@ __global__ void __launch_bounds__(ListVariant<V>::kThreads, ListVariant<V>::kMin
     const int base = S.part_base, end = S.part_base + S.n;
     const long long ni0 = *ni_base;
     bool need = a.flag[rep] != 0;
+    if constexpr (V == 5) {
+        if (lp.resident) {
+            need = replica_steps_resident<EXTRA>(a, lp, S, rep, ni0, nsteps, need, dsm);
+            if (threadIdx.x == 0) a.flag[rep] = need ? 1 : 0;
+            return;
+        }
+    }
     for (int s = 0; s < nsteps; s++) {
         ListArgs as = a;
         const bool odd = ((lp.cur0 + s) & 1) != 0;  // a select, not an indexed (local-memory) copy
@@ -955,7 +1028,7 @@ __global__ void __launch_bounds__(ListVariant<V>::kThreads, ListVariant<V>::kMin
         if (need) {
             bool done = false;
             if constexpr (V == 5) {
-                if (lp.shared_build) {
+                if (lp.smem > 0) {
                     replica_rebuild_shared(as, lp, S, dsm);
                     done = true;
                 }
@@ -968,7 +1041,8 @@ __global__ void __launch_bounds__(ListVariant<V>::kThreads, ListVariant<V>::kMin
         }
         bool beyond = false;
         for (int sid = base + (int)threadIdx.x; sid < end; sid += blockDim.x)
-            beyond |= list_particle_step<kRngPhilox, EXTRA, ListVariant<V>::kLate, false>(as, sid, rep, ni0 + s, s);
+            beyond |= list_particle_step<kRngPhilox, EXTRA, ListVariant<V>::kLate, false>(
+                as, ListGlobal<false>(as, sid), as.pos_in[sid], as.pos_out + sid, sid, rep, ni0 + s, s);
         need = __syncthreads_or(beyond) != 0;
     }
     if (threadIdx.x == 0) a.flag[rep] = need ? 1 : 0;

@@ -20,7 +20,7 @@
 //    rebuilds its own particles' lists, with one more cluster barrier before
 //    that buffer is written again.
 // Lists, force sums, updates and rebuild decisions are those of the other
-// launches (replica_partners, list_force, advance_wrap, list_beyond), so the
+// launches (replica_partners_rows, list_force, advance_wrap, list_beyond), so the
 // bits are the same.  Lists and state go back to global memory at the end of
 // the launch.
 // Measured, one replica at T = 0.1: 1.57, 1.86 and 2.78 us a step at N = 500,
@@ -236,7 +236,7 @@ __global__ void __launch_bounds__(2 * kClusterMaxOwners, 1)
             const float4 v = owner ? pi : cur[lid];
             int found = 0;
             if (live)
-                found = replica_partners(S, v, cells, owner ? 0 : 5, owner ? 5 : 9, [&](int k, int sj) {
+                found = replica_partners_rows(S, v, cells, owner ? 0 : 5, owner ? 5 : 9, [&](int k, int sj) {
                     if (k < kMaxNbr / 2) my_list[list_at(owner ? k : kMaxNbr - 1 - k)] = (unsigned short)(sj - base);
                 });
             if (!owner) helped[tid] = found;
@@ -247,7 +247,7 @@ __global__ void __launch_bounds__(2 * kClusterMaxOwners, 1)
                     for (int k = 0; k < more; k++) my_list[list_at(found + k)] = my_list[list_at(kMaxNbr - 1 - k)];
                     found += more;
                 } else {  // a long list: both halves into its front
-                    found = replica_partners(S, v, cells, 0, 9, [&](int k, int sj) {
+                    found = replica_partners_rows(S, v, cells, 0, 9, [&](int k, int sj) {
                         if (k < kMaxNbr) my_list[list_at(k)] = (unsigned short)(sj - base);
                         else set_status(a.status, kStatCellOverflow);
                     });
@@ -271,8 +271,13 @@ __global__ void __launch_bounds__(2 * kClusterMaxOwners, 1)
             const float nx = z[0], ny = z[T], nz = z[2 * T];
             float fx, fy, fz;
             const ListShared src{cur, s_list + tid, T, n};
-            if (general) list_force<EXTRA>(src, S, nl, pi, tm, fx, fy, fz);
-            else list_forces_wide(src, nl, pi, L, Linv, sg0 * sg0, sg1 * sg1, c0, c1, fx, fy, fz);
+            if (general) {
+                int jn[kGather];
+                src.words(0, jn);
+                list_force<EXTRA>(src, S, nl, jn, pi, tm, fx, fy, fz);
+            } else {
+                list_forces_wide(src, nl, pi, L, Linv, sg0 * sg0, sg1 * sg1, c0, c1, fx, fy, fz);
+            }
             if (ni0 + s == 0) {  // origin of the unwrapped positions (main.cu:497-506)
                 a.x0[3 * (size_t)gid] = (double)pi.x + (double)lx;
                 a.x0[3 * (size_t)gid + 1] = (double)pi.y + (double)ly;

@@ -264,8 +264,13 @@ __global__ void __launch_bounds__(kGridMaxOwners, 1)
             const float nx = z[0], ny = z[T], nz = z[2 * T];
             float fx, fy, fz;
             const ListGrid src{cur, s_list + tid, T, a.np};
-            if (general) list_force<EXTRA>(src, S, nl, pi, tm, fx, fy, fz);
-            else list_forces_wide(src, nl, pi, L, Linv, sg0 * sg0, sg1 * sg1, c0, c1, fx, fy, fz);
+            if (general) {
+                int jn[kGather];
+                src.words(0, jn);
+                list_force<EXTRA>(src, S, nl, jn, pi, tm, fx, fy, fz);
+            } else {
+                list_forces_wide(src, nl, pi, L, Linv, sg0 * sg0, sg1 * sg1, c0, c1, fx, fy, fz);
+            }
             if (ni0 + s == 0) {  // origin of the unwrapped positions (main.cu:497-506)
                 a.x0[3 * (size_t)gid] = (double)pi.x + (double)lx;
                 a.x0[3 * (size_t)gid + 1] = (double)pi.y + (double)ly;

@@ -292,9 +292,10 @@ typedef struct bd_engine_opts {
     int list_variant;          /* list-step launch variant 0 .. BD_LIST_VARIANTS-1, same
                                   results in every variant: 0-2 launch each step (CTA size,
                                   registers, load placement) with separate rebuild kernels,
-                                  except that 0 runs small and mid-size batches (Philox
-                                  noise, up to 512 particles per SM) in one launch per batch
-                                  of steps, a cluster per replica or the whole grid;
+                                  except that 0 runs (with Philox noise) small and mid-size
+                                  batches and batches of many replicas in one launch per
+                                  batch of steps: a cluster per replica, the whole grid, or
+                                  a block per replica;
                                   3-5 run a whole batch of steps in one launch, one block
                                   of 256 / 512 / 1024 threads per replica that rebuilds its
                                   replica's lists itself (Philox noise; the other noise

@@ -258,11 +258,13 @@ def test_list_autotuner_and_launch_variants_change_speed_not_results():
     ([(60 + 7 * k, 71 + 3 * k) for k in range(20)], {}), ([(300, 30 + k) for k in range(60)], {}),
     ([(100 + k % 5, 150) for k in range(140)], {}),
     ([(1100, 1001)], {}), ([(1500, 2900), (90, 41), (3000, 500)], {"potential": "wca"}),
-    ([(2500 + 100 * k, 2000) for k in range(6)], {}), ([(18000, 22003)], {})])
+    ([(2500 + 100 * k, 2000) for k in range(6)], {}), ([(18000, 22003)], {}),
+    ([(150, 150 + k % 7) for k in range(280)], {}), ([(3700, 3801)] + [(600, 530)] * 90, {})])
 def test_resident_launches_match_the_per_step_kernels(sizes, kw):
     """Small replicas run in clusters of 8, 4, 2 and 1 CTAs (by their number),
-    mid-size batches on the whole grid with and without helper threads: the
-    same bits, rebuild counts and neighbour sets as the per-step launches, over
+    mid-size batches on the whole grid with and without helper threads, and
+    batches of many replicas a block each, with resident positions where they
+    fit: the same bits, rebuild counts and neighbour sets as the per-step launches, over
     whole batches and odd remainders, hot enough to rebuild often."""
     systems, poss = [], []
     for k, (nb, ns) in enumerate(sizes):
