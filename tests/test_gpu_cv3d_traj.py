@@ -48,6 +48,36 @@ def test_cv3d_fp64_normal_equations_against_oracle():
     np.testing.assert_allclose(cv.get_vector(), ref, rtol=1e-3, atol=1e-3 * np.abs(ref).max())
 
 
+@pytest.mark.parametrize("n,bins,rng,side", [(5, 3, 2.0, 6.0), (64, 17, 2.5, 9.0), (1025, 16, 4.4, 9.0),
+                                             (333, 40, 3.0, None), (1500, 33, 2.0, 12.0),
+                                             (900, 65, 3.0, 8.0)])
+def test_cv3d_edges_match_the_oracle(n, bins, rng, side):
+    """Particle counts around the row tiles, partner tiles and splits, a range
+    near half the box (every pair takes the reference's test), no periodic
+    images, and coordinates outside the box.  Bound: the oracle's float sums
+    of up to 1500 terms are within 1e-5 of exact (relative), on both sides of
+    a solve that amplifies by the condition of the kept singular values."""
+    g = np.random.default_rng(n)
+    pos = g.uniform(0, side or 8.0, (n, 3)).astype(np.float32)
+    if bins == 33:
+        pos[::9] += np.float32(3 * side)
+    xx = g.normal(size=(n, 3)).astype(np.float32)
+    ata, atb, bad = O.cv3d_add(bins, rng, pos, xx, -1.0 if side is None else side)
+    cv = B.Contracting_Vector3D(bins, rng)
+    cv.add_statistics(dev(pos), dev(xx), n, side)
+    cv.calculate_vector()
+    got = cv.get_vector().astype(np.float64)
+    assert bad == 0
+    ref, bound = np.zeros(bins), 0.0
+    for c in range(3):
+        u, w, vt = np.linalg.svd(ata[c].astype(np.float64))
+        keep = w > 1e-6 * w[0]
+        x = vt[keep].T @ ((u[:, keep].T @ atb[c].astype(np.float64)) / w[keep])
+        ref += x / 3.0
+        bound += 2e-5 * w[0] / w[keep][-1] * np.linalg.norm(x) / 3.0
+    assert np.linalg.norm(got - ref) <= bound
+
+
 def test_cv3d_state_errors_replace_reference_throws():
     cv = B.Contracting_Vector3D(8, 2.0)
     with pytest.raises(B.BDError) as e1:
