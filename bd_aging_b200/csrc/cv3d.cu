@@ -324,8 +324,7 @@ struct bd_cv3d {
     float range = 0.f;
     int samples = 0;
     bool calculated = false;
-    double *d_ata = nullptr, *d_atb = nullptr;  // one allocation: [3][bins][bins], [3][bins], the status word
-    unsigned *d_status = nullptr;
+    double *d_ata = nullptr, *d_atb = nullptr;  // one allocation: [3][bins][bins], [3][bins]
     void *d_work = nullptr;                     // partial normal equations, then H
     size_t work_cap = 0;
     std::vector<float> result;
@@ -340,13 +339,12 @@ int bd_cv3d_create(int bins, float range, bd_cv3d **out) {
     cv->range = range;
     cv->result.assign(bins, 0.f);
     const size_t sums = 3 * (size_t)bins * bins + 3 * (size_t)bins;
-    if (cudaMalloc(&cv->d_ata, sizeof(double) * (sums + 1)) != cudaSuccess) {
+    if (cudaMalloc(&cv->d_ata, sizeof(double) * sums) != cudaSuccess) {
         bd_cv3d_destroy(cv);
         return BD_ERR_NOMEM;
     }
     cv->d_atb = cv->d_ata + 3 * (size_t)bins * bins;
-    cv->d_status = reinterpret_cast<unsigned *>(cv->d_ata + sums);
-    cudaMemset(cv->d_ata, 0, sizeof(double) * (sums + 1));
+    cudaMemset(cv->d_ata, 0, sizeof(double) * sums);
     *out = cv;
     return BD_OK;
 }
@@ -375,10 +373,11 @@ int bd_cv3d_add_statistics(bd_cv3d *cv, const float *rr, const float *xx, int n,
     const int warps = cv_hits_smem(bins, fused, 16) <= (size_t)226 * 1024 ? 16 : 8;
     const size_t sm = cv_hits_smem(bins, fused, warps);
     if (sm > 48 * 1024) BD_CUDA_TRY(cudaFuncSetAttribute(k_cv_hits, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
-    BD_CUDA_TRY(cudaMemsetAsync(cv->d_status, 0, sizeof(unsigned), s));
+    CallSlot w;
+    if (!w.ok()) return BD_ERR_NOMEM;
     if (!fused) BD_CUDA_TRY(cudaMemsetAsync(d_H, 0, sizeof(float) * 3 * (size_t)n * bins, s));
     k_cv_hits<<<div_up(n, kCvBlock), warps * 32, sm, s>>>({rr, xx, n, side, cv->range, bins, d_H, cv->d_ata, cv->d_atb,
-                                                           cv->d_status});
+                                                           w.status()});
     BD_LAUNCH_CHECK();
     if (!fused) {
         k_cv_normal<<<dim3(tiles, tiles, 3 * splits), dim3(16, 16), 0, s>>>(d_H, xx, n, bins, splits, d_part, cv->d_ata,
@@ -389,11 +388,9 @@ int bd_cv3d_add_statistics(bd_cv3d *cv, const float *rr, const float *xx, int n,
         k_cv_reduce<<<div_up((long)sums, 64), 64, 0, s>>>(d_part, splits, (int)sums, cv->d_ata);
         BD_LAUNCH_CHECK();
     }
-    unsigned bits = 0;
-    BD_CUDA_TRY(cudaMemcpyAsync(&bits, cv->d_status, sizeof(unsigned), cudaMemcpyDeviceToHost, s));
     BD_CUDA_TRY(cudaStreamSynchronize(s));
     cv->samples++;
-    return status_from_bits(bits);
+    return status_from_bits(*static_cast<volatile unsigned *>(&w.host->status));
 }
 
 int bd_cv3d_calculate_vector(bd_cv3d *cv) {

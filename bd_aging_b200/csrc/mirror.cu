@@ -6,9 +6,12 @@
 #include <curand_kernel.h>
 
 #include <algorithm>
+#include <atomic>
+#include <climits>
 #include <cmath>
 #include <cstring>
 #include <mutex>
+#include <thread>
 #include <type_traits>
 #include <vector>
 
@@ -46,31 +49,77 @@ unsigned long long current_context_id() {
     return get_id(c, &id) == CUDA_SUCCESS ? id + 1 : 0;  // +1: a valid id is never 0 here
 }
 
-DeviceWork *device_work() {
+namespace {
+constexpr int kSlots = 32;
+struct SlotState {
+    std::atomic_flag busy = ATOMIC_FLAG_INIT;
+};
+struct DeviceSlots {
+    HostWords *host = nullptr, *dev = nullptr;  // [kSlots] words, 128 bytes apart
+    double *accum = nullptr;                    // [kSlots][kWorkAccum], then the counters
+    unsigned long long ctx = 0;                 // context the pointers belong to
+    SlotState slot[kSlots];
+};
+constexpr size_t kWordStride = 128 / sizeof(HostWords);
+static_assert(128 % sizeof(HostWords) == 0, "slots on their own lines");
+
+DeviceSlots *device_slots() {
     static std::mutex mu;
-    static DeviceWork works[64];
+    static DeviceSlots all[64];
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return nullptr;
     const unsigned long long ctx = current_context_id();
     if (!ctx) return nullptr;
     std::lock_guard<std::mutex> lock(mu);
-    DeviceWork &w = works[dev];
-    if (w.ctx != ctx) {  // first use, or the context was destroyed (its memory with it)
-        w = DeviceWork{};
-        if (cudaMalloc(&w.status, 256) != cudaSuccess) return nullptr;
-        if (cudaMalloc(&w.accum, kWorkAccum * sizeof(double)) != cudaSuccess) return nullptr;
-        if (cudaMemset(w.status, 0, 256) != cudaSuccess) return nullptr;
-        w.ctx = ctx;
+    DeviceSlots &d = all[dev];
+    if (d.ctx != ctx) {  // first use, or the context was destroyed (its memory with it)
+        d.ctx = 0;
+        void *h = nullptr, *p = nullptr, *acc = nullptr;
+        if (cudaHostAlloc(&h, 128 * kSlots, cudaHostAllocMapped) != cudaSuccess) return nullptr;
+        const size_t sums = sizeof(double) * kWorkAccum * kSlots, bytes = sums + 256 * kSlots;
+        if (cudaHostGetDevicePointer(&p, h, 0) != cudaSuccess || cudaMalloc(&acc, bytes) != cudaSuccess) {
+            cudaFreeHost(h);
+            return nullptr;
+        }
+        if (cudaMemset(acc, 0, bytes) != cudaSuccess || cudaDeviceSynchronize() != cudaSuccess) {
+            cudaFreeHost(h);
+            cudaFree(acc);
+            return nullptr;
+        }
+        d.host = static_cast<HostWords *>(h);
+        d.dev = static_cast<HostWords *>(p);
+        d.accum = static_cast<double *>(acc);
+        d.ctx = ctx;
     }
-    return &w;
+    return &d;
+}
+}  // namespace
+
+CallSlot::CallSlot() {
+    DeviceSlots *d = device_slots();
+    if (!d) return;
+    int k = 0;
+    while (d->slot[k].busy.test_and_set(std::memory_order_acquire)) {
+        if (++k == kSlots) {
+            k = 0;
+            std::this_thread::yield();
+        }
+    }
+    state = &d->slot[k];
+    host = d->host + k * kWordStride;
+    dev = d->dev + k * kWordStride;
+    accum = d->accum + (size_t)k * kWorkAccum;
+    counter = reinterpret_cast<unsigned *>(d->accum + (size_t)kSlots * kWorkAccum) + 64 * k;
+    host->status = 0;
+}
+CallSlot::~CallSlot() {
+    if (state) static_cast<SlotState *>(state)->busy.clear(std::memory_order_release);
 }
 
-// Reset the status word, run nothing else; read it back after the kernels.
-static int read_status(DeviceWork *w, cudaStream_t s) {
-    unsigned bits = 0;
-    BD_CUDA_TRY(cudaMemcpyAsync(&bits, w->status, sizeof(unsigned), cudaMemcpyDeviceToHost, s));
+// Waits for the call's kernels and maps their status.
+static int read_status(const CallSlot &w, cudaStream_t s) {
     BD_CUDA_TRY(cudaStreamSynchronize(s));
-    return status_from_bits(bits);
+    return status_from_bits(*static_cast<volatile unsigned *>(&w.host->status));
 }
 
 // ------------------------------------------------------------ cell list
@@ -99,8 +148,26 @@ __global__ void k_cell_bin(const float *__restrict__ rr, int n, float csi, int n
     if (s < ntags) cell_vec[(long)c * ntags + s] = m;
     if (s + 1 >= ntags) set_status(st, kStatCellOverflow);  // main.cu:655 (nocup_max >= ntags)
 }
-// Slots in ascending particle order (the order cell_locate_hst produces).
+// Slots in ascending particle order (the order cell_locate_hst produces), the
+// unused ones -1.  G lanes per cell (ntags <= G): a lane holds a slot's entry
+// and counts the smaller ones by shuffles, so a cell is one load and one store
+// per slot, and the clear of cell_vec before the binning is saved.
+template <int G>
 __global__ void k_cell_sort(const int *nocup, int *cell_vec, int nc3, int ntags) {
+    const int c = (int)(((size_t)blockIdx.x * blockDim.x + threadIdx.x) / G), t = threadIdx.x % G;
+    const bool live = c < nc3;
+    const int k = live ? min(nocup[c], ntags) : 0;
+    int *v = cell_vec + (size_t)c * ntags;
+    const int key = t < k ? v[t] : INT_MAX;
+    int rank = 0;
+#pragma unroll
+    for (int u = 0; u < G; u++) rank += __shfl_sync(0xffffffffu, key, u, G) < key;
+    if (t < k) v[rank] = key;
+    else if (live && t < ntags) v[t] = -1;
+}
+// The same for more slots per cell, a thread per cell (unused slots cleared
+// before the binning).
+__global__ void k_cell_sort_long(const int *nocup, int *cell_vec, int nc3, int ntags) {
     int c = blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= nc3) return;
     int k = min(nocup[c], ntags);
@@ -113,20 +180,25 @@ __global__ void k_cell_sort(const int *nocup, int *cell_vec, int nc3, int ntags)
 }
 
 // ------------------------------------------------------------ forces
-// get_forces_same_dev / get_forces_diff_dev (get_forces.cu:297-558): one
-// thread per particle over the (2 nrange + 1)^3 cells around its own cell of
-// the partner species; pair selection with the reference's rounding
-// (min_image_f, dist2_rn), WCA-modified pair; results ADDED to ff/vir/pot.
-template <bool SAME>
+// get_forces_same_dev / get_forces_diff_dev (get_forces.cu:297-558): G lanes
+// per particle share the (2 nrange + 1)^3 cells around its own cell of the
+// partner species; pair selection with the reference's rounding (min_image_f,
+// dist2_rn), WCA-modified pair; results ADDED to ff/vir/pot.
+// Bound: the chain of loads position -> cell count -> cell entry -> partner
+// position, which a thread per particle walks 27 or 125 times with 110 threads
+// on an SM (16384 particles).  A warp per particle walks it once or four times
+// and fills the chip; with more particles fewer lanes each, and so fewer
+// instructions, win (launch_forces).
+template <bool SAME, int G, int W>
 __global__ void k_forces(const float *__restrict__ rr, float *ff, float *vir, float *pot,
                          const float *__restrict__ rr_o, const int *__restrict__ nocup,
                          const int *__restrict__ cell_vec, int n, int ncell, int ntags, int nrange, float csi,
                          float sigma, float side, unsigned *st) {
-    int m = blockIdx.x * blockDim.x + threadIdx.x;
-    if (m >= n) return;
+    const int m = (int)(((size_t)blockIdx.x * blockDim.x + threadIdx.x) / G), sub = threadIdx.x % G;
+    if (m >= n) return;  // the lanes of a particle leave together
     const float side_inv = __fdiv_rn(1.0f, side);
     const float cut2 = __fmul_rn(sigma, sigma);
-    float rx = rr[3 * m], ry = rr[3 * m + 1], rz = rr[3 * m + 2];
+    float rx = rr[3 * (size_t)m], ry = rr[3 * (size_t)m + 1], rz = rr[3 * (size_t)m + 2];
     int ii = (int)__fmul_rn(csi, rx), jj = (int)__fmul_rn(csi, ry), kk = (int)__fmul_rn(csi, rz);
     if (ii == ncell) ii--;
     if (jj == ncell) jj--;
@@ -137,36 +209,81 @@ __global__ void k_forces(const float *__restrict__ rr, float *ff, float *vir, fl
         jj = min(max(jj, 0), ncell - 1);
         kk = min(max(kk, 0), ncell - 1);
     }
-    float fx = ff[3 * m], fy = ff[3 * m + 1], fz = ff[3 * m + 2], v = vir[m], p = pot[m];
-    for (int di = -nrange; di <= nrange; di++)
-        for (int dj = -nrange; dj <= nrange; dj++)
-            for (int dk = -nrange; dk <= nrange; dk++) {
-                int ip = (ii + di + ncell) % ncell, jp = (jj + dj + ncell) % ncell, kp = (kk + dk + ncell) % ncell;
-                int c = ip + ncell * (jp + ncell * kp);
-                int occ = min(nocup[c], ntags);
-                const int *cv = cell_vec + (long)c * ntags;
-                for (int t = 0; t < occ; t++) {
-                    int nn = cv[t];
-                    if (SAME && nn == m) continue;
-                    float dx = min_image_f(__fsub_rn(rr_o[3 * nn], rx), side, side_inv);
-                    float dy = min_image_f(__fsub_rn(rr_o[3 * nn + 1], ry), side, side_inv);
-                    float dz = min_image_f(__fsub_rn(rr_o[3 * nn + 2], rz), side, side_inv);
-                    float d2 = dist2_rn(dx, dy, dz);
-                    if (d2 < cut2) {
-                        PairOut o = wca_modified_pair(sigma, d2, dx, dy, dz);
-                        fx += o.fx;
-                        fy += o.fy;
-                        fz += o.fz;
-                        p += o.pot;
-                        v += o.vir;
-                    }
-                }
+    float fx = 0.f, fy = 0.f, fz = 0.f, v = 0.f, p = 0.f;
+    if (G == 1) fx = ff[3 * (size_t)m], fy = ff[3 * (size_t)m + 1], fz = ff[3 * (size_t)m + 2], v = vir[m], p = pot[m];
+    const int w = W > 0 ? W : 2 * nrange + 1, cells = w * w * w, reach = W > 0 ? W / 2 : nrange;
+    auto wrap = [&](int k) {
+        while (k < 0) k += ncell;
+        while (k >= ncell) k -= ncell;
+        return k;
+    };
+    for (int t0 = sub; t0 < cells; t0 += G) {
+        // consecutive lanes take cells that follow one another in memory (x runs
+        // fastest there); a single thread keeps the reference's order of sums
+        const int slow = t0 / (w * w) - reach, fast = t0 % w - reach;
+        const int ip = wrap(ii + (G == 1 ? slow : fast)), jp = wrap(jj + t0 / w % w - reach),
+                  kp = wrap(kk + (G == 1 ? fast : slow));
+        int c = ip + ncell * (jp + ncell * kp);
+        int occ = min(nocup[c], ntags);
+        const int *cv = cell_vec + (long)c * ntags;
+#pragma unroll 2
+        for (int t = 0; t < occ; t++) {
+            int nn = cv[t];
+            if (SAME && nn == m) continue;
+            float dx = min_image_f(__fsub_rn(rr_o[3 * (size_t)nn], rx), side, side_inv);
+            float dy = min_image_f(__fsub_rn(rr_o[3 * (size_t)nn + 1], ry), side, side_inv);
+            float dz = min_image_f(__fsub_rn(rr_o[3 * (size_t)nn + 2], rz), side, side_inv);
+            float d2 = dist2_rn(dx, dy, dz);
+            if (d2 < cut2) {
+                PairOut o = wca_modified_pair(sigma, d2, dx, dy, dz);
+                fx += o.fx;
+                fy += o.fy;
+                fz += o.fz;
+                p += o.pot;
+                v += o.vir;
             }
-    ff[3 * m] = fx;
-    ff[3 * m + 1] = fy;
-    ff[3 * m + 2] = fz;
+        }
+    }
+    if (G > 1) {
+        const unsigned mask = __activemask();
+#pragma unroll
+        for (int o = G / 2; o; o >>= 1) {
+            fx += __shfl_xor_sync(mask, fx, o);
+            fy += __shfl_xor_sync(mask, fy, o);
+            fz += __shfl_xor_sync(mask, fz, o);
+            v += __shfl_xor_sync(mask, v, o);
+            p += __shfl_xor_sync(mask, p, o);
+        }
+        if (sub != 0) return;
+        fx += ff[3 * (size_t)m], fy += ff[3 * (size_t)m + 1], fz += ff[3 * (size_t)m + 2], v += vir[m], p += pot[m];
+    }
+    ff[3 * (size_t)m] = fx;
+    ff[3 * (size_t)m + 1] = fy;
+    ff[3 * (size_t)m + 2] = fz;
     vir[m] = v;
     pot[m] = p;
+}
+template <bool SAME, int G>
+static auto forces_kernel(int nrange) {
+    return nrange == 1 ? k_forces<SAME, G, 3> : nrange == 2 ? k_forces<SAME, G, 5> : k_forces<SAME, G, 0>;
+}
+template <bool SAME>
+static int launch_forces(const float *rr, float *ff, float *vir, float *pot, const float *rr_o, const int *nocup,
+                         const int *cell_vec, int n, int ncell, int ntags, int nrange, float csi, float sigma, float side,
+                         cudaStream_t s) {
+    CallSlot w;
+    if (!w.ok()) return BD_ERR_NOMEM;
+    // lanes per particle.  A call's time (us) with 32, 8 and 1 lanes over 27
+    // cells: 20, 24, 68 at 6000 particles; 30, 27, 74 at 16384; 64, 49, 76 at
+    // 60000; 255, 163, 159 at 300000; over 125 cells: 26, 41, 193 at 6000; 45,
+    // 46, 220 at 16384; 112, 106, 226 at 60000; 487, 402, 494 at 300000.
+    const int lanes = nrange > 1 ? (n <= 32768 ? 32 : 8) : n <= 8192 ? 32 : n <= 131072 ? 8 : 1;
+    auto kern = lanes == 32 ? forces_kernel<SAME, 32>(nrange) : lanes == 8 ? forces_kernel<SAME, 8>(nrange)
+                                                                          : forces_kernel<SAME, 1>(nrange);
+    kern<<<div_up((long)n * lanes, 128), 128, 0, s>>>(rr, ff, vir, pot, rr_o, nocup, cell_vec, n, ncell, ntags, nrange, csi,
+                                                      sigma, side, w.status());
+    BD_LAUNCH_CHECK();
+    return read_status(w, s);
 }
 
 // ------------------------------------------------------------ update
@@ -391,14 +508,15 @@ __global__ void __launch_bounds__(kGderThreads) k_gder(const GderArgs a) {
 // ------------------------------------------------------------ F_s, MSD
 // fself_isotropic (fself.cu:3-21) and the MSD loop (main.cu:776-792): per
 // particle float terms as in the reference, summed in FP64.
-// One FP64 partial per block, then one block adds the partials in index
-// order, so the result does not depend on the order in which blocks finish.
+// One FP64 partial per block; the last block to finish adds the partials in
+// index order into the call's host word, so the result does not depend on the
+// order in which blocks finish.
 constexpr int kDispThreads = 256, kDispMaxBlocks = 148 * 8;
-static_assert(kDispMaxBlocks + 1 <= kWorkAccum, "partials fit the workspace");
+static_assert(kDispMaxBlocks <= kWorkAccum, "partials fit the workspace");
 template <int KIND>  // 0: F_s, 1: MSD
 __global__ void __launch_bounds__(kDispThreads) k_disp_reduce(const float *__restrict__ raw,
                                                               const float *__restrict__ r0, int n, float q,
-                                                              double *part) {
+                                                              double *part, unsigned *counter, double *result) {
     double s = 0.0;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         float dx = raw[3 * i] - r0[3 * i], dy = raw[3 * i + 1] - r0[3 * i + 1], dz = raw[3 * i + 2] - r0[3 * i + 2];
@@ -411,40 +529,43 @@ __global__ void __launch_bounds__(kDispThreads) k_disp_reduce(const float *__res
         }
     }
     for (int o = 16; o; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
-    __shared__ double red[kDispThreads / 32];
+    __shared__ double red[kDispThreads];
+    __shared__ bool last;
     if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = s;
     __syncthreads();
     if (threadIdx.x == 0) {
         double t = 0.0;
         for (int w = 0; w < kDispThreads / 32; w++) t += red[w];
-        part[1 + blockIdx.x] = t;
+        part[blockIdx.x] = t;
+        __threadfence();
+        last = atomicAdd(counter, 1u) == gridDim.x - 1;
     }
-}
-// part[0] = sum of part[1 .. nblocks] in a fixed order
-__global__ void __launch_bounds__(kDispThreads) k_disp_finish(double *part, int nblocks) {
-    __shared__ double red[kDispThreads];
-    double s = 0.0;
-    for (int b = threadIdx.x; b < nblocks; b += blockDim.x) s += part[1 + b];
+    __syncthreads();
+    if (!last) return;
+    __threadfence();
+    s = 0.0;
+    for (int b = threadIdx.x; b < gridDim.x; b += blockDim.x) s += __ldcg(part + b);
     red[threadIdx.x] = s;
     __syncthreads();
     for (int w = kDispThreads / 2; w > 0; w >>= 1) {
         if (threadIdx.x < w) red[threadIdx.x] += red[threadIdx.x + w];
         __syncthreads();
     }
-    if (threadIdx.x == 0) part[0] = red[0];
+    if (threadIdx.x == 0) {
+        *result = red[0];
+        *counter = 0u;
+    }
 }
 
 static int disp_reduce(int kind, const float *raw, const float *r0, int n, float q, double *out, cudaStream_t s) {
-    DeviceWork *w = device_work();
-    if (!w) return BD_ERR_NOMEM;
+    CallSlot w;
+    if (!w.ok()) return BD_ERR_NOMEM;
     const int blocks = std::min(div_up(n, kDispThreads), kDispMaxBlocks);
-    if (kind == 0) k_disp_reduce<0><<<blocks, kDispThreads, 0, s>>>(raw, r0, n, q, w->accum);
-    else k_disp_reduce<1><<<blocks, kDispThreads, 0, s>>>(raw, r0, n, q, w->accum);
+    auto kern = kind == 0 ? k_disp_reduce<0> : k_disp_reduce<1>;
+    kern<<<blocks, kDispThreads, 0, s>>>(raw, r0, n, q, w.accum, w.counter, &w.dev->value);
     BD_LAUNCH_CHECK();
-    k_disp_finish<<<1, kDispThreads, 0, s>>>(w->accum, blocks);
-    BD_LAUNCH_CHECK();
-    BD_CUDA_TRY(cudaMemcpyAsync(out, w->accum, sizeof(double), cudaMemcpyDeviceToHost, s));
     BD_CUDA_TRY(cudaStreamSynchronize(s));
+    *out = *static_cast<volatile double *>(&w.host->value);
     return BD_OK;
 }
 
@@ -580,16 +701,17 @@ int bd_cell_locate(char type, const float *rr, int *nocup, int *cell_vec, const 
     const float csi = (float)(1.0 / (b ? p->cell_side_big : p->cell_side_sml));
     const int nc3 = ncell * ncell * ncell;
     cudaStream_t s = as_stream(stream);
-    DeviceWork *w = device_work();
-    if (!w) return BD_ERR_NOMEM;
-    BD_CUDA_TRY(cudaMemsetAsync(w->status, 0, sizeof(unsigned), s));
+    CallSlot w;
+    if (!w.ok()) return BD_ERR_NOMEM;
     BD_CUDA_TRY(cudaMemsetAsync(nocup, 0, sizeof(int) * (size_t)nc3, s));
-    BD_CUDA_TRY(cudaMemsetAsync(cell_vec, 0xff, sizeof(int) * (size_t)nc3 * ntags, s));
+    if (ntags > 32) BD_CUDA_TRY(cudaMemsetAsync(cell_vec, 0xff, sizeof(int) * (size_t)nc3 * ntags, s));
     if (n > 0) {
-        k_cell_bin<<<div_up(n, 256), 256, 0, s>>>(rr, n, csi, ncell, ntags, nocup, cell_vec, w->status);
+        k_cell_bin<<<div_up(n, 256), 256, 0, s>>>(rr, n, csi, ncell, ntags, nocup, cell_vec, w.status());
         BD_LAUNCH_CHECK();
     }
-    k_cell_sort<<<div_up(nc3, 256), 256, 0, s>>>(nocup, cell_vec, nc3, ntags);
+    if (ntags <= 16) k_cell_sort<16><<<div_up((long)nc3 * 16, 256), 256, 0, s>>>(nocup, cell_vec, nc3, ntags);
+    else if (ntags <= 32) k_cell_sort<32><<<div_up((long)nc3 * 32, 256), 256, 0, s>>>(nocup, cell_vec, nc3, ntags);
+    else k_cell_sort_long<<<div_up(nc3, 256), 256, 0, s>>>(nocup, cell_vec, nc3, ntags);
     BD_LAUNCH_CHECK();
     return read_status(w, s);
 }
@@ -605,14 +727,8 @@ int bd_get_forces_same(char type, const float *rr, float *ff, float *vir, float 
     const float csi = 1.0f / (b ? p->cell_side_big : p->cell_side_sml);
     const int ntags = b ? p->ntags_big : p->ntags_sml, ncell = b ? p->ncell_big : p->ncell_sml;
     const int nrange = b ? p->nrange_bb : p->nrange_ss;
-    cudaStream_t s = as_stream(stream);
-    DeviceWork *w = device_work();
-    if (!w) return BD_ERR_NOMEM;
-    BD_CUDA_TRY(cudaMemsetAsync(w->status, 0, sizeof(unsigned), s));
-    k_forces<true><<<div_up(n, 128), 128, 0, s>>>(rr, ff, vir, pot, rr, nocup, cell_vec, n, ncell, ntags, nrange,
-                                                   csi, sigma, p->side, w->status);
-    BD_LAUNCH_CHECK();
-    return read_status(w, s);
+    return launch_forces<true>(rr, ff, vir, pot, rr, nocup, cell_vec, n, ncell, ntags, nrange, csi, sigma, p->side,
+                               as_stream(stream));
 }
 
 int bd_get_forces_diff(char type, char type_other, const float *rr, float *ff, const float *rr_other, float *vir,
@@ -627,14 +743,8 @@ int bd_get_forces_diff(char type, char type_other, const float *rr, float *ff, c
     const float sigma = b ? 0.5f * (p->sigma_big + p->sigma_sml) : 0.5f * (p->sigma_sml + p->sigma_big);
     const int ntags = b ? p->ntags_sml : p->ntags_big, ncell = b ? p->ncell_sml : p->ncell_big;
     const int nrange = b ? p->nrange_bs : p->nrange_sb;
-    cudaStream_t s = as_stream(stream);
-    DeviceWork *w = device_work();
-    if (!w) return BD_ERR_NOMEM;
-    BD_CUDA_TRY(cudaMemsetAsync(w->status, 0, sizeof(unsigned), s));
-    k_forces<false><<<div_up(n, 128), 128, 0, s>>>(rr, ff, vir, pot, rr_other, nocup_o, cell_o, n, ncell, ntags,
-                                                    nrange, csi, sigma, p->side, w->status);
-    BD_LAUNCH_CHECK();
-    return read_status(w, s);
+    return launch_forces<false>(rr, ff, vir, pot, rr_other, nocup_o, cell_o, n, ncell, ntags, nrange, csi, sigma, p->side,
+                                as_stream(stream));
 }
 
 size_t bd_rng_state_size(void) { return sizeof(curandState); }

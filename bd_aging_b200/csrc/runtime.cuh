@@ -19,17 +19,30 @@ inline cudaStream_t as_stream(void *s) { return reinterpret_cast<cudaStream_t>(s
 // context and every address in it, changes the id.  0 when none can be had.
 unsigned long long current_context_id();
 
-// Per-device workspace for the mirror entry points: a status word and the
-// FP64 partial sums of the fixed-order reductions.  Allocated on first use in
-// each device's context (again after a device reset) and kept until exit.
-constexpr int kWorkAccum = 2048;  // FP64 slots: one per reduction block plus the result
-struct DeviceWork {
-    unsigned *status = nullptr;   // device status word (kStat* bits)
-    double *accum = nullptr;      // kWorkAccum FP64 partial sums
-    unsigned long long ctx = 0;   // context the pointers belong to
+// What a synchronous mirror call needs on its device, one slot per call in
+// flight: a status word and a result in host memory that the kernels write to
+// directly (no clear before and no copy after them; the stream's
+// synchronisation is all the call waits for), and the FP64 partial sums of the
+// fixed-order reductions.  The slots are allocated on first use in each
+// device's context (again after a device reset) and kept until exit.
+constexpr int kWorkAccum = 2048;  // FP64 slots: one per reduction block
+struct HostWords {
+    unsigned status;  // kStat* bits
+    double value;
 };
-
-DeviceWork *device_work();  // nullptr on allocation failure
+struct CallSlot {
+    HostWords *host = nullptr;     // host address
+    HostWords *dev = nullptr;      // the same words as kernels see them
+    double *accum = nullptr;       // kWorkAccum FP64 partial sums
+    unsigned *counter = nullptr;   // finished blocks of a reduction, zero between calls
+    void *state = nullptr;
+    CallSlot();                    // takes a free slot of the current device (waits when all are taken)
+    ~CallSlot();
+    CallSlot(const CallSlot &) = delete;
+    CallSlot &operator=(const CallSlot &) = delete;
+    bool ok() const { return host != nullptr; }  // false: allocation failed
+    unsigned *status() const { return &dev->status; }
+};
 
 // Map the device status word to a BD_* code.  A non-finite position also
 // piles particles into one cell, so it is reported before the overflow.

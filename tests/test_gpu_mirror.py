@@ -73,6 +73,26 @@ def test_forces_match_reference(golden, name):
         np.testing.assert_allclose(v, ref, rtol=2e-5, atol=2e-5 * np.abs(ref).max(), err_msg=k)
 
 
+@pytest.mark.parametrize("nb,ns,ntags", [(1, 2, 8), (33, 31, 9), (700, 500, 16), (700, 500, 17), (700, 500, 40),
+                                         (8200, 33000, 16), (131073, 40000, 16)])
+def test_cell_sort_and_force_paths_match_the_oracle(nb, ns, ntags):
+    """16, 32 and more slots per cell (sorted by 16 or 32 lanes or a thread), a
+    warp, eight lanes or a thread per particle by their number: cell lists exact, forces
+    within the rounding of a float sum in another order."""
+    side = CF.side_from_phi(max(nb, 60), max(ns, 60), 0.45)
+    pos = CF.lattice_config(nb, ns, side, 17)
+    p = O.setup_params(side, nb, ns, float(CF.SIGMA_BIG), float(CF.SIGMA_SML), ntags=(ntags, ntags))
+    pp = B.Parametros.from_buffer_copy(bytes(p))
+    for sp, rr in (("b", pos[:nb]), ("s", pos[nb:])):
+        nocup, cell = cells(pp, sp, dev(rr))
+        ref = O.cell_locate(p, sp, rr)
+        np.testing.assert_array_equal(host(nocup), ref[0])
+        np.testing.assert_array_equal(host(cell), ref[1])
+    out, ref = forces_four_calls(pp, pos[:nb], pos[nb:]), O.ref_forces(p, pos[:nb].copy(), pos[nb:].copy())
+    for k, v in out.items():
+        np.testing.assert_allclose(v, ref[k], rtol=2e-5, atol=2e-5 * np.abs(ref[k]).max(), err_msg=k)
+
+
 @pytest.mark.parametrize("name", SYSTEMS)
 def test_update_noise_bit_exact(golden, name):
     p = params(golden, name)
