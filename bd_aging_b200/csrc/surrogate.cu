@@ -8,15 +8,17 @@
 //   forward   Z_l  = H_{l-1} W_l^T + b_l        A = H_{l-1} [B][K_l], B = W_l  [N_l][K_l]
 //   input     dH_{l-1} = dZ_l W_l               A = dZ_l    [B][N_l], B = W_l^T [K_l][N_l]
 //   weights   dW_l = dZ_l^T H_{l-1}             A = dZ_l^T  [N_l][B], B = H_{l-1}^T [K_l][B]
-// The forward and input-gradient GEMMs of a training step run in one launch
-// of the fused kernel (mlp_chain.cuh), which keeps each 128-row block's
-// activations and gradients in shared memory and writes H_l^T and dZ_l^T for
-// the weight-gradient GEMMs (umma.cuh).  dW is split over the batch (256
+// A training step is three launches: the fused kernel (mlp_chain.cuh) draws
+// the minibatch and runs every forward and input-gradient GEMM, keeping each
+// 32-row block's activations and gradients on chip and writing H_l^T and
+// dZ_l^T; one launch runs every weight-gradient GEMM (umma.cuh); one launch
+// sums the bias gradients and applies Adam.  dW is split over the batch (256
 // rows per CTA) into FP32 partials that the Adam kernel adds in a fixed
 // order, so a training step is deterministic.
 #include <cuda.h>
 #include <cuda_bf16.h>
 
+#include <algorithm>
 #include <cmath>
 #include <cstring>
 #include <new>
@@ -29,7 +31,8 @@
 namespace bd {
 namespace {
 
-using umma::GemmArgs;
+using umma::GemmJob;
+using umma::GemmTable;
 using umma::kBK;
 using umma::kBM;
 using umma::kBN;
@@ -54,7 +57,7 @@ EncodeTiledFn encode_fn() {
 
 // 2-D BF16 row-major matrix [rows][cols] as a TMA map with a box of 64
 // columns (128 bytes, 128-byte swizzle) by box_rows rows (kBM for A
-// operands, kBN for B operands); out-of-range rows and columns read as zero.
+// operands, the tile width for B operands); out-of-range rows and columns read as zero.
 int make_tmap(CUtensorMap *map, const void *ptr, int rows, int cols, int box_rows) {
     EncodeTiledFn enc = encode_fn();
     if (!enc) return BD_ERR_CUDA;
@@ -73,16 +76,26 @@ int make_tmap(CUtensorMap *map, const void *ptr, int rows, int cols, int box_row
 // called outside stream capture (create, direct GEMM)
 int set_gemm_attrs() {
     BD_CUDA_TRY(cudaFuncSetAttribute(umma::k_umma_gemm, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     umma::kSmemBytes));
+                                     umma::gemm_smem(umma::kMaxBN)));
     BD_CUDA_TRY(cudaFuncSetAttribute(umma::k_mlp_chain, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                      umma::kChainSmem));
     return BD_OK;
 }
 
-int launch_gemm(const CUtensorMap &a, const CUtensorMap &b, const GemmArgs &g, cudaStream_t st) {
-    if (g.k_split % kBK || g.k_split > umma::kMaxChunks * kBK || g.k_split < kBK) return BD_ERR_ARG;
-    dim3 grid(div_up(g.M, kBM), div_up(g.N, kBN), div_up(g.K, g.k_split));
-    umma::k_umma_gemm<<<grid, umma::kThreads, umma::kSmemBytes, st>>>(a, b, g);
+// the table's GEMMs side by side; fills in each job's first block
+int launch_gemms(GemmTable &t, cudaStream_t st) {
+    int blocks = 0, bn = 0;
+    for (int i = 0; i < t.n_jobs; i++) {
+        GemmJob &g = t.job[i];
+        if (g.k_split % kBK || g.k_split > umma::kMaxChunks * kBK || g.k_split < kBK) return BD_ERR_ARG;
+        if (g.bn % kBN || g.bn < kBN || g.bn > umma::kMaxBN) return BD_ERR_ARG;
+        const long long n = (long long)div_up(g.M, kBM) * div_up(g.N, g.bn) * div_up(g.K, g.k_split);
+        if (n > 0x7fffffffLL - blocks) return BD_ERR_ARG;
+        g.first = blocks;
+        blocks += (int)n;
+        bn = std::max(bn, g.bn);
+    }
+    umma::k_umma_gemm<<<blocks, umma::kThreads, umma::gemm_smem(bn), st>>>(t);
     BD_LAUNCH_CHECK();
     return BD_OK;
 }
@@ -96,152 +109,157 @@ __global__ void k_sum_splits(const float *part, int splits, size_t n, float *out
     out[i] = s;
 }
 
-// counter-based sample index (splitmix64 of seed, step, row)
-__device__ __forceinline__ unsigned long long mix64(unsigned long long x) {
-    x += 0x9E3779B97F4A7C15ULL;
-    x = (x ^ (x >> 30)) * 0xBF58476D1CE4E5B9ULL;
-    x = (x ^ (x >> 27)) * 0x94D049BB133111EBULL;
-    return x ^ (x >> 31);
-}
-
-// minibatch rows: x (FP32 [n_data][n_in]) -> X0 [B][k0] and X0^T [k0][B]
-// (BF16, zero padded), targets -> T [n_out_pad][B].  A block takes 32 rows
-// (lane = row), its warps split the columns: the transposed writes of a warp
-// are 32 consecutive rows.
-constexpr int kGatherRows = 32;
-__global__ void k_gather(const float *x, const float *y, int n_data, int n_in, int n_out, int k0, int n_out_pad,
-                         int B, const int *rows, const long long *step, unsigned long long seed, __nv_bfloat16 *X0,
-                         __nv_bfloat16 *X0t, float *T) {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-    const int r = blockIdx.x * kGatherRows + lane;
-    if (r >= B) return;
-    int src;
-    if (rows) {
-        src = rows[r];
-    } else {
-        src = (int)(mix64(seed ^ mix64((unsigned long long)*step * 1315423911ULL + (unsigned long long)r)) %
-                    (unsigned long long)n_data);
-    }
-    const bool valid = src >= 0 && src < n_data;
-    for (int k = warp; k < k0; k += nw) {
-        const float v = (valid && k < n_in) ? x[(size_t)src * n_in + k] : 0.f;
-        const __nv_bfloat16 b = __float2bfloat16_rn(v);
-        X0[(size_t)r * k0 + k] = b;
-        X0t[(size_t)k * B + r] = b;
-    }
-    if (T)  // targets transposed [n_out_pad][B], as the loss epilogue reads them
-        for (int k = warp; k < n_out_pad; k += nw)
-            T[(size_t)k * B + r] = (valid && k < n_out) ? y[(size_t)src * n_out + k] : 0.f;
-}
-
-// Bias gradients of every layer in one launch: block `row` of the layer
-// table sums dZ_l^T[n][:] over the batch (16-byte loads, a fixed order: the
-// thread's strided slice, then the warp, then the block's warps).
+// Bias gradients: row n of layer l's dZ_l^T summed over the batch by one warp,
+// in the fixed order of eight strided slices (16-byte loads), each a shuffle
+// tree, added in turn.  The slices are independent chains, which keeps enough
+// loads in flight for one warp.
 struct BiasGradArgs {
     const __nv_bfloat16 *dzt[umma::kChainMaxLayers];  // [N_l][B]
     float *db[umma::kChainMaxLayers];                 // [N_l]
-    int first[umma::kChainMaxLayers + 1];             // first block of each layer
+    int first[umma::kChainMaxLayers + 1];             // first row of each layer
     int L, B;                                         // B a multiple of 8
 };
-__global__ void k_bias_grads(const __grid_constant__ BiasGradArgs a) {
-    const int row = blockIdx.x;
-    int l = 0;
-    while (l + 1 < a.L && row >= a.first[l + 1]) l++;
-    const int n = row - a.first[l];
-    const uint4 *src = reinterpret_cast<const uint4 *>(a.dzt[l] + (size_t)n * a.B);
-    float sum = 0.f;
-    for (int i = threadIdx.x; i < a.B / 8; i += blockDim.x) {
-        const uint4 v = src[i];
-        const __nv_bfloat162 *h = reinterpret_cast<const __nv_bfloat162 *>(&v);
+constexpr int kBiasSlices = 8;
+__device__ __forceinline__ float bias_row_sum(const __nv_bfloat16 *row, int B, int lane) {
+    const uint4 *src = reinterpret_cast<const uint4 *>(row);
+    float sum[kBiasSlices];
 #pragma unroll
-        for (int j = 0; j < 4; j++) {
-            const float2 f = __bfloat1622float2(h[j]);
-            sum += f.x;
-            sum += f.y;
+    for (int w = 0; w < kBiasSlices; w++) sum[w] = 0.f;
+    for (int i0 = 0; i0 < B / 8; i0 += 32 * kBiasSlices) {
+        uint4 v[kBiasSlices];
+#pragma unroll
+        for (int w = 0; w < kBiasSlices; w++) {
+            const int i = i0 + w * 32 + lane;
+            v[w] = i < B / 8 ? src[i] : make_uint4(0u, 0u, 0u, 0u);
+        }
+#pragma unroll
+        for (int w = 0; w < kBiasSlices; w++) {
+            const __nv_bfloat162 *h = reinterpret_cast<const __nv_bfloat162 *>(&v[w]);
+#pragma unroll
+            for (int j = 0; j < 4; j++) {
+                const float2 f = __bfloat1622float2(h[j]);
+                sum[w] += f.x;
+                sum[w] += f.y;
+            }
         }
     }
+    float t = 0.f;
 #pragma unroll
-    for (int off = 16; off > 0; off >>= 1) sum += __shfl_down_sync(0xffffffffu, sum, off);
-    __shared__ float red[32];
-    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = sum;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        float t = 0.f;
-        for (int w = 0; w < (int)(blockDim.x >> 5); w++) t += red[w];
-        a.db[l][n] = t;
+    for (int w = 0; w < kBiasSlices; w++) {
+#pragma unroll
+        for (int off = 16; off > 0; off >>= 1) sum[w] += __shfl_down_sync(0xffffffffu, sum[w], off);
+        t += sum[w];
     }
+    return t;  // of lane 0
+}
+__device__ __forceinline__ int layer_of_row(const int *first, int L, int row) {
+    int l = 0;
+    while (l + 1 < L && row >= first[l + 1]) l++;
+    return l;
+}
+constexpr int kBiasRows = 8;  // rows (warps) per block
+__global__ void k_bias_grads(const __grid_constant__ BiasGradArgs a) {
+    const int row = blockIdx.x * kBiasRows + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+    if (row >= a.first[a.L]) return;
+    const int l = layer_of_row(a.first, a.L, row), n = row - a.first[l];
+    const float g = bias_row_sum(a.dzt[l] + (size_t)n * a.B, a.B, lane);
+    if (lane == 0) a.db[l][n] = g;
 }
 
 struct AdamArgs {
     float lr, b1, b2, eps;
-    const long long *step;  // number of updates so far (incremented by the caller's counter kernel)
+    const long long *step;  // number of this update (1 for the first)
 };
-// Every layer's weights and biases in one launch: element i of the table
-// (weights of layer 0, 1, ... then biases of layer 0, 1, ...).  Weights are
-// updated in [k][n] order (the gradient is the sum of the split partials,
-// stored [splits][K][N] by the weight-gradient GEMM); the FP32 master weights
-// and the moments are kept in that order too, so every FP32 access is
-// coalesced.  Writes the BF16 copies W [N][K] and W^T [K][N].  The
-// bias-correction denominators 1 - b^t are computed once per block.
+// Every layer's weights and biases in one launch.  The first blocks take tiles
+// of 16 k by 64 n of the weights of layer 0, 1, ...: the gradient is the sum of
+// the split partials, stored [splits][K][N] by the weight-gradient GEMM, and
+// the FP32 master weights and moments are kept in that order too, so a thread's
+// four n are one 16-byte access each.  It writes the BF16 copies W^T [K][N]
+// directly and W [N][K] through shared memory in 32-byte runs (written lane by
+// lane, each 2-byte store touched a sector of its own).  The other blocks sum
+// eight bias gradients each, a warp a row, and update the biases.
+// What bounds it: the partials, 14.7 MB at the 256-wide network and a batch of
+// 4096, which the GEMM has just left in L2.
+// 9.1 us at that size (before: 13, and 5 and 2.5 for the bias sums' and the
+// step counter's own launches).
+constexpr int kAdamK = 16, kAdamN = 64;
 struct AdamTable {
     float *w[umma::kChainMaxLayers], *wm[umma::kChainMaxLayers], *wv[umma::kChainMaxLayers];
     const float *part[umma::kChainMaxLayers];
     __nv_bfloat16 *wb[umma::kChainMaxLayers], *wbt[umma::kChainMaxLayers];
     float *b[umma::kChainMaxLayers], *bm[umma::kChainMaxLayers], *bv[umma::kChainMaxLayers];
-    const float *db[umma::kChainMaxLayers];
     int N[umma::kChainMaxLayers], K[umma::kChainMaxLayers];
     int n_live[umma::kChainMaxLayers], k_live[umma::kChainMaxLayers];
-    long long first_w[umma::kChainMaxLayers + 1];  // prefix of N K over the layers
-    int first_b[umma::kChainMaxLayers + 1];        // prefix of N over the layers
+    int first_w[umma::kChainMaxLayers + 1];  // first weight tile of each layer
     int L, splits;
+    BiasGradArgs bias;                       // db unused
 };
-__global__ void k_adam_all(const __grid_constant__ AdamTable t, AdamArgs a) {
+__device__ __forceinline__ float adam_update(const AdamArgs &a, const float *corr, float w, float g, float &m, float &v) {
+    m = a.b1 * m + (1.f - a.b1) * g;
+    v = a.b2 * v + (1.f - a.b2) * g * g;
+    const float mh = m / corr[0], vh = v / corr[1];
+    return w - a.lr * mh / (sqrtf(vh) + a.eps);
+}
+__global__ void __launch_bounds__(256) k_adam_all(const __grid_constant__ AdamTable t, AdamArgs a) {
     __shared__ float corr[2];
-    if (threadIdx.x == 0) {
-        const float tt = (float)(*a.step + 1);
-        corr[0] = 1.f - powf(a.b1, tt);
-        corr[1] = 1.f - powf(a.b2, tt);
-    }
-    __syncthreads();
-    const long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    const long long nw = t.first_w[t.L];
-    if (e < nw) {
-        int l = 0;
-        while (l + 1 < t.L && e >= t.first_w[l + 1]) l++;
-        const size_t i = (size_t)(e - t.first_w[l]);  // [k][n] order
-        const int N = t.N[l], K = t.K[l];
-        const int k = (int)(i / N), n = (int)(i % N);
-        float gsum = 0.f;
-        for (int s = 0; s < t.splits; s++) gsum += t.part[l][(size_t)s * N * K + i];
-        float wv = t.w[l][i];
-        if (n < t.n_live[l] && k < t.k_live[l]) {
-            const float mm = a.b1 * t.wm[l][i] + (1.f - a.b1) * gsum;
-            const float vv = a.b2 * t.wv[l][i] + (1.f - a.b2) * gsum * gsum;
-            t.wm[l][i] = mm;
-            t.wv[l][i] = vv;
-            const float mh = mm / corr[0], vh = vv / corr[1];
-            wv -= a.lr * mh / (sqrtf(vh) + a.eps);
-            t.w[l][i] = wv;
+    __shared__ __nv_bfloat16 tile[kAdamK][kAdamN + 2];
+    if (threadIdx.x < 2) corr[threadIdx.x] = 1.f - powf(threadIdx.x ? a.b2 : a.b1, (float)*a.step);
+    const int tiles = t.first_w[t.L];
+    if ((int)blockIdx.x < tiles) {
+        const int l = layer_of_row(t.first_w, t.L, blockIdx.x);
+        const int N = t.N[l], K = t.K[l], ti = blockIdx.x - t.first_w[l];
+        const int k0 = ti / (N / kAdamN) * kAdamK, n0 = ti % (N / kAdamN) * kAdamN;
+        const int kk = threadIdx.x >> 4, nn = (threadIdx.x & 15) * 4, k = k0 + kk, n = n0 + nn;
+        const size_t i = (size_t)k * N + n;
+        const float *part = t.part[l] + i;
+        float g[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll 8
+        for (int s = 0; s < t.splits; s++) {
+            const float4 p = *reinterpret_cast<const float4 *>(part + (size_t)s * N * K);
+            g[0] += p.x;
+            g[1] += p.y;
+            g[2] += p.z;
+            g[3] += p.w;
         }
-        const __nv_bfloat16 bv = __float2bfloat16_rn(wv);
-        t.wb[l][(size_t)n * K + k] = bv;
-        t.wbt[l][i] = bv;
+        __align__(16) float w[4], m[4], v[4];
+        *reinterpret_cast<float4 *>(w) = *reinterpret_cast<const float4 *>(t.w[l] + i);
+        *reinterpret_cast<float4 *>(m) = *reinterpret_cast<const float4 *>(t.wm[l] + i);
+        *reinterpret_cast<float4 *>(v) = *reinterpret_cast<const float4 *>(t.wv[l] + i);
+        __syncthreads();
+        if (k < t.k_live[l]) {
+#pragma unroll
+            for (int j = 0; j < 4; j++)
+                if (n + j < t.n_live[l]) w[j] = adam_update(a, corr, w[j], g[j], m[j], v[j]);
+            *reinterpret_cast<float4 *>(t.w[l] + i) = *reinterpret_cast<float4 *>(w);
+            *reinterpret_cast<float4 *>(t.wm[l] + i) = *reinterpret_cast<float4 *>(m);
+            *reinterpret_cast<float4 *>(t.wv[l] + i) = *reinterpret_cast<float4 *>(v);
+        }
+        __align__(8) __nv_bfloat162 q[2] = {__floats2bfloat162_rn(w[0], w[1]), __floats2bfloat162_rn(w[2], w[3])};
+        *reinterpret_cast<uint2 *>(t.wbt[l] + i) = *reinterpret_cast<uint2 *>(q);
+        *reinterpret_cast<__nv_bfloat162 *>(&tile[kk][nn]) = q[0];
+        *reinterpret_cast<__nv_bfloat162 *>(&tile[kk][nn + 2]) = q[1];
+        __syncthreads();
+        const int tn = threadIdx.x >> 2, tk = (threadIdx.x & 3) * 4;
+        __nv_bfloat16 o[4];
+#pragma unroll
+        for (int j = 0; j < 4; j++) o[j] = tile[tk + j][tn];
+        __align__(8) __nv_bfloat162 oq[2] = {__nv_bfloat162(o[0], o[1]), __nv_bfloat162(o[2], o[3])};
+        *reinterpret_cast<uint2 *>(t.wb[l] + (size_t)(n0 + tn) * K + k0 + tk) = *reinterpret_cast<uint2 *>(oq);
         return;
     }
-    const long long j = e - nw;
-    if (j >= t.first_b[t.L]) return;
-    int l = 0;
-    while (l + 1 < t.L && j >= t.first_b[l + 1]) l++;
-    const int n = (int)(j - t.first_b[l]);
+    __syncthreads();
+    const int row = ((int)blockIdx.x - tiles) * kBiasRows + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+    if (row >= t.bias.first[t.L]) return;
+    const int l = layer_of_row(t.bias.first, t.L, row), n = row - t.bias.first[l];
     if (n >= t.n_live[l]) return;
-    const float g = t.db[l][n];
-    const float mm = a.b1 * t.bm[l][n] + (1.f - a.b1) * g;
-    const float vv = a.b2 * t.bv[l][n] + (1.f - a.b2) * g * g;
-    t.bm[l][n] = mm;
-    t.bv[l][n] = vv;
-    t.b[l][n] -= a.lr * (mm / corr[0]) / (sqrtf(vv / corr[1]) + a.eps);
+    const float g = bias_row_sum(t.bias.dzt[l] + (size_t)n * t.bias.B, t.bias.B, lane);
+    if (lane == 0) {
+        float m = t.bm[l][n], v = t.bv[l][n];
+        t.b[l][n] = adam_update(a, corr, t.b[l][n], g, m, v);
+        t.bm[l][n] = m;
+        t.bv[l][n] = v;
+    }
 }
-__global__ void k_count(long long *step) { *step += 1; }
 // BF16 copies W [N][K] and W^T [K][N] of the FP32 master weights (kept [K][N])
 __global__ void k_to_bf16(const float *w, int N, int K, __nv_bfloat16 *wb, __nv_bfloat16 *wbt) {
     const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;  // [k][n] order
@@ -250,6 +268,35 @@ __global__ void k_to_bf16(const float *w, int N, int K, __nv_bfloat16 *wb, __nv_
     const __nv_bfloat16 b = __float2bfloat16_rn(w[i]);
     wb[(size_t)n * K + k] = b;
     wbt[i] = b;
+}
+
+// The flat host order (for each layer W [N_l][K_l] then b [N_l], live sizes)
+// of the parameters, or of the gradients (sums of the split partials), written
+// on the device, so that one copy of the live values replaces a padded copy
+// and a host transpose a layer.  Element order [k][n]: reads coalesce.
+struct FlatTable {
+    const float *w[umma::kChainMaxLayers];   // [splits][K][N]
+    const float *b[umma::kChainMaxLayers];
+    int N[umma::kChainMaxLayers], K[umma::kChainMaxLayers];
+    int n_live[umma::kChainMaxLayers], k_live[umma::kChainMaxLayers];
+    int out[umma::kChainMaxLayers];          // first flat element of the layer
+    int first[umma::kChainMaxLayers + 1];    // prefix of (K + 1) N: the weights, then the biases
+    int L, splits;
+};
+__global__ void k_flatten(const __grid_constant__ FlatTable t, float *flat) {
+    const int e = blockIdx.x * blockDim.x + threadIdx.x;
+    if (e >= t.first[t.L]) return;
+    const int l = layer_of_row(t.first, t.L, e), i = e - t.first[l];
+    const int N = t.N[l], K = t.K[l], k = i / N, n = i % N;
+    if (n >= t.n_live[l]) return;
+    float *out = flat + t.out[l];
+    if (k == K) {
+        out[(size_t)t.n_live[l] * t.k_live[l] + n] = t.b[l][n];
+    } else if (k < t.k_live[l]) {
+        float s = 0.f;
+        for (int j = 0; j < t.splits; j++) s += t.w[l][(size_t)j * N * K + i];
+        out[(size_t)n * t.k_live[l] + k] = s;
+    }
 }
 
 }  // namespace
@@ -267,26 +314,28 @@ struct bd_surrogate {
     // parameters (FP32 master weights [K][N] and Adam moments in that order, biases), BF16 copies
     std::vector<float *> w, b, wm, wv, bm, bv;
     std::vector<__nv_bfloat16 *> wb, wbt;
-    // activations (BF16 row-major and transposed), pre-activations FP32
-    __nv_bfloat16 *x0 = nullptr;          // input X0 [B][K_0]
+    // activations and gradients the weight-gradient GEMMs read
     std::vector<__nv_bfloat16 *> ht;      // ht[0] = X0^T; ht[l+1] = H_l^T, output of hidden layer l [N_l][B]
-    std::vector<float *> z;               // z[l] pre-activation of layer l, transposed [N_l][B]
+    std::vector<float *> dg;              // gelu'(Z_l) [N_l][B] of the hidden layers tensor memory has no room for
     std::vector<__nv_bfloat16 *> dzt;     // dZ_l^T, gradient w.r.t. z[l] [N_l][B]
-    float *y = nullptr, *t = nullptr, *tw = nullptr;  // output [128][B], target [128][B] (transposed), weights
+    float *tw = nullptr;                  // loss weight per output
     float *part = nullptr;            // weight-gradient split partials [splits][K_l][N_l] per layer
     std::vector<float *> db;          // bias gradients
-    float *loss_part = nullptr;
+    float *flat = nullptr;            // parameters or gradients in the flat host order
     long long *step = nullptr;
+    // loss partials, then the error flag, copied together to the pinned words
+    float *loss_part = nullptr;
     unsigned *err = nullptr;
+    float *host = nullptr;
+    // inputs and outputs of predict and gradients on the device, kept (pred_rows rows)
+    float *px = nullptr, *py = nullptr;
+    int pred_rows = 0;
     float *data_x = nullptr, *data_y = nullptr;
     int n_data = 0;
     unsigned long long seed = 1;
-    // TMA maps: X0 (box 128 rows), the weight-gradient GEMMs' operands dZ_l^T and
-    // H_{l-1}^T, and W_l, W_l^T in boxes of a quarter of their rows (one CTA of a
-    // fused kernel's cluster each)
-    CUtensorMap tm_x;
+    // TMA maps: the weight-gradient GEMMs' operands dZ_l^T and H_{l-1}^T, and
+    // the fused kernel's W_l, W_l^T
     std::vector<CUtensorMap> tm_ht, tm_dzt, tm_w, tm_wt;
-    cudaGraphExec_t graph = nullptr;
     float lr = 1e-3f;
     int loss_cells = 0;
     int ksplit = 256;
@@ -295,7 +344,6 @@ struct bd_surrogate {
 namespace {
 
 void free_surrogate(bd_surrogate *s) {
-    if (s->graph) cudaGraphExecDestroy(s->graph);
     auto F = [](void *p) {
         if (p) cudaFree(p);
     };
@@ -308,112 +356,106 @@ void free_surrogate(bd_surrogate *s) {
     for (auto *p : s->wb) F(p);
     for (auto *p : s->wbt) F(p);
     for (auto *p : s->ht) F(p);
-    for (auto *p : s->z) F(p);
+    for (auto *p : s->dg) F(p);
     for (auto *p : s->dzt) F(p);
     for (auto *p : s->db) F(p);
-    F(s->x0); F(s->y); F(s->t); F(s->tw); F(s->part); F(s->loss_part); F(s->step); F(s->err); F(s->data_x);
-    F(s->data_y);
+    F(s->tw); F(s->part); F(s->flat); F(s->step); F(s->loss_part); F(s->data_x); F(s->data_y); F(s->px); F(s->py);
+    if (s->host) cudaFreeHost(s->host);
     if (s->stream) cudaStreamDestroy(s->stream);
     delete s;
 }
 
-int sg_status(bd_surrogate *s) {
-    unsigned e = 0;
-    BD_CUDA_TRY(cudaMemcpyAsync(&e, s->err, sizeof(unsigned), cudaMemcpyDeviceToHost, s->stream));
+// waits for the stream's work; the loss partials and the error flag come over
+// in one copy to pinned memory
+int sg_finish(bd_surrogate *s, double *loss_sum) {
+    BD_CUDA_TRY(cudaMemcpyAsync(s->host, s->loss_part, (size_t)(s->loss_cells + 1) * 4, cudaMemcpyDeviceToHost,
+                                s->stream));
     BD_CUDA_TRY(cudaStreamSynchronize(s->stream));
+    if (loss_sum) {
+        double sum = 0;
+        for (int i = 0; i < s->loss_cells; i++) sum += s->host[i];
+        *loss_sum = sum;
+    }
+    unsigned e;
+    std::memcpy(&e, s->host + s->loss_cells, 4);
     return e ? BD_ERR_TIMEOUT : BD_OK;
 }
 
-GemmArgs base_args(bd_surrogate *s) {
-    GemmArgs g;
-    std::memset(&g, 0, sizeof(g));
-    g.err = s->err;
-    g.k_split = 256;
-    return g;
-}
-
-// The forward pass of every 128-row block of the batch, and in training its
-// loss gradient and input-gradient chain (dZ_l for every layer), in one
-// launch of k_mlp_chain (a cluster of four CTAs per block).
-int chain_launch(bd_surrogate *s, bool train) {
+// The fused kernel (a CTA per 32 rows): training (`train`)
+// on the batch, from the training set (`draw`) or from rows in order, with the
+// loss gradient and every dZ_l; or the outputs y of `rows` rows of x.
+int chain_launch(bd_surrogate *s, bool train, bool draw, const float *x, const float *target, int rows, float *y) {
     umma::ChainMaps maps;
     std::memset(&maps, 0, sizeof(maps));
-    maps.x = s->tm_x;
     umma::ChainArgs g;
     std::memset(&g, 0, sizeof(g));
     g.L = s->L;
-    g.M = s->batch;
+    g.M = train ? s->batch : rows;
     g.backward = train ? 1 : 0;
     for (int l = 0; l < s->L; l++) {
         maps.w[l] = s->tm_w[l];
         maps.wt[l] = s->tm_wt[l];
-        const bool hidden = l < s->L - 1;
-        g.lay[l] = {s->Kp[l], s->Np[l], s->b[l], hidden ? s->z[l] : s->y, hidden ? s->ht[l + 1] : nullptr, s->dzt[l]};
+        g.lay[l] = {s->Kp[l], s->Np[l], s->b[l], s->dg[l], l < s->L - 1 ? s->ht[l + 1] : nullptr, s->dzt[l]};
     }
+    g.x = x;
+    g.n_data = rows;
+    g.n_in = s->n_in;
+    g.step = draw ? s->step : nullptr;
+    g.seed = s->seed;
+    g.n_out = s->n_out;
+    g.y = y;
     if (train) {
-        g.target = s->t;
+        g.x0t = s->ht[0];
+        g.target = target;
         g.tweight = s->tw;
-        g.n_valid = s->n_out;
         g.grad_scale = 2.0f / ((float)s->batch * (float)s->n_out);
         g.loss_part = s->loss_part;
     }
     g.err = s->err;
-    cudaLaunchConfig_t cfg;
-    std::memset(&cfg, 0, sizeof(cfg));
-    cfg.gridDim = dim3((s->batch / kBM) * umma::kChainCluster);
-    cfg.blockDim = dim3(umma::kChainThreads);
-    cfg.dynamicSmemBytes = umma::kChainSmem;
-    cfg.stream = s->stream;
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeClusterDimension;
-    at[0].val.clusterDim.x = umma::kChainCluster;
-    at[0].val.clusterDim.y = 1;
-    at[0].val.clusterDim.z = 1;
-    cfg.attrs = at;
-    cfg.numAttrs = 1;
-    BD_CUDA_TRY(cudaLaunchKernelEx(&cfg, umma::k_mlp_chain, maps, g));
+    umma::k_mlp_chain<<<div_up(g.M, umma::kChainRows), umma::kChainThreads, umma::kChainSmem, s->stream>>>(maps, g);
+    BD_LAUNCH_CHECK();
     return BD_OK;
 }
 
-// forward of the whole network on the batch in h[0]; with a target also the
-// loss gradient and every dZ_l (the fused kernel's input-gradient chain)
-int forward(bd_surrogate *s, bool with_target) { return chain_launch(s, with_target); }
-
-// gradients of every layer into the split partials and db; dW_l partials go
-// to part + offset(l)
 size_t part_offset(const bd_surrogate *s, int l) {
     size_t off = 0;
     for (int i = 0; i < l; i++) off += (size_t)(s->batch / s->ksplit) * s->Np[i] * s->Kp[i];
     return off;
 }
 
-// weight and bias gradients from the dZ_l^T and H_{l-1}^T the forward
-// launch wrote
-int backward(bd_surrogate *s) {
-    const int B = s->batch;
-    for (int l = s->L - 1; l >= 0; l--) {
-        // dW_l = dZ_l^T H_{l-1}
-        GemmArgs g = base_args(s);
+// weight gradients dW_l = dZ_l^T H_{l-1} of every layer, as split partials at
+// part + part_offset(l); `count` also counts the training step
+int weight_grads(bd_surrogate *s, bool count) {
+    GemmTable t;
+    std::memset(&t, 0, sizeof(t));
+    t.n_jobs = s->L;
+    t.count = count ? s->step : nullptr;
+    t.err = s->err;
+    for (int l = 0; l < s->L; l++) {
+        GemmJob &g = t.job[l];
+        g.a = s->tm_dzt[l];
+        g.b = s->tm_ht[l];
+        g.out_f32 = s->part + part_offset(s, l);
         g.M = s->Np[l];
         g.N = s->Kp[l];
-        g.K = B;
+        g.K = s->batch;
         g.k_split = s->ksplit;
-        g.out_f32 = s->part + part_offset(s, l);
-        int rc = launch_gemm(s->tm_dzt[l], s->tm_ht[l], g, s->stream);
-        if (rc) return rc;
+        g.bn = s->Kp[l];
     }
+    return launch_gemms(t, s->stream);
+}
+
+BiasGradArgs bias_args(const bd_surrogate *s) {
     BiasGradArgs a;
     std::memset(&a, 0, sizeof(a));
     a.L = s->L;
-    a.B = B;
+    a.B = s->batch;
     for (int l = 0; l < s->L; l++) {
         a.dzt[l] = s->dzt[l];
         a.db[l] = s->db[l];
         a.first[l + 1] = a.first[l] + s->Np[l];
     }
-    k_bias_grads<<<a.first[s->L], 256, 0, s->stream>>>(a);
-    BD_LAUNCH_CHECK();
-    return BD_OK;
+    return a;
 }
 
 int adam(bd_surrogate *s) {
@@ -422,6 +464,7 @@ int adam(bd_surrogate *s) {
     std::memset(&t, 0, sizeof(t));
     t.L = s->L;
     t.splits = s->batch / s->ksplit;
+    t.bias = bias_args(s);
     for (int l = 0; l < s->L; l++) {
         t.w[l] = s->w[l];
         t.wm[l] = s->wm[l];
@@ -432,31 +475,54 @@ int adam(bd_surrogate *s) {
         t.b[l] = s->b[l];
         t.bm[l] = s->bm[l];
         t.bv[l] = s->bv[l];
-        t.db[l] = s->db[l];
         t.N[l] = s->Np[l];
         t.K[l] = s->Kp[l];
         t.n_live[l] = s->Nl[l];
         t.k_live[l] = s->Kl[l];
-        t.first_w[l + 1] = t.first_w[l] + (long long)s->Np[l] * s->Kp[l];
-        t.first_b[l + 1] = t.first_b[l] + s->Np[l];
+        t.first_w[l + 1] = t.first_w[l] + s->Np[l] / kAdamN * (s->Kp[l] / kAdamK);
     }
-    const long long total = t.first_w[s->L] + t.first_b[s->L];
-    k_adam_all<<<(unsigned)div_up(total, 256), 256, 0, s->stream>>>(t, a);
-    k_count<<<1, 1, 0, s->stream>>>(s->step);
+    k_adam_all<<<t.first_w[s->L] + div_up(t.bias.first[s->L], kBiasRows), 256, 0, s->stream>>>(t, a);
     BD_LAUNCH_CHECK();
     return BD_OK;
 }
 
-int train_step_launches(bd_surrogate *s) {
-    k_gather<<<div_up(s->batch, kGatherRows), 256, 0, s->stream>>>(
-        s->data_x, s->data_y, s->n_data, s->n_in, s->n_out, s->Kp[0], s->Np[s->L - 1], s->batch, nullptr, s->step,
-        s->seed, s->x0, s->ht[0], s->t);
+// the flat host order of the parameters or (gradients) of the last backward pass
+int flatten(bd_surrogate *s, bool gradients, float *out) {
+    FlatTable t;
+    std::memset(&t, 0, sizeof(t));
+    t.L = s->L;
+    t.splits = gradients ? s->batch / s->ksplit : 1;
+    int off = 0;
+    for (int l = 0; l < s->L; l++) {
+        t.w[l] = gradients ? s->part + part_offset(s, l) : s->w[l];
+        t.b[l] = gradients ? s->db[l] : s->b[l];
+        t.N[l] = s->Np[l];
+        t.K[l] = s->Kp[l];
+        t.n_live[l] = s->Nl[l];
+        t.k_live[l] = s->Kl[l];
+        t.out[l] = off;
+        off += s->Nl[l] * (s->Kl[l] + 1);
+        t.first[l + 1] = t.first[l] + s->Np[l] * (s->Kp[l] + 1);
+    }
+    k_flatten<<<div_up(t.first[s->L], 256), 256, 0, s->stream>>>(t, s->flat);
     BD_LAUNCH_CHECK();
-    int rc = forward(s, true);
-    if (!rc) rc = backward(s);
-    if (!rc) rc = adam(s);
-    return rc;
+    BD_CUDA_TRY(cudaMemcpyAsync(out, s->flat, (size_t)off * 4, cudaMemcpyDeviceToHost, s->stream));
+    return BD_OK;
 }
+
+// device rows for predict and gradients; grows, freed with the object
+int io_rows(bd_surrogate *s, int rows) {
+    if (rows <= s->pred_rows) return BD_OK;
+    if (s->px) cudaFree(s->px);
+    if (s->py) cudaFree(s->py);
+    s->px = s->py = nullptr;
+    s->pred_rows = 0;
+    BD_CUDA_TRY(cudaMalloc(&s->px, (size_t)rows * s->n_in * 4));
+    BD_CUDA_TRY(cudaMalloc(&s->py, (size_t)rows * s->n_out * 4));
+    s->pred_rows = rows;
+    return BD_OK;
+}
+constexpr int kPredictRows = 32768;  // rows predict keeps on the device at a time
 
 }  // namespace
 
@@ -507,21 +573,24 @@ int bd_surrogate_create(int n_in, int n_out, int width, int depth, int batch, un
         A((void **)&p, s->Np[l] * 4); s->db.push_back(p);
         A((void **)&q, nk * 2); s->wb.push_back(q);
         A((void **)&q, nk * 2); s->wbt.push_back(q);
-        if (l == 0) A((void **)&s->x0, (size_t)batch * s->Kp[0] * 2);
         A((void **)&q, (size_t)batch * s->Kp[l] * 2); s->ht.push_back(q);
-        A((void **)&p, (size_t)batch * s->Np[l] * 4); s->z.push_back(p);
+        p = nullptr;
+        if (l >= umma::kChainTmemLayers && l < s->L - 1) A((void **)&p, (size_t)batch * s->Np[l] * 4);
+        s->dg.push_back(p);
         A((void **)&q, (size_t)batch * s->Np[l] * 2); s->dzt.push_back(q);
         part_total += (size_t)(batch / s->ksplit) * nk;
     }
-    A((void **)&s->y, (size_t)batch * 128 * 4);
-    A((void **)&s->t, (size_t)batch * 128 * 4);
     A((void **)&s->tw, 128 * 4);
     A((void **)&s->part, part_total * 4);
     // loss partials: one per CTA of the fused kernel
-    s->loss_cells = (batch / kBM) * umma::kChainCluster;
-    A((void **)&s->loss_part, (size_t)s->loss_cells * 4);
+    s->loss_cells = batch / umma::kChainRows;
+    A((void **)&s->loss_part, (size_t)(s->loss_cells + 1) * 4);
+    s->err = reinterpret_cast<unsigned *>(s->loss_part + s->loss_cells);
     A((void **)&s->step, sizeof(long long));
-    A((void **)&s->err, sizeof(unsigned));
+    size_t n_param = 0;
+    for (int l = 0; l < s->L; l++) n_param += (size_t)s->Nl[l] * (s->Kl[l] + 1);
+    A((void **)&s->flat, n_param * 4);
+    if (ok && cudaMallocHost(&s->host, (size_t)(s->loss_cells + 1) * 4) != cudaSuccess) ok = false;
     if (!ok) {
         free_surrogate(s);
         return BD_ERR_NOMEM;
@@ -549,14 +618,12 @@ int bd_surrogate_create(int n_in, int n_out, int width, int depth, int batch, un
     s->tm_dzt.resize(s->L);
     s->tm_w.resize(s->L);
     s->tm_wt.resize(s->L);
-    rc |= make_tmap(&s->tm_x, s->x0, batch, s->Kp[0], kBM);
     for (int l = 0; l < s->L && !rc; l++) {
-        // weight gradient: A = dZ_l^T, B = H_{l-1}^T; fused kernel: W_l and W_l^T,
-        // a quarter of the rows per CTA of a cluster
+        // weight gradient: A = dZ_l^T, B = H_{l-1}^T; fused kernel: W_l and W_l^T
         rc |= make_tmap(&s->tm_dzt[l], s->dzt[l], s->Np[l], batch, kBM);
-        rc |= make_tmap(&s->tm_ht[l], s->ht[l], s->Kp[l], batch, kBN);
-        rc |= make_tmap(&s->tm_w[l], s->wb[l], s->Np[l], s->Kp[l], s->Np[l] / umma::kChainCluster);
-        rc |= make_tmap(&s->tm_wt[l], s->wbt[l], s->Kp[l], s->Np[l], s->Kp[l] / umma::kChainCluster);
+        rc |= make_tmap(&s->tm_ht[l], s->ht[l], s->Kp[l], batch, s->Kp[l]);
+        rc |= make_tmap(&s->tm_w[l], s->wb[l], s->Np[l], s->Kp[l], kBM);
+        rc |= make_tmap(&s->tm_wt[l], s->wbt[l], s->Kp[l], s->Np[l], kBM);
     }
     if (rc || cudaStreamSynchronize(s->stream) != cudaSuccess) {
         free_surrogate(s);
@@ -590,16 +657,9 @@ int bd_surrogate_param_count(const bd_surrogate *s, long long *count) {
 // Parameters as a flat FP32 vector: for each layer W [N_l][K_l] then b [N_l].
 int bd_surrogate_get_params(bd_surrogate *s, float *out) {
     if (!s || !out) return BD_ERR_ARG;
-    size_t off = 0;
-    for (int l = 0; l < s->L; l++) {
-        std::vector<float> hw((size_t)s->Np[l] * s->Kp[l]), hb(s->Np[l]);
-        BD_CUDA_TRY(cudaMemcpyAsync(hw.data(), s->w[l], hw.size() * 4, cudaMemcpyDeviceToHost, s->stream));
-        BD_CUDA_TRY(cudaMemcpyAsync(hb.data(), s->b[l], hb.size() * 4, cudaMemcpyDeviceToHost, s->stream));
-        BD_CUDA_TRY(cudaStreamSynchronize(s->stream));
-        for (int n = 0; n < s->Nl[l]; n++)
-            for (int k = 0; k < s->Kl[l]; k++) out[off++] = hw[(size_t)k * s->Np[l] + n];  // master kept [K][N]
-        for (int n = 0; n < s->Nl[l]; n++) out[off++] = hb[n];
-    }
+    const int rc = flatten(s, false, out);
+    if (rc) return rc;
+    BD_CUDA_TRY(cudaStreamSynchronize(s->stream));
     return BD_OK;
 }
 
@@ -634,7 +694,6 @@ int bd_surrogate_set_output_weights(bd_surrogate *s, const float *w) {
 // Training set on the device: x [n][n_in], y [n][n_out] (host, FP32).
 int bd_surrogate_set_data(bd_surrogate *s, const float *x, const float *y, int n) {
     if (!s || !x || !y || n < 1) return BD_ERR_ARG;
-    if (s->graph) { cudaGraphExecDestroy(s->graph); s->graph = nullptr; }
     if (s->data_x) cudaFree(s->data_x);
     if (s->data_y) cudaFree(s->data_y);
     s->data_x = s->data_y = nullptr;
@@ -648,32 +707,21 @@ int bd_surrogate_set_data(bd_surrogate *s, const float *x, const float *y, int n
 }
 
 // `steps` Adam steps on random minibatches (with replacement) of the
-// training set, captured once as a CUDA graph; mean loss of the last step.
+// training set, three launches each; mean loss of the last step.
 int bd_surrogate_train(bd_surrogate *s, int steps, float lr, float *last_loss) {
     if (!s || steps < 0 || !(lr > 0.f)) return BD_ERR_ARG;
     if (!s->data_x) return BD_ERR_STATE;
-    if (lr != s->lr && s->graph) { cudaGraphExecDestroy(s->graph); s->graph = nullptr; }
     s->lr = lr;
-    if (!s->graph && steps > 0) {
-        cudaGraph_t g;
-        BD_CUDA_TRY(cudaStreamBeginCapture(s->stream, cudaStreamCaptureModeThreadLocal));
-        int rc = train_step_launches(s);
-        cudaError_t ce = cudaStreamEndCapture(s->stream, &g);
+    for (int i = 0; i < steps; i++) {
+        int rc = chain_launch(s, true, true, s->data_x, s->data_y, s->n_data, nullptr);
+        if (!rc) rc = weight_grads(s, true);
+        if (!rc) rc = adam(s);
         if (rc) return rc;
-        BD_CUDA_TRY(ce);
-        BD_CUDA_TRY(cudaGraphInstantiate(&s->graph, g, 0));
-        cudaGraphDestroy(g);
     }
-    for (int i = 0; i < steps; i++) BD_CUDA_TRY(cudaGraphLaunch(s->graph, s->stream));
-    if (last_loss) {
-        std::vector<float> lp(s->loss_cells);
-        BD_CUDA_TRY(cudaMemcpyAsync(lp.data(), s->loss_part, lp.size() * 4, cudaMemcpyDeviceToHost, s->stream));
-        BD_CUDA_TRY(cudaStreamSynchronize(s->stream));
-        double sum = 0;
-        for (float v : lp) sum += v;
-        *last_loss = (float)(sum / ((double)s->batch * s->n_out));
-    }
-    return sg_status(s);
+    double sum = 0;
+    const int rc = sg_finish(s, &sum);
+    if (last_loss) *last_loss = (float)(sum / ((double)s->batch * s->n_out));
+    return rc;
 }
 
 // Gradients of the mean loss over one batch (x [batch][n_in], y
@@ -682,84 +730,39 @@ int bd_surrogate_train(bd_surrogate *s, int steps, float lr, float *last_loss) {
 int bd_surrogate_gradients(bd_surrogate *s, const float *x, const float *y, float *grad, float *loss) {
     if (!s || !x || !y || !grad) return BD_ERR_ARG;
     const int B = s->batch;
-    float *dx = nullptr, *dy = nullptr;
-    BD_CUDA_TRY(cudaMalloc(&dx, (size_t)B * s->n_in * 4));
-    BD_CUDA_TRY(cudaMalloc(&dy, (size_t)B * s->n_out * 4));
-    cudaMemcpyAsync(dx, x, (size_t)B * s->n_in * 4, cudaMemcpyHostToDevice, s->stream);
-    cudaMemcpyAsync(dy, y, (size_t)B * s->n_out * 4, cudaMemcpyHostToDevice, s->stream);
-    std::vector<int> rows(B);
-    for (int i = 0; i < B; i++) rows[i] = i;
-    int *drows = nullptr;
-    BD_CUDA_TRY(cudaMalloc(&drows, B * 4));
-    cudaMemcpyAsync(drows, rows.data(), B * 4, cudaMemcpyHostToDevice, s->stream);
-    k_gather<<<div_up(B, kGatherRows), 256, 0, s->stream>>>(dx, dy, B, s->n_in, s->n_out, s->Kp[0],
-                                                             s->Np[s->L - 1], B, drows, s->step, s->seed, s->x0,
-                                                             s->ht[0], s->t);
-    int rc = forward(s, true);
-    if (!rc) rc = backward(s);
-    const int splits = B / s->ksplit;
-    size_t off = 0;
-    std::vector<float> lp(s->loss_cells);
-    if (!rc) {
-        for (int l = 0; l < s->L && !rc; l++) {
-            const size_t n = (size_t)s->Np[l] * s->Kp[l];
-            float *gsum = nullptr;
-            if (cudaMalloc(&gsum, n * 4) != cudaSuccess) { rc = BD_ERR_NOMEM; break; }
-            k_sum_splits<<<div_up((long)n, 256), 256, 0, s->stream>>>(s->part + part_offset(s, l), splits, n, gsum);
-            std::vector<float> hg(n), hb(s->Np[l]);
-            cudaMemcpyAsync(hg.data(), gsum, n * 4, cudaMemcpyDeviceToHost, s->stream);
-            cudaMemcpyAsync(hb.data(), s->db[l], s->Np[l] * 4, cudaMemcpyDeviceToHost, s->stream);
-            cudaStreamSynchronize(s->stream);
-            cudaFree(gsum);
-            for (int nn = 0; nn < s->Nl[l]; nn++)  // partial sums are [K][N]
-                for (int k = 0; k < s->Kl[l]; k++) grad[off++] = hg[(size_t)k * s->Np[l] + nn];
-            for (int nn = 0; nn < s->Nl[l]; nn++) grad[off++] = hb[nn];
-        }
-        cudaMemcpyAsync(lp.data(), s->loss_part, lp.size() * 4, cudaMemcpyDeviceToHost, s->stream);
-    }
-    cudaStreamSynchronize(s->stream);
-    cudaFree(dx);
-    cudaFree(dy);
-    cudaFree(drows);
+    int rc = io_rows(s, B);
     if (rc) return rc;
-    if (loss) {
-        double sum = 0;
-        for (float v : lp) sum += v;
-        *loss = (float)(sum / ((double)B * s->n_out));
-    }
-    return sg_status(s);
+    BD_CUDA_TRY(cudaMemcpyAsync(s->px, x, (size_t)B * s->n_in * 4, cudaMemcpyHostToDevice, s->stream));
+    BD_CUDA_TRY(cudaMemcpyAsync(s->py, y, (size_t)B * s->n_out * 4, cudaMemcpyHostToDevice, s->stream));
+    rc = chain_launch(s, true, false, s->px, s->py, B, nullptr);
+    if (!rc) rc = weight_grads(s, false);
+    if (rc) return rc;
+    const BiasGradArgs a = bias_args(s);
+    k_bias_grads<<<div_up(a.first[s->L], kBiasRows), kBiasRows * 32, 0, s->stream>>>(a);
+    BD_LAUNCH_CHECK();
+    rc = flatten(s, true, grad);
+    if (rc) return rc;
+    double sum = 0;
+    rc = sg_finish(s, &sum);
+    if (loss) *loss = (float)(sum / ((double)B * s->n_out));
+    return rc;
 }
 
 // Network outputs for n inputs (host x [n][n_in] -> y [n][n_out]).
 int bd_surrogate_predict(bd_surrogate *s, const float *x, int n, float *y) {
     if (!s || !x || !y || n < 0) return BD_ERR_ARG;
-    const int B = s->batch;
-    float *dx = nullptr;
-    int *drows = nullptr;
-    BD_CUDA_TRY(cudaMalloc(&dx, (size_t)std::max(n, 1) * s->n_in * 4));
-    BD_CUDA_TRY(cudaMalloc(&drows, B * 4));
-    BD_CUDA_TRY(cudaMemcpyAsync(dx, x, (size_t)n * s->n_in * 4, cudaMemcpyHostToDevice, s->stream));
-    std::vector<int> rows(B);
-    std::vector<float> hy((size_t)B * 128);
-    int rc = BD_OK;
-    for (int r0 = 0; r0 < n && !rc; r0 += B) {
-        const int cnt = std::min(B, n - r0);
-        for (int i = 0; i < B; i++) rows[i] = i < cnt ? r0 + i : -1;
-        cudaMemcpyAsync(drows, rows.data(), B * 4, cudaMemcpyHostToDevice, s->stream);
-        k_gather<<<div_up(B, kGatherRows), 256, 0, s->stream>>>(dx, nullptr, n, s->n_in, s->n_out, s->Kp[0],
-                                                                 s->Np[s->L - 1], B, drows, s->step, s->seed,
-                                                                 s->x0, s->ht[0], nullptr);
-        rc = forward(s, false);
-        if (rc) break;
-        cudaMemcpyAsync(hy.data(), s->y, hy.size() * 4, cudaMemcpyDeviceToHost, s->stream);
-        if (cudaStreamSynchronize(s->stream) != cudaSuccess) rc = BD_ERR_CUDA;
-        for (int i = 0; i < cnt; i++)  // outputs are [128][B]
-            for (int k = 0; k < s->n_out; k++) y[(size_t)(r0 + i) * s->n_out + k] = hy[(size_t)k * B + i];
+    int rc = io_rows(s, std::min(n, kPredictRows));
+    for (int r0 = 0; r0 < n && !rc; r0 += kPredictRows) {
+        const int cnt = std::min(kPredictRows, n - r0);
+        BD_CUDA_TRY(cudaMemcpyAsync(s->px, x + (size_t)r0 * s->n_in, (size_t)cnt * s->n_in * 4, cudaMemcpyHostToDevice,
+                                    s->stream));
+        rc = chain_launch(s, false, false, s->px, nullptr, cnt, s->py);
+        if (!rc)
+            BD_CUDA_TRY(cudaMemcpyAsync(y + (size_t)r0 * s->n_out, s->py, (size_t)cnt * s->n_out * 4,
+                                        cudaMemcpyDeviceToHost, s->stream));
     }
-    cudaFree(dx);
-    cudaFree(drows);
     if (rc) return rc;
-    return sg_status(s);
+    return sg_finish(s, nullptr);
 }
 
 // Plain GEMM through the same kernel, for tests and measurement:
@@ -787,15 +790,20 @@ int bd_umma_gemm_bf16(const unsigned short *a, const unsigned short *b, int M, i
         if (!rc) rc = make_tmap(&tb, db, N, K, kBN);
     }
     if (!rc) {
-        GemmArgs g;
-        std::memset(&g, 0, sizeof(g));
+        GemmTable t;
+        std::memset(&t, 0, sizeof(t));
+        t.n_jobs = 1;
+        t.err = err;
+        GemmJob &g = t.job[0];
+        g.a = ta;
+        g.b = tb;
         g.M = M;
         g.N = N;
         g.K = K;
         g.k_split = ks;
         g.out_f32 = part;
-        g.err = err;
-        rc = launch_gemm(ta, tb, g, st);
+        g.bn = kBN;
+        rc = launch_gemms(t, st);
     }
     if (!rc) {
         k_sum_splits<<<div_up((long)M * N, 256), 256, 0, st>>>(part, splits, (size_t)M * N, dc);

@@ -513,7 +513,7 @@ class Surrogate:
             [(self.n_out, self.width)]
 
     def get_params(self) -> np.ndarray:
-        out = np.zeros(self.n_params, np.float32)
+        out = np.empty(self.n_params, np.float32)
         _check(_lib().bd_surrogate_get_params(self._h, _ptr(out)), "get_params")
         return out
 
@@ -539,14 +539,14 @@ class Surrogate:
     def gradients(self, x: np.ndarray, y: np.ndarray):
         x = np.ascontiguousarray(x, np.float32).reshape(self.batch, self.n_in)
         y = np.ascontiguousarray(y, np.float32).reshape(self.batch, self.n_out)
-        g = np.zeros(self.n_params, np.float32)
+        g = np.empty(self.n_params, np.float32)
         loss = C.c_float(0)
         _check(_lib().bd_surrogate_gradients(self._h, _ptr(x), _ptr(y), _ptr(g), C.byref(loss)), "gradients")
         return g, loss.value
 
     def predict(self, x: np.ndarray) -> np.ndarray:
         x = np.ascontiguousarray(x, np.float32).reshape(-1, self.n_in)
-        y = np.zeros((len(x), self.n_out), np.float32)
+        y = np.empty((len(x), self.n_out), np.float32)
         _check(_lib().bd_surrogate_predict(self._h, _ptr(x), len(x), _ptr(y)), "predict")
         return y
 

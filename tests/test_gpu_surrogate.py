@@ -102,3 +102,52 @@ def test_held_out_fs_error_below_0_02():
     model.close()
     assert n > 1000
     assert mean_err < 0.02, (mean_err, max_err)
+
+
+@pytest.mark.parametrize("width,depth,batch,n_in,n_out", [
+    (256, 8, 256, 5, 34),     # the eighth hidden layer keeps gelu' in global memory
+    (256, 7, 512, 64, 128),   # every column of tensor memory; no padding in the inputs and outputs
+    (192, 5, 768, 3, 1),      # a second tile of 64 features
+    (128, 1, 256, 1, 17),     # one tile, one hidden layer
+    (64, 8, 1024, 8, 64),     # half a tile
+])
+def test_network_shapes_match_oracle(width, depth, batch, n_in, n_out):
+    s, layers, x, t = _net(width, depth, batch, seed=width + depth, n_in=n_in, n_out=n_out)
+    x, t = x.astype(np.float32), t.astype(np.float32)
+    g, loss = s.gradients(x, t)
+    lo, grads, _ = M.loss_and_grad(layers, x, t, bf16=True)
+    go = M.flatten(grads)
+    assert abs(loss - lo) <= 1e-3 * lo
+    assert np.max(np.abs(g - go)) <= 2e-2 * np.max(np.abs(go))
+    # a row's outputs do not depend on how many rows a call has, edges of the
+    # 32-row blocks and of the 32768 rows a pass takes among them
+    y = s.predict(x)
+    yo = M.predict(layers, x, bf16=True)
+    assert np.max(np.abs(y - yo)) <= 2e-2 * np.max(np.abs(yo))
+    for n in (1, 31, 33, batch - 1):
+        assert np.array_equal(s.predict(x[:n]), y[:n])
+    many = np.tile(x, (33000 // batch + 1, 1))[:33000]
+    assert np.array_equal(s.predict(many), np.tile(y, (33000 // batch + 1, 1))[:33000])
+    # one Adam step on the rows the counter hash draws: each parameter moves by
+    # lr g / (|g| + eps)
+    data_x, data_y = np.tile(x, (3, 1)), np.tile(t, (3, 1)) * np.float32(0.5)
+    s.set_data(data_x, data_y)
+    before = s.get_params().astype(np.float64)
+    loss1 = s.train(1, 1e-3)
+    mask = (1 << 64) - 1
+
+    def mix(v):
+        v = (v + 0x9E3779B97F4A7C15) & mask
+        v = ((v ^ (v >> 30)) * 0xBF58476D1CE4E5B9) & mask
+        v = ((v ^ (v >> 27)) * 0x94D049BB133111EB) & mask
+        return v ^ (v >> 31)
+
+    rows = np.array([mix((width + depth) ^ mix(r)) % len(data_x) for r in range(batch)])
+    lo1, grads, _ = M.loss_and_grad(layers, data_x[rows], data_y[rows], bf16=True)
+    go = M.flatten(grads)
+    assert abs(loss1 - lo1) <= 1e-3 * lo1
+    big = np.abs(go) > 4e-2 * np.max(np.abs(go))
+    moved = s.get_params().astype(np.float64) - before
+    # |g| >> eps there; the FP32 parameters (below 8 in size) round the sum
+    assert np.all(np.abs(moved + 1e-3 * np.sign(go))[big] <= 1e-3 * 1e-3 + 2.0 ** -21)
+    s.close()
