@@ -14,8 +14,18 @@
 // Reduction layout: a replica's storage ids are contiguous, so the batch is
 // cut into segments of kCorrChunk ids that never straddle two replicas.
 // k_corr_partial writes one partial sum per (segment, slot, field);
-// k_corr_finish adds a replica's segments in index order.  No atomics: the
+// k_corr_finish adds a replica's segments in a fixed order.  No atomics: the
 // result is bit-reproducible.
+//
+// What bounds it: the snapshots (24 B a particle and slot, 201 MB at 16 slots
+// of 524288 particles: 31 us at the copy rate) and the FP64 instructions.  So
+// a thread loads the next slot's values under the arithmetic of this one's
+// (waiting for them was two thirds of the time); the slots are cut into groups
+// of 8, a block each, which leaves no nearly empty last wave and re-reads the
+// current displacement once a group; and a warp's six sums are reduced
+// together: at each level the lanes exchange half of the fields they still
+// hold, 8 exchanges instead of 30.  At that size 68 us (101 before, with four
+// particles a thread, all slots in one block and no prefetch).
 #include <climits>
 #include <vector>
 
@@ -24,10 +34,33 @@
 namespace bd {
 
 constexpr int kCorrThreads = 256;
-constexpr int kCorrPerThread = 4;
+constexpr int kCorrPerThread = 2;
 constexpr int kCorrChunk = kCorrThreads * kCorrPerThread;
 constexpr int kCorrFields = 6;  // msd, r4, fs of big; msd, r4, fs of small
 constexpr int kMaxCorrSlots = 64;
+constexpr int kCorrGroup = 8;  // slots of one block
+
+// Warp sums of six values at once.  Level 1 splits the fields 0-2 | 3-5 over
+// the lane halves, level 2 the fields 0, 1 | 2 over the quarters, level 3 the
+// fields 0 | 1; the lanes `corr_field(lane)` >= 0 end with that field's sum.
+__device__ __forceinline__ double corr_warp_sums(const double *v, int lane) {
+    const bool h16 = lane & 16, h8 = lane & 8, h4 = lane & 4;
+    double w[3];
+#pragma unroll
+    for (int k = 0; k < 3; k++)
+        w[k] = (h16 ? v[k + 3] : v[k]) + __shfl_xor_sync(0xffffffffu, h16 ? v[k] : v[k + 3], 16);
+    const double u0 = (h8 ? w[2] : w[0]) + __shfl_xor_sync(0xffffffffu, h8 ? w[0] : w[2], 8);
+    const double u1 = w[1] + __shfl_xor_sync(0xffffffffu, w[1], 8);
+    // the quarter that holds field 2 keeps it in all of its lanes
+    double t = (h4 && !h8 ? u1 : u0) + __shfl_xor_sync(0xffffffffu, h4 || h8 ? u0 : u1, 4);
+    t += __shfl_xor_sync(0xffffffffu, t, 2);
+    t += __shfl_xor_sync(0xffffffffu, t, 1);
+    return t;
+}
+__device__ __forceinline__ int corr_field(int lane) {
+    if ((lane & 3) || (lane & 12) == 12) return -1;
+    return ((lane & 16) ? 3 : 0) + ((lane & 8) ? 2 : ((lane & 4) ? 1 : 0));
+}
 
 struct SlotList {
     int n;
@@ -44,7 +77,8 @@ __global__ void __launch_bounds__(kCorrThreads) k_corr_partial(const int2 *__res
                                                                SlotList sl, double q, double *__restrict__ part) {
     // per-warp partial sums of every slot; one barrier, then a fixed-order
     // reduction over the warps
-    __shared__ double red[kMaxCorrSlots][kCorrThreads / 32][kCorrFields];
+    __shared__ double red[kCorrGroup][kCorrThreads / 32][kCorrFields];
+    const int j0 = blockIdx.y * kCorrGroup, nj = min(kCorrGroup, sl.n - j0);
     const int2 sg = segs[blockIdx.x];  // (replica, first storage id)
     const SysDev &S = sys[sg.x];
     const int end = min(sg.y + kCorrChunk, S.part_base + S.n);
@@ -65,53 +99,75 @@ __global__ void __launch_bounds__(kCorrThreads) k_corr_partial(const int2 *__res
             sid[i] = -1;
         }
     }
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-#pragma unroll 2
-    for (int j = 0; j < sl.n; j++) {
-        const double *bx = snaps + (size_t)sl.slot[j] * 3 * (size_t)P;
-        const double *by = bx + P, *bz = by + P;
-        double acc[kCorrFields];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, field = corr_field(lane);
+    // the next slot's displacements load under the arithmetic of this one's
+    double b[kCorrPerThread][3];
+    auto load = [&](int j) {
+        const double *bx = snaps + (size_t)sl.slot[j0 + j] * 3 * (size_t)P;
+#pragma unroll
+        for (int i = 0; i < kCorrPerThread; i++)
+#pragma unroll
+            for (int k = 0; k < 3; k++) b[i][k] = sid[i] >= 0 ? bx[k * P + sid[i]] : 0.0;
+    };
+    load(0);
+#pragma unroll 1
+    for (int j = 0; j < nj; j++) {
+        double e[kCorrPerThread][3], acc[kCorrFields];
+#pragma unroll
+        for (int i = 0; i < kCorrPerThread; i++) {
+            e[i][0] = px[i] - b[i][0];
+            e[i][1] = py[i] - b[i][1];
+            e[i][2] = pz[i] - b[i][2];
+        }
+        if (j + 1 < nj) load(j + 1);
 #pragma unroll
         for (int f = 0; f < kCorrFields; f++) acc[f] = 0.0;
 #pragma unroll
         for (int i = 0; i < kCorrPerThread; i++) {
             if (sid[i] < 0) continue;
-            const double ex = px[i] - bx[sid[i]], ey = py[i] - by[sid[i]], ez = pz[i] - bz[sid[i]];
+            const double ex = e[i][0], ey = e[i][1], ez = e[i][2];
             const double r2 = ex * ex + ey * ey + ez * ez;
             const double qr = q * sqrt(r2);
             const double fs = qr > 0.0 ? sin(qr) / qr : 1.0;
-            const int o = big[i] ? 0 : 3;
-            acc[o] += r2;
-            acc[o + 1] += r2 * r2;
-            acc[o + 2] += fs;
+            if (big[i]) {
+                acc[0] += r2;
+                acc[1] += r2 * r2;
+                acc[2] += fs;
+            } else {
+                acc[3] += r2;
+                acc[4] += r2 * r2;
+                acc[5] += fs;
+            }
         }
-#pragma unroll
-        for (int f = 0; f < kCorrFields; f++) {
-            double v = acc[f];
-#pragma unroll
-            for (int off = 16; off > 0; off >>= 1) v += __shfl_down_sync(0xffffffffu, v, off);
-            if (lane == 0) red[j][warp][f] = v;
-        }
+        const double sum = corr_warp_sums(acc, lane);
+        if (field >= 0) red[j][warp][field] = sum;
     }
     __syncthreads();
-    for (int t = threadIdx.x; t < sl.n * kCorrFields; t += kCorrThreads) {
+    for (int t = threadIdx.x; t < nj * kCorrFields; t += kCorrThreads) {
         const int j = t / kCorrFields, f = t % kCorrFields;
         double v = 0.0;
 #pragma unroll
         for (int w = 0; w < kCorrThreads / 32; w++) v += red[j][w][f];
-        part[((size_t)blockIdx.x * sl.n + j) * kCorrFields + f] = v;
+        part[((size_t)blockIdx.x * sl.n + j0 + j) * kCorrFields + f] = v;
     }
 }
 
-// out[(j * R + r) * kCorrFields + f] = sum over the segments of replica r
-__global__ void k_corr_finish(const int *__restrict__ seg_first, const double *__restrict__ part, int nslot, int R,
-                              double *__restrict__ out) {
-    const int r = blockIdx.x, t = threadIdx.x;
+// out[(j * R + r) * kCorrFields + f] = sum over the segments of replica r:
+// a warp per (replica, slot, field), its lanes' strided sums added in a tree
+// (in a fixed order; one thread adding 64 segments in turn took 20 us)
+constexpr int kCorrFinishThreads = 256;
+__global__ void __launch_bounds__(kCorrFinishThreads) k_corr_finish(const int *__restrict__ seg_first,
+                                                                    const double *__restrict__ part, int nslot, int R,
+                                                                    double *__restrict__ out) {
+    const int t = blockIdx.y * (kCorrFinishThreads / 32) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+    const int r = blockIdx.x;
     if (t >= nslot * kCorrFields) return;
-    const int j = t / kCorrFields, f = t % kCorrFields;
     double v = 0.0;
-    for (int s = seg_first[r]; s < seg_first[r + 1]; s++) v += part[((size_t)s * nslot + j) * kCorrFields + f];
-    out[((size_t)j * R + r) * kCorrFields + f] = v;
+    for (int s = seg_first[r] + lane; s < seg_first[r + 1]; s += 32) v += part[(size_t)s * nslot * kCorrFields + t];
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) v += __shfl_down_sync(0xffffffffu, v, off);
+    const int j = t / kCorrFields, f = t % kCorrFields;
+    if (lane == 0) out[((size_t)j * R + r) * kCorrFields + f] = v;
 }
 
 // out[3 * gid + k] = displacement component k of the particle with global index gid
@@ -220,11 +276,11 @@ int bd_engine_correlate(bd_engine *e, const int *slots, int nslots, double q, bd
     if ((rc = ensure_scratch(e->corr_part, e->corr_part_cap, (size_t)e->nsegs * nslots * kCorrFields))) return rc;
     if ((rc = ensure_scratch(e->corr_out, e->corr_out_cap, (size_t)e->R * nslots * kCorrFields))) return rc;
     if ((rc = sync_dsp(e))) return rc;
-    k_corr_partial<<<e->nsegs, kCorrThreads, 0, e->stream>>>(e->d_segs, e->d_sys, e->gid_of, e->dsp[0], e->dsp[1],
-                                                             e->dsp[2], e->snaps, e->P, sl, q, e->corr_part);
+    k_corr_partial<<<dim3(e->nsegs, div_up(nslots, kCorrGroup)), kCorrThreads, 0, e->stream>>>(
+        e->d_segs, e->d_sys, e->gid_of, e->dsp[0], e->dsp[1], e->dsp[2], e->snaps, e->P, sl, q, e->corr_part);
     BD_LAUNCH_CHECK();
-    const int nt = (nslots * kCorrFields + 31) / 32 * 32;
-    k_corr_finish<<<e->R, nt, 0, e->stream>>>(e->d_seg_first, e->corr_part, nslots, e->R, e->corr_out);
+    k_corr_finish<<<dim3(e->R, div_up(nslots * kCorrFields, kCorrFinishThreads / 32)), kCorrFinishThreads, 0,
+                    e->stream>>>(e->d_seg_first, e->corr_part, nslots, e->R, e->corr_out);
     BD_LAUNCH_CHECK();
     std::vector<double> h((size_t)e->R * nslots * kCorrFields);
     BD_CUDA_TRY(cudaMemcpyAsync(h.data(), e->corr_out, sizeof(double) * h.size(), cudaMemcpyDeviceToHost, e->stream));

@@ -205,3 +205,38 @@ def test_aging_command_line_writes_every_decade(tmp_path):
         assert (d / f"gder_{len(idx) - 1}.out").exists()
         fs = np.loadtxt(d / "fself.out")
         assert np.all(fs[:, 1] <= 1.0) and np.all(fs[:, 1] > -0.5)
+
+
+@pytest.mark.parametrize("nslots", [1, 7, 8, 9, 17, 64])
+def test_slot_groups_match_numpy_fp64(nslots):
+    # groups of 8 slots, segments of 512 particles: sizes on both sides of an edge
+    systems = []
+    for k, n in enumerate((511, 512, 513, 1100)):
+        nb = n // 3 if k else 0
+        side = float(np.float32(CF.side_from_phi(nb, n - nb, 0.4)))
+        systems.append(B.System(n_big=nb, n_sml=n - nb, side=side, sigma_big=SB, sigma_sml=SS, dt=1e-4, seed=900 + k,
+                                T0=1.0, Tf=1.0, t0=0.0, tf=0.005, protocol="linear", force_cap=200.0))
+    pos = np.concatenate([CF.lattice_config(s.n_big, s.n_sml, s.side, 40 + k) for k, s in enumerate(systems)])
+    e = B.Engine(systems, ni_start=0)
+    e.set_positions(pos)
+    e.reserve_snapshots(nslots)
+    then = []
+    e.run(3)
+    for j in range(nslots):
+        e.snapshot(j)
+        then.append(e.get_displacements())
+        e.run(1)
+    now = e.get_displacements()
+    slots = list(range(nslots))[::-1]
+    c = e.correlate(slots, Q)
+    for row, j in zip(c, slots):
+        exp = expected(systems, now, then[j])
+        for r, s in enumerate(systems):
+            if not s.n_big:  # an absent species reads zero
+                for k in ("msd_big", "r4_big", "fself_big"):
+                    assert row[r][k] == 0.0
+                    del exp[r][k]
+        check(row, exp)
+    # a slot's bits do not depend on the group it falls into
+    for k in (0, nslots - 1):
+        np.testing.assert_array_equal(e.correlate([slots[k]], Q)[0], c[k])
