@@ -938,22 +938,32 @@ int bd_engine_set_positions(bd_engine *e, const float *pos) {
     BD_CUDA_TRY(cudaMemcpyAsync(&bad, e->ld_bad, sizeof(unsigned), cudaMemcpyDeviceToHost, e->stream));
     BD_CUDA_TRY(cudaStreamSynchronize(e->stream));
     if (bad) return BD_ERR_ARG;  // nothing of the engine state has changed
-    int *start = e->ld_start;  // the scan runs on a copy of the counts
-    cudaMemcpyAsync(start, e->ld_cnt, sizeof(int) * T, cudaMemcpyDeviceToDevice, e->stream);
-    k_scan_local<<<nb, kScanThreads, 0, e->stream>>>(start, n, e->ld_bsum);
-    k_scan_totals<<<1, kScanThreads, 0, e->stream>>>(e->ld_bsum, nb);
-    k_scan_add<<<div_up(T, 256), 256, 0, e->stream>>>(start, n, e->ld_bsum);
+    int *start = e->ld_start;
+    if (nb <= kScanWhole) {
+        k_scan_local<true><<<nb, kScanThreads, 0, e->stream>>>(e->ld_cnt, start, n, nullptr);
+    } else {
+        k_scan_local<false><<<nb, kScanThreads, 0, e->stream>>>(e->ld_cnt, start, n, e->ld_bsum);
+        k_scan_totals<<<1, kScanThreads, 0, e->stream>>>(e->ld_bsum, nb);
+        k_scan_add<<<div_up(T, 256), 256, 0, e->stream>>>(start, n, e->ld_bsum);
+    }
     k_order_fill<<<gp, 256, 0, e->stream>>>(e->ld_slot, (int)P, start, e->ld_cnt, e->ld_bucket);
     k_order_emit<<<gt, 256, 0, e->stream>>>(start, n, (int)P, e->cap, e->ld_bucket, e->ld_in, e->rep_of_gid,
                                             e->d_sys, e->ld_staged, e->gid_of, e->rep_of_sid);
     BD_LAUNCH_CHECK();
+    LoadReset lr;
     for (int k = 0; k < 3; k++) {
-        cudaMemsetAsync(e->cnt[k], 0, sizeof(int) * e->C, e->stream);
-        cudaMemsetAsync(e->lo[k], 0, sizeof(float) * P, e->stream);
-        cudaMemsetAsync(e->dsp[k], 0, sizeof(double) * P, e->stream);
+        lr.cnt[k] = e->cnt[k];
+        lr.lo[k] = e->lo[k];
+        lr.dsp[k] = e->dsp[k];
     }
-    if (e->img) cudaMemsetAsync(e->img, 0, sizeof(int) * 3 * P, e->stream);
-    cudaMemsetAsync(e->status, 0, 256, e->stream);
+    lr.img = e->img;
+    lr.status = e->status;
+    lr.n_status = 256 / (int)sizeof(unsigned);
+    lr.flag = e->list ? e->lflag : nullptr;
+    lr.n_flag = e->R + 1;
+    lr.C = e->C;
+    lr.np = (long long)P;
+    k_load_reset<<<rebuild_grid(e, div_up(std::max((long long)P, (long long)e->C), 256)), 256, 0, e->stream>>>(lr);
     e->cur = 0;
     e->generation++;  // displacement snapshots of earlier positions are void
     if (e->rng == BD_RNG_RANNEW64) {  // streams keyed by particle, stored by storage id
@@ -964,17 +974,13 @@ int bd_engine_set_positions(bd_engine *e, const float *pos) {
     k_load<<<div_up((long)P, 256), 256, 0, e->stream>>>(e->ld_staged, (int)P, e->rep_of_sid, e->d_sys, e->cnt[0],
                                                         e->pos[0], e->cap, e->x0, e->gid_of, e->status,
                                                         e->list ? e->lpos[0] : nullptr);
-    if (e->list) {  // every replica's lists are built before its first step
-        std::vector<int> ones(e->R + 1, 1);
-        cudaMemcpyAsync(e->lflag, ones.data(), sizeof(int) * (e->R + 1), cudaMemcpyHostToDevice, e->stream);
-    }
     if (e->rng == BD_RNG_RANNEW64)
         k_rannew64_seed<<<div_up((long)P, 128), 128, 0, e->stream>>>(e->rn_ring, e->rn_lcg, e->d_sys, e->rep_of_sid,
                                                                      e->gid_of, (int)P);
-    cudaError_t le = cudaGetLastError();
-    cudaStreamSynchronize(e->stream);
-    if (le != cudaSuccess) return BD_ERR_CUDA;
-
+    if (cudaGetLastError() != cudaSuccess) {
+        cudaStreamSynchronize(e->stream);
+        return BD_ERR_CUDA;
+    }
     e->loaded = true;
     return engine_status(e);
 }

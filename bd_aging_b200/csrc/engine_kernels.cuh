@@ -147,15 +147,33 @@ __global__ void k_order_keys(const float *__restrict__ pos3, int P, const int *_
     }
 }
 
-// exclusive scan, pass 1: each block scans kScanBlock entries in place and
-// writes its total
-__global__ void __launch_bounds__(kScanThreads) k_scan_local(int *__restrict__ v, int n, int *__restrict__ bsum) {
+// exclusive scan of src into v, pass 1: each block scans kScanBlock entries and
+// writes its total.  WHOLE: each block also sums all entries before its own,
+// and no further pass is needed: one launch instead of three where re-reading
+// them costs less than a launch (up to kScanWhole blocks, 64 entries a thread).
+constexpr int kScanWhole = 16;
+template <bool WHOLE>
+__global__ void __launch_bounds__(kScanThreads) k_scan_local(const int *__restrict__ src, int *__restrict__ v, int n,
+                                                             int *__restrict__ bsum) {
     __shared__ int wsum[kScanThreads / 32];
+    __shared__ int s_before;
+    int before = 0;
+    if (WHOLE) {
+        if (threadIdx.x == 0) s_before = 0;
+        __syncthreads();
+#pragma unroll 8
+        for (int i = threadIdx.x; i < (int)blockIdx.x * kScanBlock; i += kScanThreads) before += src[i];
+#pragma unroll
+        for (int off = 16; off > 0; off >>= 1) before += __shfl_down_sync(0xffffffffu, before, off);
+        if ((threadIdx.x & 31) == 0) atomicAdd(&s_before, before);
+        __syncthreads();
+        before = s_before;
+    }
     const int base = blockIdx.x * kScanBlock + threadIdx.x * kScanPer;
     int x[kScanPer], t = 0;
 #pragma unroll
     for (int i = 0; i < kScanPer; i++) {
-        x[i] = base + i < n ? v[base + i] : 0;
+        x[i] = base + i < n ? src[base + i] : 0;
         t += x[i];
     }
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -177,13 +195,13 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_local(int *__restrict__ v
         wsum[lane] = w;  // inclusive over warps
     }
     __syncthreads();
-    int run = inc - t + (warp ? wsum[warp - 1] : 0);
+    int run = before + inc - t + (warp ? wsum[warp - 1] : 0);
 #pragma unroll
     for (int i = 0; i < kScanPer; i++) {
         if (base + i < n) v[base + i] = run;
         run += x[i];
     }
-    if (threadIdx.x == kScanThreads - 1) bsum[blockIdx.x] = run;
+    if (!WHOLE && threadIdx.x == kScanThreads - 1) bsum[blockIdx.x] = run;
 }
 // pass 2 (one block): exclusive scan of the block totals
 __global__ void __launch_bounds__(kScanThreads) k_scan_totals(int *bsum, int nb) {
@@ -273,6 +291,37 @@ __global__ void k_order_emit(const int *__restrict__ start, int T, int P, int ca
 
 // ------------------------------------------------------------- load/export
 // Bin particles given in storage order (float4 w = sid | species << 31).
+// Everything a load of positions resets: cell counts, remainders,
+// displacements, crossings, status, and in list mode the replicas' flags (every
+// list is built before the first step).  One launch for what were twelve
+// memsets and a copy.
+struct LoadReset {
+    int *cnt[3];
+    float *lo[3];
+    double *dsp[3];
+    int *img;         // [3][np] or nullptr
+    unsigned *status;
+    int n_status;
+    int *flag;        // [n_flag] set to 1, or nullptr
+    int n_flag;
+    long long C, np;
+};
+__global__ void k_load_reset(const __grid_constant__ LoadReset a) {
+    const long long t0 = (long long)blockIdx.x * blockDim.x + threadIdx.x, nt = (long long)gridDim.x * blockDim.x;
+    for (long long i = t0; i < a.C; i += nt)
+#pragma unroll
+        for (int k = 0; k < 3; k++) a.cnt[k][i] = 0;
+    for (long long i = t0; i < a.np; i += nt)
+#pragma unroll
+        for (int k = 0; k < 3; k++) {
+            a.lo[k][i] = 0.f;
+            a.dsp[k][i] = 0.0;
+            if (a.img) a.img[k * a.np + i] = 0;
+        }
+    for (long long i = t0; i < a.n_status; i += nt) a.status[i] = 0;
+    if (a.flag)
+        for (long long i = t0; i < a.n_flag; i += nt) a.flag[i] = 1;
+}
 __global__ void k_load(const float4 *__restrict__ staged, int P, const int *__restrict__ rep_of_sid,
                        const SysDev *sys, int *cnt, float4 *pos, int cap, double *x0, const int *gid_of,
                        unsigned *st, float4 *pos_sid) {
