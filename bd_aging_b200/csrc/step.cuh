@@ -352,7 +352,10 @@ __device__ void process_brick(const StepArgs &a, int bidx, long long ni, unsigne
             a.nbr_count[gid] = ps.nbr;
             a.nbr_hash[gid] = ps.hsh;
         }
-        if (!a.do_update) continue;
+        // observation passes never update, and known so at compile time the
+        // forces, caps and noise are not compiled in (66 registers instead of 72;
+        // 262144 particles: 130 us a pass instead of 146)
+        if (OBS || CENSUS || !a.do_update) continue;
         if (ni == 0) {  // origin of the unwrapped positions (main.cu:497-506)
             qx = qy = qz = 0.0;
             a.x0[3 * (size_t)gid] = (double)mx + (double)lx;
