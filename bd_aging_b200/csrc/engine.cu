@@ -1221,13 +1221,17 @@ int bd_engine_get_positions(bd_engine *e, float *pos_host, float *raw_host) {
         if (cudaMalloc(&e->out_pos, sizeof(float) * 3 * P) != cudaSuccess) return BD_ERR_NOMEM;
         if (cudaMalloc(&e->out_raw, sizeof(float) * 3 * P) != cudaSuccess) return BD_ERR_NOMEM;
     }
-    {
-        int rcb = sync_buckets(e);
-        if (rcb) return rcb;
+    if (e->list) {
+        // the binning reports a cell that holds more particles than it has slots for
+        if (int rc = list_bin(e, e->cur, e->d_one, nullptr)) return rc;
+        k_list_export<<<div_up((long)P, 256), 256, 0, e->stream>>>(e->lpos[e->cur & 1], e->lo[0], e->lo[1], e->lo[2],
+                                                                   e->img, e->x0, e->gid_of, e->rep_of_sid, e->d_sys,
+                                                                   (int)P, e->out_pos, e->out_raw);
+    } else {
+        k_export<<<div_up(e->C, 128), 128, 0, e->stream>>>(e->cnt[obs_buf(e)], e->pos[obs_buf(e)], (int)e->C, e->cap,
+                                                           (int)e->P, e->gid_of, e->x0, e->dsp[0], e->dsp[1],
+                                                           e->dsp[2], e->out_pos, e->out_raw, nullptr);
     }
-    k_export<<<div_up(e->C, 128), 128, 0, e->stream>>>(e->cnt[obs_buf(e)], e->pos[obs_buf(e)], (int)e->C, e->cap, (int)e->P, e->gid_of,
-                                                       e->x0, e->dsp[0], e->dsp[1], e->dsp[2], e->out_pos,
-                                                       e->out_raw, e->snap);
     BD_LAUNCH_CHECK();
     if (pos_host) BD_CUDA_TRY(cudaMemcpyAsync(pos_host, e->out_pos, sizeof(float) * 3 * P, cudaMemcpyDeviceToHost, e->stream));
     if (raw_host) BD_CUDA_TRY(cudaMemcpyAsync(raw_host, e->out_raw, sizeof(float) * 3 * P, cudaMemcpyDeviceToHost, e->stream));
