@@ -1,5 +1,5 @@
 // runtime.cuh -- host-side plumbing shared by the translation units of
-// libbd_aging_b200: status mapping, per-device workspace, launch checks.
+// libbd_aging_b200: status mapping, per-call workspaces, launch checks.
 #pragma once
 #include <cuda_runtime.h>
 

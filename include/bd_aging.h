@@ -17,7 +17,9 @@
  *     (big particles first, main.cu:377-394).
  *
  * All functions are thread-compatible (no hidden global state apart from
- * per-device kernel attributes); handles are not shared across threads.
+ * per-device kernel attributes and a fixed set of per-device workspaces, one
+ * held by each synchronous call at a time); handles are not shared across
+ * threads.
  */
 #ifndef BD_AGING_H
 #define BD_AGING_H
