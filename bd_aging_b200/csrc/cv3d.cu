@@ -17,7 +17,8 @@
 // slack on the squared range; a lane notes the partners that pass in a bit
 // mask per 32 (no branch in that loop), and the reference's arithmetic decides
 // on those, eight masks at a time.  Where that test could miss a pair (range
-// beyond 0.49 side, a coordinate far outside the box) every pair is noted.  A lane adds to a row of its own (a copy per warp, summed
+// beyond 0.49 side, a coordinate far outside the box) every pair is noted.  A
+// lane adds to a row of its own (a copy per warp, summed
 // at the end), so it needs no atomics; with H in memory it adds there.
 // Measured, 4000 particles, 24 bins to 3.5: 38 us a configuration (84 + 259 for
 // a warp per particle with a double-precision floor per component of every
@@ -369,8 +370,11 @@ int bd_cv3d_add_statistics(bd_cv3d *cv, const float *rr, const float *xx, int n,
     }
     double *d_part = static_cast<double *>(cv->d_work);
     float *d_H = fused ? nullptr : reinterpret_cast<float *>(static_cast<unsigned char *>(cv->d_work) + part);
-    // 16 warps a block where their copies of the rows fit, else 8
-    const int warps = cv_hits_smem(bins, fused, 16) <= (size_t)226 * 1024 ? 16 : 8;
+    // 16 warps a block where their copies of the rows fit beside the static
+    // shared memory (33 bins), else 8 (60 bins), else 4 (148 KB at kCvFused bins)
+    const size_t most = (size_t)227 * 1024 - 256;
+    int warps = 16;
+    while (warps > 4 && cv_hits_smem(bins, fused, warps) > most) warps /= 2;
     const size_t sm = cv_hits_smem(bins, fused, warps);
     if (sm > 48 * 1024) BD_CUDA_TRY(cudaFuncSetAttribute(k_cv_hits, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
     CallSlot w;

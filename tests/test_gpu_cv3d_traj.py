@@ -78,6 +78,30 @@ def test_cv3d_edges_match_the_oracle(n, bins, rng, side):
     assert np.linalg.norm(got - ref) <= bound
 
 
+@pytest.mark.parametrize("n,bins", [(700, 33), (700, 34), (700, 60), (700, 61), (40, 61), (1500, 64)])
+def test_cv3d_block_widths(n, bins):
+    """Bin counts on both sides of each width of the block, with the bound of
+    the edge cases above."""
+    g = np.random.default_rng(bins)
+    side, rng = 9.0, 4.0
+    pos = g.uniform(0, side, (n, 3)).astype(np.float32)
+    xx = g.normal(size=(n, 3)).astype(np.float32)
+    cv = B.Contracting_Vector3D(bins, rng)
+    cv.add_statistics(dev(pos), dev(xx), n, side)
+    cv.calculate_vector()
+    got = cv.get_vector().astype(np.float64)
+    ata, atb, bad = O.cv3d_add(bins, rng, pos, xx, side)
+    assert bad == 0
+    ref, bound = np.zeros(bins), 0.0
+    for c in range(3):
+        u, w, vt = np.linalg.svd(ata[c].astype(np.float64))
+        keep = w > 1e-6 * w[0]
+        x = vt[keep].T @ ((u[:, keep].T @ atb[c].astype(np.float64)) / w[keep])
+        ref += x / 3.0
+        bound += 2e-5 * w[0] / w[keep][-1] * np.linalg.norm(x) / 3.0
+    assert np.linalg.norm(got - ref) <= bound
+
+
 def test_cv3d_state_errors_replace_reference_throws():
     cv = B.Contracting_Vector3D(8, 2.0)
     with pytest.raises(B.BDError) as e1:
