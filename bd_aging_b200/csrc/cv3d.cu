@@ -42,6 +42,7 @@ constexpr int kCvBlock = 32;   // particles per block
 constexpr int kCvTile = 1024;  // partners staged at a time
 constexpr int kCvMasks = 8;    // masks of 32 partners a lane notes before they are settled
 constexpr int kCvFused = 64;
+constexpr size_t kCvSmemMost = (size_t)227 * 1024 - 256;  // beside the static shared memory
 struct CvHits {
     const float *rr, *xx;
     int n;
@@ -340,6 +341,10 @@ int bd_cv3d_create(int bins, float range, bd_cv3d **out) {
     cv->range = range;
     cv->result.assign(bins, 0.f);
     const size_t sums = 3 * (size_t)bins * bins + 3 * (size_t)bins;
+    if (int rc = allow_smem(k_cv_hits, kCvSmemMost)) {
+        bd_cv3d_destroy(cv);
+        return rc;
+    }
     if (cudaMalloc(&cv->d_ata, sizeof(double) * sums) != cudaSuccess) {
         bd_cv3d_destroy(cv);
         return BD_ERR_NOMEM;
@@ -372,11 +377,9 @@ int bd_cv3d_add_statistics(bd_cv3d *cv, const float *rr, const float *xx, int n,
     float *d_H = fused ? nullptr : reinterpret_cast<float *>(static_cast<unsigned char *>(cv->d_work) + part);
     // 16 warps a block where their copies of the rows fit beside the static
     // shared memory (33 bins), else 8 (60 bins), else 4 (148 KB at kCvFused bins)
-    const size_t most = (size_t)227 * 1024 - 256;
     int warps = 16;
-    while (warps > 4 && cv_hits_smem(bins, fused, warps) > most) warps /= 2;
+    while (warps > 4 && cv_hits_smem(bins, fused, warps) > kCvSmemMost) warps /= 2;
     const size_t sm = cv_hits_smem(bins, fused, warps);
-    if (sm > 48 * 1024) BD_CUDA_TRY(cudaFuncSetAttribute(k_cv_hits, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
     CallSlot w;
     if (!w.ok()) return BD_ERR_NOMEM;
     if (!fused) BD_CUDA_TRY(cudaMemsetAsync(d_H, 0, sizeof(float) * 3 * (size_t)n * bins, s));

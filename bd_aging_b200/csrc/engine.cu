@@ -56,11 +56,7 @@ StepArgs make_args(bd_engine *e, int buf, int do_update) {
 template <int RNG, bool OBS, bool CENSUS>
 int launch_step_t(bd_engine *e, const StepArgs &a, int ni_off, bool attr_only = false) {
     auto kern = k_step<RNG, OBS, CENSUS>;
-    if (attr_only) {
-        BD_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)(CENSUS ? e->smem_census : e->smem)));
-        return BD_OK;
-    }
+    if (attr_only) return allow_smem(kern, CENSUS ? e->smem_census : e->smem);
     kern<<<e->nbricks, e->threads, CENSUS ? e->smem_census : e->smem, e->stream>>>(a, e->d_ni, ni_off);
     BD_LAUNCH_CHECK();
     return BD_OK;
@@ -69,10 +65,7 @@ int launch_step_t(bd_engine *e, const StepArgs &a, int ni_off, bool attr_only = 
 template <int RNG>
 int launch_persistent_t(bd_engine *e, const StepArgs &a, int nsteps, bool attr_only = false) {
     auto kern = k_step_persistent<RNG>;
-    if (attr_only) {
-        BD_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)e->smem));
-        return BD_OK;
-    }
+    if (attr_only) return allow_smem(kern, e->smem);
     cudaLaunchConfig_t cfg;
     std::memset(&cfg, 0, sizeof(cfg));
     cfg.gridDim = dim3(e->nclusters * e->cluster);
@@ -141,24 +134,15 @@ int configure_kernels(bd_engine *e) {
     BD_ATTR(kRngNoise)
     BD_ATTR(kRngRannew64)
 #undef BD_ATTR
-    if (cudaFuncSetAttribute(k_list_build, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)e->lsmem) != cudaSuccess)
-        rc = 1;
-    if (e->lgr_blocks > 0 && cudaFuncSetAttribute(grid_kernel(e), cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                  (int)grid_smem_bytes(e->lgr_owners)) != cudaSuccess)
-        rc = 1;
+    rc |= allow_smem(k_list_build, e->lsmem);
+    if (e->lgr_blocks > 0) rc |= allow_smem(grid_kernel(e), grid_smem_bytes(e->lgr_owners));
     if (e->lcl_ctas > 0) {
-        if (cudaFuncSetAttribute(k_list_cluster<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)e->lcl_smem) != cudaSuccess ||
-            cudaFuncSetAttribute(k_list_cluster<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)e->lcl_smem) != cudaSuccess)
-            rc = 1;
+        rc |= allow_smem(k_list_cluster<false>, e->lcl_smem);
+        rc |= allow_smem(k_list_cluster<true>, e->lcl_smem);
     }
     if (e->lrep_smem > 0) {  // variant 5: resident positions or rebuilds in shared memory
-        if (cudaFuncSetAttribute(k_list_replica<false, 5>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)e->lrep_smem) != cudaSuccess ||
-            cudaFuncSetAttribute(k_list_replica<true, 5>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)e->lrep_smem) != cudaSuccess)
-            rc = 1;
+        rc |= allow_smem(k_list_replica<false, 5>, e->lrep_smem);
+        rc |= allow_smem(k_list_replica<true, 5>, e->lrep_smem);
     }
     return rc ? BD_ERR_CUDA : BD_OK;
 }

@@ -609,7 +609,7 @@ int run_gder(bd_engine *e, std::vector<int> &m_of, int nbins, float range, unsig
         BD_CUDA_TRY(cudaMemcpyAsync(d_m, m_of.data(), sizeof(int) * e->R, cudaMemcpyHostToDevice, st));
         BD_CUDA_TRY(cudaMemsetAsync(d_bad, 0, sizeof(int) * e->R, st));
         const size_t sm = gder_cells_smem(nbins);
-        BD_CUDA_TRY(cudaFuncSetAttribute(k_gr_cells, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+        if (int rc = allow_smem(k_gr_cells, sm)) return rc;
         GrArgs a;
         a.sys = e->d_sys;
         a.cnt = e->cnt[obs_buf(e)];
@@ -662,7 +662,7 @@ int run_gder(bd_engine *e, std::vector<int> &m_of, int nbins, float range, unsig
     a.jchunk = (int)std::min(8192.0, std::max(64.0, 64.0 * std::ceil(want / 64.0)));
     const size_t sm = 3 * kGrPairTile * sizeof(float) + sizeof(unsigned) * 3 * ((size_t)nbins + kGrSpare);
     if (sm > 48 * 1024)
-        BD_CUDA_TRY(cudaFuncSetAttribute(k_gr_pairs, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+        if (int rc = allow_smem(k_gr_pairs, sm)) return rc;
     const int most = 65535;  // grid limit of y and z
     a.jchunk = std::max(a.jchunk, div_up(nmax, most));
     for (size_t first = 0; first < reps.size(); first += most) {

@@ -848,7 +848,8 @@ int bd_get_gder(char type, char type_other, const float *rr, const float *rr_oth
     const bool check = !(a.bins.near <= edge * edge);
     auto kern = same ? (check ? k_gder<true, true> : k_gder<true, false>)
                      : (check ? k_gder<false, true> : k_gder<false, false>);
-    if (sm > 48 * 1024) BD_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+    if (sm > 48 * 1024)
+        if (int rc = allow_smem(kern, sm)) return rc;
     kern<<<grid, kGderThreads, sm, s>>>(a);
     BD_LAUNCH_CHECK();
     return BD_OK;

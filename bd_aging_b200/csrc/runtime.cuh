@@ -68,4 +68,22 @@ inline int status_from_bits(unsigned bits) {
 
 inline int div_up(long a, long b) { return (int)((a + b - 1) / b); }
 
+// Lets launches of `kern` take as much dynamic shared memory as the device
+// gives a block; a launch passes what it needs, `bytes` at most (BD_ERR_CUDA
+// when that does not fit).  The limit belongs to the kernel on its device, not
+// to the engine or call that sets it: every caller sets the same value, so that
+// none lowers it below what another's launches need.
+template <class K>
+inline int allow_smem(K kern, size_t bytes) {
+    int dev = 0, most = 0;
+    cudaFuncAttributes at;
+    BD_CUDA_TRY(cudaGetDevice(&dev));
+    BD_CUDA_TRY(cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
+    BD_CUDA_TRY(cudaFuncGetAttributes(&at, kern));
+    most -= (int)at.sharedSizeBytes;
+    if (bytes > (size_t)most) return BD_ERR_CUDA;
+    BD_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, most));
+    return BD_OK;
+}
+
 }  // namespace bd

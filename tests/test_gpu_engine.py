@@ -290,6 +290,40 @@ def test_resident_launches_match_the_per_step_kernels(sizes, kw):
             np.testing.assert_array_equal(a, b)
 
 
+@pytest.mark.parametrize("big,small,kw", [
+    ([(16000, 16768)], [(2000, 2000)], {}), ([(1000, 1000)], [(60, 60)], {}),
+    ([(2000, 2000)] * 3, [(100, 100)] * 2, {"list_variant": 5}),
+    ([(700, 700)], [(100, 100)], {"neighbor_skin": 0.0, "brick": (5, 4, 4), "threads": 192})])
+def test_engines_of_different_sizes_run_in_turn(big, small, kw):
+    """A live engine keeps running after a smaller one of the same launch
+    (whole grid, cluster, block per replica, sweep) is created: shared-memory
+    limits are the kernel's, not the engine's.  Bits of the engine run alone,
+    over direct launches, a graph of its own and one built afterwards."""
+    def make(sizes, kw):
+        parts = [system(nb, ns, 0.4, 5 + k, T0=1.0, force_cap=100.0) for k, (nb, ns) in enumerate(sizes)]
+        e = B.Engine([s for s, _ in parts], **kw)
+        e.set_positions(np.concatenate([p for _, p in parts]))
+        return e
+    alone = make(big, kw)
+    for k in (3, 5, 96, 7):
+        alone.run(k)
+    want = alone.get_positions()
+    alone.close()
+    first = make(big, kw)
+    first.run(3)
+    second = make(small, dict(kw, brick=(2, 2, 2), threads=64) if "brick" in kw else kw)
+    second.run(2)
+    for k in (5, 96, 7):
+        first.run(k)
+        second.run(k)
+    got = first.get_positions()
+    first.observe()
+    first.close()
+    second.close()
+    for a, b in zip(got, want):
+        np.testing.assert_array_equal(a, b)
+
+
 def test_first_step_temperature_carried_over():
     """A replica given T_first takes its first update at that temperature and
     then follows its protocol (the drop-in executable uses this for
