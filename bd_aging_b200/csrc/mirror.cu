@@ -189,6 +189,13 @@ __global__ void k_cell_sort_long(const int *nocup, int *cell_vec, int nc3, int n
 // on an SM (16384 particles).  A warp per particle walks it once or four times
 // and fills the chip; with more particles fewer lanes each, and so fewer
 // instructions, win (launch_forces).
+template <int G>  // the aligned group of G lanes that `lane` belongs to
+__host__ __device__ constexpr unsigned lanes_of_group(int lane) {
+    return (unsigned)(((1ull << G) - 1ull) << (lane & ~(G - 1)));
+}
+static_assert(lanes_of_group<32>(5) == 0xffffffffu && lanes_of_group<8>(0) == 0xffu &&
+                  lanes_of_group<8>(15) == 0xff00u && lanes_of_group<8>(31) == 0xff000000u,
+              "a particle's lanes");
 template <bool SAME, int G, int W>
 __global__ void k_forces(const float *__restrict__ rr, float *ff, float *vir, float *pot,
                          const float *__restrict__ rr_o, const int *__restrict__ nocup,
@@ -245,7 +252,9 @@ __global__ void k_forces(const float *__restrict__ rr, float *ff, float *vir, fl
         }
     }
     if (G > 1) {
-        const unsigned mask = __activemask();
+        // this particle's lanes: they left together at m >= n, and the loop has not
+        // rejoined them, which the shuffles do for the lanes they name
+        const unsigned mask = lanes_of_group<G>(threadIdx.x & 31);
 #pragma unroll
         for (int o = G / 2; o; o >>= 1) {
             fx += __shfl_xor_sync(mask, fx, o);

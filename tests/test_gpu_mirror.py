@@ -93,6 +93,21 @@ def test_cell_sort_and_force_paths_match_the_oracle(nb, ns, ntags):
         np.testing.assert_allclose(v, ref[k], rtol=2e-5, atol=2e-5 * np.abs(ref[k]).max(), err_msg=k)
 
 
+@pytest.mark.parametrize("nb,ns", [(1000, 1200), (8200, 9000)])
+def test_forces_of_a_drop_match_the_oracle(nb, ns):
+    """A dense drop in an empty box: the lanes of a particle (32, then eight)
+    visit full, half-full and empty cells, so they leave the cell loop at
+    different times, and their sums still meet.  Same bounds as above."""
+    inner = CF.side_from_phi(nb, ns, 0.5)
+    side = float(np.float32(1.6 * inner))
+    pos = (CF.lattice_config(nb, ns, inner, 23) + np.float32(0.2 * inner)).astype(np.float32)
+    p = O.setup_params(side, nb, ns, float(CF.SIGMA_BIG), float(CF.SIGMA_SML), ntags=(16, 16))
+    pp = B.Parametros.from_buffer_copy(bytes(p))
+    out, ref = forces_four_calls(pp, pos[:nb], pos[nb:]), O.ref_forces(p, pos[:nb].copy(), pos[nb:].copy())
+    for k, v in out.items():
+        np.testing.assert_allclose(v, ref[k], rtol=2e-5, atol=2e-5 * np.abs(ref[k]).max(), err_msg=k)
+
+
 @pytest.mark.parametrize("name", SYSTEMS)
 def test_update_noise_bit_exact(golden, name):
     p = params(golden, name)
