@@ -83,11 +83,15 @@ struct GrArgs {
     unsigned *status;
 };
 
-// bounds of the estimate for positions shifted by up to one side of a box
-// (coordinates up to 1.5 L: half an ulp of each, below 2^-24 1.5 L)
+// Bounds of the estimate for positions shifted by a side of the box.  Per
+// component, x_j + s is off by half an ulp and the reference, which rounds
+// x_i - x_j first, by half an ulp of that.  At a distance d across a face the
+// two are below L + d and L - d in size, so their errors add up to less than
+// 2^-24 2 L (and reach it: on equal grids a tie may round either way).
 __device__ __forceinline__ GrBins gr_with_shift(GrBins g, float side, float range) {
-    const float err = 1.6e-7f * side;  // sqrt(3) 2^-24 1.5 L
-    g.near *= 1.f + 2.f * err / range;
+    const float err = 2.1e-7f * side;  // sqrt(3) 2^-24 2 L
+    const float f = 1.f + err / range;
+    g.near *= f * f;
     g.c0 += 1.1f * err * g.inv_bin;
     return g;
 }
