@@ -223,10 +223,11 @@ __global__ void __launch_bounds__(kGridMaxOwners, 1)
         if (need) {
             const bool mine = a.flag[rep] != 0;
             const int me = blockIdx.x * blockDim.x + threadIdx.x, all = gridDim.x * blockDim.x;
-            for (int r = 0; r < a.nrep; r++) {
-                if (a.flag[r] == 0) continue;
-                const int cells = a.sys[r].ncell * a.sys[r].ncell * a.sys[r].ncell, base = a.sys[r].cell_base;
-                for (int c = me; c < cells; c += all) lp.cnt[base + c] = 0;
+            // a flagged replica's particles clear its cells (a walk over the
+            // replicas by every thread took 0.15 us a replica, 38 us at 300)
+            if (owner && live && mine) {
+                const int cells = S.ncell * S.ncell * S.ncell, n = S.n, base = S.cell_base;
+                for (int c = sid - S.part_base; c < cells; c += n) lp.cnt[base + c] = 0;
             }
             if (!grid_sync()) return;
             if (me < a.nrep || (blockIdx.x == 0 && threadIdx.x == 0)) {  // every block has read the flags
