@@ -517,11 +517,32 @@ int rebuild_bricks(bd_engine *e) {
     return BD_OK;
 }
 
+// Estimated us a step of the batch, one block per replica (variant 5's
+// launch): of the most loaded SM, blocks going to SMs largest replica first,
+// 1.5 a block and 5.2 per 1000 particles with resident positions, 5.9 without.
+// Measured / estimated: 148 x 150 2.9 / 2.3, 100 x 700 5.0 / 5.1, 38 x 1000 6.2
+// / 6.7, 150 x 500 7.1 / 8.2, 300 x 250 7.7 / 8.4, 40 x 1900 11.5 / 11.4,
+// 60 x 3000 17 / 17, 148 x 6000 33 / 33, 256 of 500 to 8000 50 / 49,
+// 250 x 8000 97 / 97.
+double replica_step_us(const bd_engine *e, int sms) {
+    std::vector<double> load(std::max(1, sms), 0.0);
+    std::vector<int> sizes;
+    for (const SysDev &S : e->sysh) sizes.push_back(S.n);
+    std::sort(sizes.begin(), sizes.end(), std::greater<int>());
+    std::make_heap(load.begin(), load.end(), std::greater<double>());
+    for (int n : sizes) {
+        std::pop_heap(load.begin(), load.end(), std::greater<double>());
+        load.back() += 1.5 + (e->lrep_resident ? 5.2e-3 : 5.9e-3) * n;
+        std::push_heap(load.begin(), load.end(), std::greater<double>());
+    }
+    return *std::max_element(load.begin(), load.end());
+}
+
 // Variant 0 runs small replicas in clusters (nlist_cluster.cuh): the most CTAs
 // per replica (up to 8) that leave every replica resident at once, one thread
-// per particle; other batches of up to 512 particles per SM on the whole grid
-// (nlist_grid.cuh); larger batches of many replicas one block per replica.
-// The others keep the per-step kernels.
+// per particle.  Other batches run on the whole grid (nlist_grid.cuh, up to
+// 512 particles per SM), one block per replica, or step by step (the per-step
+// kernels), whichever is estimated to be the fastest.
 void choose_resident(bd_engine *e) {
     int nmax = 0, cmax = 0;
     for (const SysDev &S : e->sysh) {
@@ -539,39 +560,30 @@ void choose_resident(bd_engine *e) {
         e->lcl_cells = cmax;
         return;
     }
-    // Batches of up to 512 particles per SM: the whole grid resident, 128
-    // particles per block until every SM has one
     int sms = 0, coop = 0;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, e->dev);
     cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, e->dev);
-    if (coop && e->P <= (long long)sms * kGridMaxOwners) {
+    // The more replicas a batch has, the more of its steps rebuild some of
+    // them, which costs the grid 28 us (two more barriers and a chain of loads
+    // through 27 cells) and the per-step kernels up to 20.  The slopes are
+    // between those of cold and hot systems.  Measured at T = 0.1 and 1, grid /
+    // per replica: 2 x 32768 4.4, 6.4 / 150, 213; 10 x 7000 6.0, 12 / 39, 45;
+    // 18 x 4000 6.5, 17 / 21, 25; 60 x 1000 9.2, 28 / 5.9, 7.0; 100 x 700 12, 31
+    // / 4.8, 5.2; 150 x 500 16, 35 / 6.7, 7.5; 300 x 250 21, 33 / 7.3, 8.3.
+    // Per-step kernels / per replica: 256 of 500 to 8000 79 / 50, 148 x 6000 63 /
+    // 33, 60 x 3000 25 / 17, 1000 x 500 62 / 24, 250 x 8000 110 / 97, 64 x 32768
+    // 93 / 195 (estimated).
+    const bool grid = coop && e->P <= (long long)sms * kGridMaxOwners;
+    const double other = grid ? 3.0 + 3.0e-5 * (double)e->P + std::min(28.0, 0.11 * e->R)
+                              : 6.0 + 4.3e-5 * (double)e->P + std::min(20.0, 0.08 * e->R);
+    if (replica_step_us(e, sms) < other) {
+        e->lrep_default = true;
+    } else if (grid) {  // 128 particles per block until every SM has one
         const int G = std::min(sms, div_up(e->P, 128));
         e->lgr_owners = (div_up(e->P, G) + 31) / 32 * 32;
         e->lgr_help = 2 * e->lgr_owners <= kGridMaxOwners;
         e->lgr_blocks = G;
-        return;
     }
-    // Many replicas, none much larger than an SM's share: variant 5's launch.
-    // Its step takes 5.5 us per 1000 particles of the most loaded SM (blocks go
-    // to SMs largest replica first) with resident positions, 6.2 without; the
-    // per-step kernels' 6 us, 43 us per million particles and, since some
-    // replica rebuilds in most steps of a large batch, up to 20 us of rebuild
-    // passes.  Measured, us a step, this launch / per-step: 256 replicas of 500
-    // to 8000 50 / 79, 148 x 6000 33 / 63, 60 x 3000 17 / 25, 1000 x 500 24 / 62,
-    // 250 x 8000 97 / 110; 64 x 32768 (183 by this rule) / 93.
-    std::vector<long long> load(std::max(1, sms), 0);
-    std::vector<int> sizes;
-    for (const SysDev &S : e->sysh) sizes.push_back(S.n);
-    std::sort(sizes.begin(), sizes.end(), std::greater<int>());
-    std::make_heap(load.begin(), load.end(), std::greater<long long>());
-    for (int n : sizes) {
-        std::pop_heap(load.begin(), load.end(), std::greater<long long>());
-        load.back() += n;
-        std::push_heap(load.begin(), load.end(), std::greater<long long>());
-    }
-    const double most = (double)*std::max_element(load.begin(), load.end());
-    e->lrep_default = (e->lrep_resident ? 5.5e-3 : 6.2e-3) * most <
-                      6.0 + 4.3e-5 * (double)e->P + std::min(20.0, 0.08 * e->R);
 }
 
 // Upload the brick layout (after rebuild_bricks) and drop graphs recorded
