@@ -538,52 +538,99 @@ double replica_step_us(const bd_engine *e, int sms) {
     return *std::max_element(load.begin(), load.end());
 }
 
-// Variant 0 runs small replicas in clusters (nlist_cluster.cuh): the most CTAs
-// per replica (up to 8) that leave every replica resident at once, one thread
-// per particle.  Other batches run on the whole grid (nlist_grid.cuh, up to
-// 512 particles per SM), one block per replica, or step by step (the per-step
-// kernels), whichever is estimated to be the fastest.
+// Clusters of C CTAs of k_list_cluster that run at once with an SM to each CTA
+// (0 if none can): clusters are placed within a GPC, so fewer than SMs / C.  At
+// least 120 KB of shared memory stands for the SM of its own.
+int cluster_capacity(int C, int owners, size_t smem) {
+    if (allow_smem(k_list_cluster<false>, smem) != BD_OK) return 0;
+    cudaLaunchConfig_t cfg;
+    std::memset(&cfg, 0, sizeof(cfg));
+    cfg.gridDim = dim3(C);
+    cfg.blockDim = dim3(2 * owners);
+    cfg.dynamicSmemBytes = std::max(smem, (size_t)120 * 1024);
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = C;
+    at[0].val.clusterDim.y = 1;
+    at[0].val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    int n = 0;
+    if (cudaOccupancyMaxActiveClusters(&n, k_list_cluster<false>, &cfg) != cudaSuccess) {
+        cudaGetLastError();
+        return 0;
+    }
+    return n;
+}
+
+// Variant 0 runs a batch of steps in clusters (nlist_cluster.cuh, small
+// replicas, one thread per particle), on the whole grid (nlist_grid.cuh, up to
+// 512 particles per SM) or one block per replica, or step by step (the
+// per-step kernels), whichever is estimated to be the fastest.
 void choose_resident(bd_engine *e) {
     int nmax = 0, cmax = 0;
     for (const SysDev &S : e->sysh) {
         nmax = std::max(nmax, S.n);
         cmax = std::max(cmax, S.ncell * S.ncell * S.ncell);
     }
+    // Clusters: as many rounds as the resident ones take, at an estimated 1.2 us
+    // a step and 5 per 1000 particles of a CTA (its owners rounded up to warps)
+    // and 0.3 per 1000 of the replica.  Measured / estimated at T = 0.5: 1 x 1000
+    // on 8 CTAs 2.1 / 2.1, 30 x 1000 on 4 2.5 / 2.8, 148 x 250 on 1 2.5 / 2.6,
+    // 15 x 1900 on 8 3.0 / 3.1; in two rounds 34 x 1000 on 4 4.4 / 5.6, 18 x 1900
+    // on 8 5.7 / 6.1.
+    double cluster_us = 1e30;
     for (int C = kClusterMaxCtas; C >= 1; C /= 2) {
         const int T = std::max(32, (div_up(nmax, C) + 31) / 32 * 32);
         const size_t sm = cluster_smem_bytes(nmax, cmax, T);
-        if ((long long)e->R * C > 148 || T > kClusterMaxOwners || sm > (size_t)226 * 1024) continue;
+        if (T > kClusterMaxOwners || sm > (size_t)226 * 1024) continue;
+        const int at_once = cluster_capacity(C, T, sm);
+        if (at_once < 1) continue;
+        const double us = div_up(e->R, at_once) * (1.2 + 5e-3 * T + 3e-4 * nmax);
+        if (us >= cluster_us) continue;
+        cluster_us = us;
         e->lcl_ctas = C;
         e->lcl_owners = T;
         e->lcl_smem = sm;
         e->lcl_nmax = nmax;
         e->lcl_cells = cmax;
-        return;
     }
     int sms = 0, coop = 0;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, e->dev);
     cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, e->dev);
     // The more replicas a batch has, the more of its steps rebuild some of
     // them, which costs the grid 28 us (two more barriers and a chain of loads
-    // through 27 cells) and the per-step kernels up to 20.  The slopes are
-    // between those of cold and hot systems.  Measured at T = 0.1 and 1, grid /
+    // through 27 cells) and the per-step kernels up to 20.  The slopes lie
+    // between those of cold and hot systems.  Measured at T = 0.1, 1, grid /
     // per replica: 2 x 32768 4.4, 6.4 / 150, 213; 10 x 7000 6.0, 12 / 39, 45;
     // 18 x 4000 6.5, 17 / 21, 25; 60 x 1000 9.2, 28 / 5.9, 7.0; 100 x 700 12, 31
     // / 4.8, 5.2; 150 x 500 16, 35 / 6.7, 7.5; 300 x 250 21, 33 / 7.3, 8.3.
     // Per-step kernels / per replica: 256 of 500 to 8000 79 / 50, 148 x 6000 63 /
     // 33, 60 x 3000 25 / 17, 1000 x 500 62 / 24, 250 x 8000 110 / 97, 64 x 32768
     // 93 / 195 (estimated).
-    const bool grid = coop && e->P <= (long long)sms * kGridMaxOwners;
-    const double other = grid ? 3.0 + 3.0e-5 * (double)e->P + std::min(28.0, 0.11 * e->R)
-                              : 6.0 + 4.3e-5 * (double)e->P + std::min(20.0, 0.08 * e->R);
-    if (replica_step_us(e, sms) < other) {
-        e->lrep_default = true;
-    } else if (grid) {  // 128 particles per block until every SM has one
+    bool grid = coop && e->P <= (long long)sms * kGridMaxOwners;
+    if (grid) {  // 128 particles per block until every SM has one, all resident
         const int G = std::min(sms, div_up(e->P, 128));
         e->lgr_owners = (div_up(e->P, G) + 31) / 32 * 32;
         e->lgr_help = 2 * e->lgr_owners <= kGridMaxOwners;
-        e->lgr_blocks = G;
+        const size_t sm = grid_smem_bytes(e->lgr_owners);
+        int per_sm = 0;
+        if (allow_smem(grid_kernel(e), sm) != BD_OK ||
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, grid_kernel(e),
+                                                          e->lgr_owners * (e->lgr_help ? 2 : 1), sm) != cudaSuccess) {
+            cudaGetLastError();
+            per_sm = 0;
+        }
+        grid = per_sm > 0;
+        if (grid) e->lgr_blocks = G;
     }
+    const double other = grid ? 3.0 + 3.0e-5 * (double)e->P + std::min(28.0, 0.2 * e->R)
+                              : 6.0 + 4.3e-5 * (double)e->P + std::min(20.0, 0.08 * e->R);
+    const double replica_us = replica_step_us(e, sms);
+    const bool cluster = cluster_us <= std::min(other, replica_us);
+    e->lrep_default = !cluster && replica_us < other;
+    if (!cluster) e->lcl_ctas = 0;
+    if (cluster || e->lrep_default) e->lgr_blocks = 0;
 }
 
 // Upload the brick layout (after rebuild_bricks) and drop graphs recorded

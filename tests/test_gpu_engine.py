@@ -324,6 +324,28 @@ def test_engines_of_different_sizes_run_in_turn(big, small, kw):
         np.testing.assert_array_equal(a, b)
 
 
+@pytest.mark.parametrize("sizes", [[(500, 500)] * 16, [(300, 301)] * 40, [(900, 1000)] * 17, [(120, 130)] * 149])
+def test_clusters_in_several_rounds_match_the_per_step_kernels(sizes):
+    """Replica counts just past what fits at once, with an SM to each CTA, at 8, 4
+    and 1 CTAs: fewer CTAs each or more rounds, and the same bits."""
+    systems, poss = [], []
+    for k, (nb, ns) in enumerate(sizes):
+        s, p = system(nb, ns, 0.4, 31 + k, T0=3.0, force_cap=100.0)
+        systems.append(s)
+        poss.append(p)
+    pos = np.concatenate(poss)
+    out = []
+    for v in (1, None):
+        e = B.Engine(list(systems), list_variant=v)
+        e.set_positions(pos)
+        e.run(103)
+        info = e.info()
+        out.append((*e.get_positions(), *e.census(), np.array([info.list_builds, info.list_rebuild_steps])))
+        e.close()
+    for a, b in zip(*out):
+        np.testing.assert_array_equal(a, b)
+
+
 def test_first_step_temperature_carried_over():
     """A replica given T_first takes its first update at that temperature and
     then follows its protocol (the drop-in executable uses this for
