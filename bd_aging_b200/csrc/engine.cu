@@ -1068,7 +1068,9 @@ int autotune_list(bd_engine *e, long long &nsteps) {
             if (e->rng == BD_RNG_PHILOX) stage2.push_back({e->bx, e->by, e->bz, v});
             continue;
         }
-        if (v == 0 && (e->lcl_ctas > 0 || e->lgr_blocks > 0 || e->lrep_default)) {
+        // variant 0 in one launch a batch (Philox noise; the other streams run it
+        // step by step, with lists built by bricks)
+        if (v == 0 && e->rng == BD_RNG_PHILOX && (e->lcl_ctas > 0 || e->lgr_blocks > 0 || e->lrep_default)) {
             stage2.push_back({e->bx, e->by, e->bz, v});
             continue;
         }

@@ -253,6 +253,30 @@ def test_list_autotuner_and_launch_variants_change_speed_not_results():
         B.Engine(list(systems), list_variant=6)
 
 
+@pytest.mark.parametrize("rng,variant,steps", [("curand", 0, 72), ("curand", None, 212), ("rannew64", 0, 72),
+                                               ("philox", 0, 99)])
+def test_list_autotuner_tries_build_bricks_where_steps_are_launched_one_by_one(rng, variant, steps):
+    """The streams other than Philox run variant 0 step by step, so its build
+    brick is tuned: five shapes over 2 + 12 steps, for each of the three
+    variants when none is given.  With Philox a small replica's variant 0 is
+    one launch a batch, timed over 2 + 96 steps.  A run one step longer than
+    the tuner needs is tuned, and its bits are an untuned run's."""
+    s, pos = system(300, 300, 0.45, 9, T0=0.5, force_cap=100.0)
+    need = {("curand", 0): 70, ("rannew64", 0): 70, ("curand", None): 210, ("philox", 0): 98}[rng, variant]
+    out = []
+    for tune in (0, 1):
+        e = B.Engine([s], rng=rng, list_variant=variant, autotune=tune)
+        e.set_positions(pos)
+        e.run(need)  # too short to tune
+        assert e.info().tuned_ms == 0
+        e.run(steps)
+        assert (e.info().tuned_ms > 0) == bool(tune)
+        out.append(e.get_positions())
+        e.close()
+    np.testing.assert_array_equal(out[0][0], out[1][0])
+    np.testing.assert_array_equal(out[0][1], out[1][1])
+
+
 @pytest.mark.parametrize("sizes,kw", [
     ([(40, 41)], {}), ([(2048, 2040)], {}), ([(500, 500)], {"potential": "wca"}),
     ([(60 + 7 * k, 71 + 3 * k) for k in range(20)], {}), ([(300, 30 + k) for k in range(60)], {}),
