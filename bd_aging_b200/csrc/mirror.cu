@@ -160,13 +160,13 @@ __global__ void k_cell_sort(const int *nocup, int *cell_vec, int nc3, int ntags)
     int *v = cell_vec + (size_t)c * ntags;
     const int key = t < k ? v[t] : INT_MAX;
     int rank = 0;
-#pragma unroll
-    for (int u = 0; u < G; u++) rank += __shfl_sync(0xffffffffu, key, u, G) < key;
+    const int most = __reduce_max_sync(0xffffffffu, k);  // of the warp's cells: two or three, not G
+    for (int u = 0; u < most; u++) rank += __shfl_sync(0xffffffffu, key, u, G) < key;
     if (t < k) v[rank] = key;
     else if (live && t < ntags) v[t] = -1;
 }
-// The same for more slots per cell, a thread per cell (unused slots cleared
-// before the binning).
+// The same for more slots per cell or many cells, a thread per cell (unused
+// slots cleared before the binning).
 __global__ void k_cell_sort_long(const int *nocup, int *cell_vec, int nc3, int ntags) {
     int c = blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= nc3) return;
@@ -713,13 +713,20 @@ int bd_cell_locate(char type, const float *rr, int *nocup, int *cell_vec, const 
     CallSlot w;
     if (!w.ok()) return BD_ERR_NOMEM;
     BD_CUDA_TRY(cudaMemsetAsync(nocup, 0, sizeof(int) * (size_t)nc3, s));
-    if (ntags > 32) BD_CUDA_TRY(cudaMemsetAsync(cell_vec, 0xff, sizeof(int) * (size_t)nc3 * ntags, s));
+    // 16 or 32 lanes per cell (a call's time, us, lanes / a thread per cell: 16
+    // slots 27 / 32 at 343 cells, 25 / 30 at 35937, 29 / 30 at 68921, 35 / 31 at
+    // 250047, 110 / 53 at 1.8 million; 32 slots 25 / 33 at 9261, 28 / 28 at 35937,
+    // 46 / 32 at 250047): up to a million lanes the launch and clear saved count
+    // more, beyond it the lanes that hold no entry do
+    const int lanes = ntags <= 16 ? 16 : 32;
+    const bool by_lanes = ntags <= 32 && (long long)nc3 * lanes <= 1 << 20;
+    if (!by_lanes) BD_CUDA_TRY(cudaMemsetAsync(cell_vec, 0xff, sizeof(int) * (size_t)nc3 * ntags, s));
     if (n > 0) {
         k_cell_bin<<<div_up(n, 256), 256, 0, s>>>(rr, n, csi, ncell, ntags, nocup, cell_vec, w.status());
         BD_LAUNCH_CHECK();
     }
-    if (ntags <= 16) k_cell_sort<16><<<div_up((long)nc3 * 16, 256), 256, 0, s>>>(nocup, cell_vec, nc3, ntags);
-    else if (ntags <= 32) k_cell_sort<32><<<div_up((long)nc3 * 32, 256), 256, 0, s>>>(nocup, cell_vec, nc3, ntags);
+    if (by_lanes && lanes == 16) k_cell_sort<16><<<div_up((long)nc3 * 16, 256), 256, 0, s>>>(nocup, cell_vec, nc3, ntags);
+    else if (by_lanes) k_cell_sort<32><<<div_up((long)nc3 * 32, 256), 256, 0, s>>>(nocup, cell_vec, nc3, ntags);
     else k_cell_sort_long<<<div_up(nc3, 256), 256, 0, s>>>(nocup, cell_vec, nc3, ntags);
     BD_LAUNCH_CHECK();
     return read_status(w, s);

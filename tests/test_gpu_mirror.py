@@ -93,6 +93,24 @@ def test_cell_sort_and_force_paths_match_the_oracle(nb, ns, ntags):
         np.testing.assert_allclose(v, ref[k], rtol=2e-5, atol=2e-5 * np.abs(ref[k]).max(), err_msg=k)
 
 
+@pytest.mark.parametrize("per_side,ntags", [(40, 16), (41, 16), (32, 17), (33, 17), (32, 32), (33, 32)])
+def test_cell_lists_on_both_sides_of_the_lane_limit(per_side, ntags):
+    """2^20 lanes in all (16 per cell, or 32 with more slots): cells sorted by
+    lanes up to there, by a thread each beyond, unused slots -1 either way."""
+    ss = float(CF.SIGMA_SML)
+    side = float(np.float32((per_side + 0.5) * 1.05 * ss))
+    n = 9000
+    pos = np.random.default_rng(per_side + ntags).uniform(0, side, (n, 3)).astype(np.float32)
+    pos[: ntags - 1] = np.float32(0.3) + pos[: ntags - 1] / np.float32(side)  # one nearly full cell
+    p = O.setup_params(side, 10, n, float(CF.SIGMA_BIG), ss, ntags=(ntags, ntags))
+    pp = B.Parametros.from_buffer_copy(bytes(p))
+    assert pp.ncell_sml == per_side
+    nocup, cell = cells(pp, "s", dev(pos))
+    ref = O.cell_locate(p, "s", pos)
+    np.testing.assert_array_equal(host(nocup), ref[0])
+    np.testing.assert_array_equal(host(cell), ref[1])
+
+
 @pytest.mark.parametrize("nb,ns", [(1000, 1200), (8200, 9000)])
 def test_forces_of_a_drop_match_the_oracle(nb, ns):
     """A dense drop in an empty box: the lanes of a particle (32, then eight)
