@@ -30,6 +30,18 @@ enum : unsigned {
 __device__ __forceinline__ void set_status(unsigned *st, unsigned bits) {
     if (st) atomicOr(st, bits);
 }
+// Status of a call whose word lies in host memory, where an atomic costs 30 ns
+// and a million failing threads took 60 ms: the first thread with a bit, told
+// by a device word per bit that then holds the call's number, sets it there.
+struct CallStatus {
+    unsigned *word;  // host word
+    unsigned *seen;  // [32] device words
+    unsigned call;
+};
+__device__ __forceinline__ void set_status(const CallStatus &st, unsigned bit) {
+    unsigned *seen = st.seen + (__ffs(bit) - 1);
+    if (*(volatile unsigned *)seen != st.call && atomicExch(seen, st.call) != st.call) atomicOr(st.word, bit);
+}
 
 
 // ------------------------------------------------------------ packed pairs

@@ -50,7 +50,7 @@ struct CvHits {
     int bins;
     float *H;            // [3][n][bins] (zero), or null: the block adds to ata and atb
     double *ata, *atb;
-    unsigned *st;
+    CallStatus st;
 };
 // shared memory: tile [3][kCvTile] and masks [warps][kCvMasks][32] (later the
 // rows in FP64, [32][3 bins | 1]), bin sums [warps][32][3 bins | 1] (an odd row

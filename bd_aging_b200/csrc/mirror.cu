@@ -53,6 +53,7 @@ namespace {
 constexpr int kSlots = 32;
 struct SlotState {
     std::atomic_flag busy = ATOMIC_FLAG_INIT;
+    unsigned calls = 0;
 };
 struct DeviceSlots {
     HostWords *host = nullptr, *dev = nullptr;  // [kSlots] words, 128 bytes apart
@@ -110,6 +111,8 @@ CallSlot::CallSlot() {
     dev = d->dev + k * kWordStride;
     accum = d->accum + (size_t)k * kWorkAccum;
     counter = reinterpret_cast<unsigned *>(d->accum + (size_t)kSlots * kWorkAccum) + 64 * k;
+    seen = counter + 32;
+    call = ++d->slot[k].calls;
     host->status = 0;
 }
 CallSlot::~CallSlot() {
@@ -127,7 +130,7 @@ static int read_status(const CallSlot &w, cudaStream_t s) {
 // with the inverse side a double division narrowed to float, ==ncell clamp,
 // linear index i + n(j + n k), slot by atomic increment of nocup.
 __global__ void k_cell_bin(const float *__restrict__ rr, int n, float csi, int ncell, int ntags, int *nocup,
-                           int *cell_vec, unsigned *st) {
+                           int *cell_vec, const CallStatus st) {
     int m = blockIdx.x * blockDim.x + threadIdx.x;
     if (m >= n) return;
     float x = rr[3 * m], y = rr[3 * m + 1], z = rr[3 * m + 2];
@@ -200,7 +203,7 @@ template <bool SAME, int G, int W>
 __global__ void k_forces(const float *__restrict__ rr, float *ff, float *vir, float *pot,
                          const float *__restrict__ rr_o, const int *__restrict__ nocup,
                          const int *__restrict__ cell_vec, int n, int ncell, int ntags, int nrange, float csi,
-                         float sigma, float side, unsigned *st) {
+                         float sigma, float side, const CallStatus st) {
     const int m = (int)(((size_t)blockIdx.x * blockDim.x + threadIdx.x) / G), sub = threadIdx.x % G;
     if (m >= n) return;  // the lanes of a particle leave together
     const float side_inv = __fdiv_rn(1.0f, side);

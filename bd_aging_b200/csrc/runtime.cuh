@@ -35,13 +35,15 @@ struct CallSlot {
     HostWords *dev = nullptr;      // the same words as kernels see them
     double *accum = nullptr;       // kWorkAccum FP64 partial sums
     unsigned *counter = nullptr;   // finished blocks of a reduction, zero between calls
+    unsigned *seen = nullptr;      // status bits already passed on (CallStatus)
+    unsigned call = 0;             // number of this call among the slot's
     void *state = nullptr;
     CallSlot();                    // takes a free slot of the current device (waits when all are taken)
     ~CallSlot();
     CallSlot(const CallSlot &) = delete;
     CallSlot &operator=(const CallSlot &) = delete;
     bool ok() const { return host != nullptr; }  // false: allocation failed
-    unsigned *status() const { return &dev->status; }
+    CallStatus status() const { return {&dev->status, seen, call}; }
 };
 
 // Map the device status word to a BD_* code.  A non-finite position also

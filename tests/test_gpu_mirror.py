@@ -220,6 +220,32 @@ def test_cell_overflow_is_reported_not_written_out_of_bounds():
     assert (host(guard)[p.ncell_big ** 3 * 2:] == -7).all()
 
 
+def test_errors_of_many_particles_cost_no_more_than_one():
+    """Every particle of a call can fail (outside the box, non-finite, a cell too
+    full): each call reports its own error, a good one after it none, and a
+    million failing particles take milliseconds at most."""
+    import time
+    n = 1 << 20
+    side = CF.side_from_phi(n, n, 0.3)
+    p = B.setup_params(side, n, n, float(CF.SIGMA_BIG), float(CF.SIGMA_SML))
+    good = dev(np.random.default_rng(1).uniform(0, 0.9 * side, (n, 3)).astype(np.float32))
+    few = B.setup_params(side, 1000, 1000, float(CF.SIGMA_BIG), float(CF.SIGMA_SML))
+    for _ in range(2):
+        for rr, code in ((good + 3 * side, 3), (good * float("nan"), 9), (good * 0 + 0.2, 3)):
+            best = 1.0
+            for _ in range(3):
+                t = time.perf_counter()
+                with pytest.raises(B.BDError) as ei:
+                    cells(p, "b", rr)
+                best = min(best, time.perf_counter() - t)
+                assert ei.value.code == code
+            assert best < 0.015
+            cells(few, "b", good[:1000].clone())
+        with pytest.raises(B.BDError) as ei:  # outside the box, each in a cell of its own
+            cells(few, "b", good[:1000] + side)
+        assert ei.value.code in (3, 1)
+
+
 def test_invalid_species_rejected():
     p = B.setup_params(10.0, 10, 10, 1.5, 1.1)
     with pytest.raises(B.BDError):
