@@ -11,6 +11,7 @@
 #include <cmath>
 #include <cstring>
 #include <mutex>
+#include <new>
 #include <thread>
 #include <type_traits>
 #include <vector>
@@ -55,49 +56,51 @@ struct SlotState {
     std::atomic_flag busy = ATOMIC_FLAG_INIT;
     unsigned calls = 0;
 };
-struct DeviceSlots {
+struct ContextSlots {
     HostWords *host = nullptr, *dev = nullptr;  // [kSlots] words, 128 bytes apart
     double *accum = nullptr;                    // [kSlots][kWorkAccum], then the counters
     unsigned long long ctx = 0;                 // context the pointers belong to
     SlotState slot[kSlots];
+    ContextSlots *next = nullptr;
 };
 constexpr size_t kWordStride = 128 / sizeof(HostWords);
 static_assert(128 % sizeof(HostWords) == 0, "slots on their own lines");
 
-DeviceSlots *device_slots() {
+// The current context's slots, made on first use and never changed after: a
+// context's id is its own for the life of the process, so one that was destroyed
+// (its memory with it) leaves an entry that no call finds again.
+ContextSlots *context_slots() {
     static std::mutex mu;
-    static DeviceSlots all[64];
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return nullptr;
+    static ContextSlots *all = nullptr;
     const unsigned long long ctx = current_context_id();
     if (!ctx) return nullptr;
     std::lock_guard<std::mutex> lock(mu);
-    DeviceSlots &d = all[dev];
-    if (d.ctx != ctx) {  // first use, or the context was destroyed (its memory with it)
-        d.ctx = 0;
-        void *h = nullptr, *p = nullptr, *acc = nullptr;
-        if (cudaHostAlloc(&h, 128 * kSlots, cudaHostAllocMapped) != cudaSuccess) return nullptr;
-        const size_t sums = sizeof(double) * kWorkAccum * kSlots, bytes = sums + 256 * kSlots;
-        if (cudaHostGetDevicePointer(&p, h, 0) != cudaSuccess || cudaMalloc(&acc, bytes) != cudaSuccess) {
-            cudaFreeHost(h);
-            return nullptr;
-        }
-        if (cudaMemset(acc, 0, bytes) != cudaSuccess || cudaDeviceSynchronize() != cudaSuccess) {
-            cudaFreeHost(h);
-            cudaFree(acc);
-            return nullptr;
-        }
-        d.host = static_cast<HostWords *>(h);
-        d.dev = static_cast<HostWords *>(p);
-        d.accum = static_cast<double *>(acc);
-        d.ctx = ctx;
+    for (ContextSlots *d = all; d; d = d->next)
+        if (d->ctx == ctx) return d;
+    ContextSlots *d = new (std::nothrow) ContextSlots();
+    if (!d) return nullptr;
+    void *h = nullptr, *p = nullptr, *acc = nullptr;
+    const size_t sums = sizeof(double) * kWorkAccum * kSlots, bytes = sums + 256 * kSlots;
+    if (cudaHostAlloc(&h, 128 * kSlots, cudaHostAllocMapped) != cudaSuccess ||
+        cudaHostGetDevicePointer(&p, h, 0) != cudaSuccess || cudaMalloc(&acc, bytes) != cudaSuccess ||
+        cudaMemset(acc, 0, bytes) != cudaSuccess || cudaDeviceSynchronize() != cudaSuccess) {
+        if (h) cudaFreeHost(h);
+        if (acc) cudaFree(acc);
+        delete d;
+        return nullptr;
     }
-    return &d;
+    d->host = static_cast<HostWords *>(h);
+    d->dev = static_cast<HostWords *>(p);
+    d->accum = static_cast<double *>(acc);
+    d->ctx = ctx;
+    d->next = all;
+    all = d;
+    return d;
 }
 }  // namespace
 
 CallSlot::CallSlot() {
-    DeviceSlots *d = device_slots();
+    ContextSlots *d = context_slots();
     if (!d) return;
     int k = 0;
     while (d->slot[k].busy.test_and_set(std::memory_order_acquire)) {

@@ -24,7 +24,7 @@ unsigned long long current_context_id();
 // directly (no clear before and no copy after them; the stream's
 // synchronisation is all the call waits for), and the FP64 partial sums of the
 // fixed-order reductions.  The slots are allocated on first use in each
-// device's context (again after a device reset) and kept until exit.
+// context (again after a device reset) and kept until exit.
 constexpr int kWorkAccum = 2048;  // FP64 slots: one per reduction block
 struct HostWords {
     unsigned status;  // kStat* bits
@@ -38,7 +38,7 @@ struct CallSlot {
     unsigned *seen = nullptr;      // status bits already passed on (CallStatus)
     unsigned call = 0;             // number of this call among the slot's
     void *state = nullptr;
-    CallSlot();                    // takes a free slot of the current device (waits when all are taken)
+    CallSlot();                    // takes a free slot of the current context (waits when all are taken)
     ~CallSlot();
     CallSlot(const CallSlot &) = delete;
     CallSlot &operator=(const CallSlot &) = delete;

@@ -246,6 +246,45 @@ def test_errors_of_many_particles_cost_no_more_than_one():
         assert ei.value.code in (3, 1)
 
 
+def test_two_contexts_keep_their_own_workspaces():
+    """Calls that alternate between the primary context and another one of the
+    same device give the same sums and allocate once per context."""
+    n = 3000
+    raw, r0 = np.random.default_rng(2).normal(size=(2, n, 3)).astype(np.float32)
+    here = dev(raw), dev(r0)
+    want = B.msd(*here, n)
+    cu = C.CDLL("libcuda.so.1")
+
+    def ok(rc):
+        assert rc == 0, rc
+
+    primary, other, free, total = C.c_void_p(), C.c_void_p(), C.c_size_t(), C.c_size_t()
+    ok(cu.cuCtxGetCurrent(C.byref(primary)))
+    ok(cu.cuCtxCreate_v2(C.byref(other), C.c_uint(0), C.c_int(0)))
+    try:
+        there = []
+        for a in (raw, r0):
+            p = C.c_uint64()
+            ok(cu.cuMemAlloc_v2(C.byref(p), C.c_size_t(a.nbytes)))
+            ok(cu.cuMemcpyHtoD_v2(p, C.c_void_p(a.ctypes.data), C.c_size_t(a.nbytes)))
+            there.append(C.c_void_p(p.value))
+        out = np.zeros(1, np.float32)
+        level = []
+        for _ in range(40):
+            ok(cu.cuCtxSetCurrent(other))
+            assert B.lib().bd_msd(there[0], there[1], n, C.c_void_p(out.ctypes.data), None) == 0
+            assert out[0] == np.float32(want)
+            ok(cu.cuMemGetInfo_v2(C.byref(free), C.byref(total)))
+            level.append(free.value)
+            ok(cu.cuCtxSetCurrent(primary))
+            assert B.msd(*here, n) == want
+        assert level[2] - level[-1] < 4 << 20
+    finally:
+        ok(cu.cuCtxSetCurrent(primary))
+        ok(cu.cuCtxDestroy_v2(other))
+    assert B.msd(*here, n) == want
+
+
 def test_invalid_species_rejected():
     p = B.setup_params(10.0, 10, 10, 1.5, 1.1)
     with pytest.raises(B.BDError):
