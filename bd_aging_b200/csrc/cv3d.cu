@@ -380,7 +380,7 @@ int bd_cv3d_add_statistics(bd_cv3d *cv, const float *rr, const float *xx, int n,
     int warps = 16;
     while (warps > 4 && cv_hits_smem(bins, fused, warps) > kCvSmemMost) warps /= 2;
     const size_t sm = cv_hits_smem(bins, fused, warps);
-    CallSlot w;
+    CallSlot w(s);
     if (!w.ok()) return BD_ERR_NOMEM;
     if (!fused) BD_CUDA_TRY(cudaMemsetAsync(d_H, 0, sizeof(float) * 3 * (size_t)n * bins, s));
     k_cv_hits<<<div_up(n, kCvBlock), warps * 32, sm, s>>>({rr, xx, n, side, cv->range, bins, d_H, cv->d_ata, cv->d_atb,
@@ -395,7 +395,7 @@ int bd_cv3d_add_statistics(bd_cv3d *cv, const float *rr, const float *xx, int n,
         k_cv_reduce<<<div_up((long)sums, 64), 64, 0, s>>>(d_part, splits, (int)sums, cv->d_ata);
         BD_LAUNCH_CHECK();
     }
-    BD_CUDA_TRY(cudaStreamSynchronize(s));
+    BD_CUDA_TRY(w.wait());
     cv->samples++;
     return status_from_bits(*static_cast<volatile unsigned *>(&w.host->status));
 }

@@ -99,7 +99,7 @@ ContextSlots *context_slots() {
 }
 }  // namespace
 
-CallSlot::CallSlot() {
+CallSlot::CallSlot(cudaStream_t s) : stream(s) {
     ContextSlots *d = context_slots();
     if (!d) return;
     int k = 0;
@@ -118,13 +118,19 @@ CallSlot::CallSlot() {
     call = ++d->slot[k].calls;
     host->status = 0;
 }
+cudaError_t CallSlot::wait() {
+    waited = true;
+    return cudaStreamSynchronize(stream);
+}
 CallSlot::~CallSlot() {
-    if (state) static_cast<SlotState *>(state)->busy.clear(std::memory_order_release);
+    if (!state) return;
+    if (!waited) cudaStreamSynchronize(stream);
+    static_cast<SlotState *>(state)->busy.clear(std::memory_order_release);
 }
 
 // Waits for the call's kernels and maps their status.
-static int read_status(const CallSlot &w, cudaStream_t s) {
-    BD_CUDA_TRY(cudaStreamSynchronize(s));
+static int read_status(CallSlot &w) {
+    BD_CUDA_TRY(w.wait());
     return status_from_bits(*static_cast<volatile unsigned *>(&w.host->status));
 }
 
@@ -286,7 +292,7 @@ template <bool SAME>
 static int launch_forces(const float *rr, float *ff, float *vir, float *pot, const float *rr_o, const int *nocup,
                          const int *cell_vec, int n, int ncell, int ntags, int nrange, float csi, float sigma, float side,
                          cudaStream_t s) {
-    CallSlot w;
+    CallSlot w(s);
     if (!w.ok()) return BD_ERR_NOMEM;
     // lanes per particle.  A call's time (us) with 32, 8 and 1 lanes over 27
     // cells: 20, 24, 68 at 6000 particles; 30, 27, 74 at 16384; 64, 49, 76 at
@@ -298,7 +304,7 @@ static int launch_forces(const float *rr, float *ff, float *vir, float *pot, con
     kern<<<div_up((long)n * lanes, 128), 128, 0, s>>>(rr, ff, vir, pot, rr_o, nocup, cell_vec, n, ncell, ntags, nrange, csi,
                                                       sigma, side, w.status());
     BD_LAUNCH_CHECK();
-    return read_status(w, s);
+    return read_status(w);
 }
 
 // ------------------------------------------------------------ update
@@ -573,13 +579,13 @@ __global__ void __launch_bounds__(kDispThreads) k_disp_reduce(const float *__res
 }
 
 static int disp_reduce(int kind, const float *raw, const float *r0, int n, float q, double *out, cudaStream_t s) {
-    CallSlot w;
+    CallSlot w(s);
     if (!w.ok()) return BD_ERR_NOMEM;
     const int blocks = std::min(div_up(n, kDispThreads), kDispMaxBlocks);
     auto kern = kind == 0 ? k_disp_reduce<0> : k_disp_reduce<1>;
     kern<<<blocks, kDispThreads, 0, s>>>(raw, r0, n, q, w.accum, w.counter, &w.dev->value);
     BD_LAUNCH_CHECK();
-    BD_CUDA_TRY(cudaStreamSynchronize(s));
+    BD_CUDA_TRY(w.wait());
     *out = *static_cast<volatile double *>(&w.host->value);
     return BD_OK;
 }
@@ -716,7 +722,7 @@ int bd_cell_locate(char type, const float *rr, int *nocup, int *cell_vec, const 
     const float csi = (float)(1.0 / (b ? p->cell_side_big : p->cell_side_sml));
     const int nc3 = ncell * ncell * ncell;
     cudaStream_t s = as_stream(stream);
-    CallSlot w;
+    CallSlot w(s);
     if (!w.ok()) return BD_ERR_NOMEM;
     BD_CUDA_TRY(cudaMemsetAsync(nocup, 0, sizeof(int) * (size_t)nc3, s));
     // 16 or 32 lanes per cell (a call's time, us, lanes / a thread per cell: 16
@@ -735,7 +741,7 @@ int bd_cell_locate(char type, const float *rr, int *nocup, int *cell_vec, const 
     else if (by_lanes) k_cell_sort<32><<<div_up((long)nc3 * 32, 256), 256, 0, s>>>(nocup, cell_vec, nc3, ntags);
     else k_cell_sort_long<<<div_up(nc3, 256), 256, 0, s>>>(nocup, cell_vec, nc3, ntags);
     BD_LAUNCH_CHECK();
-    return read_status(w, s);
+    return read_status(w);
 }
 
 int bd_get_forces_same(char type, const float *rr, float *ff, float *vir, float *pot, const int *nocup,

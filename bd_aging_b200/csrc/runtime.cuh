@@ -38,8 +38,11 @@ struct CallSlot {
     unsigned *seen = nullptr;      // status bits already passed on (CallStatus)
     unsigned call = 0;             // number of this call among the slot's
     void *state = nullptr;
-    CallSlot();                    // takes a free slot of the current context (waits when all are taken)
-    ~CallSlot();
+    cudaStream_t stream;           // of the call's kernels
+    bool waited = false;
+    explicit CallSlot(cudaStream_t s);  // takes a free slot of the current context (waits when all are taken)
+    ~CallSlot();                   // gives it back, after the call's kernels also where the call failed
+    cudaError_t wait();            // for the call's kernels
     CallSlot(const CallSlot &) = delete;
     CallSlot &operator=(const CallSlot &) = delete;
     bool ok() const { return host != nullptr; }  // false: allocation failed

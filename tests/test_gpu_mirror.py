@@ -285,6 +285,30 @@ def test_two_contexts_keep_their_own_workspaces():
     assert B.msd(*here, n) == want
 
 
+def test_a_call_that_fails_waits_for_its_kernels():
+    """An error left pending by the caller makes a call return after its launch;
+    the workspace goes back only when that kernel is done, so the next call's
+    result is its own."""
+    import torch
+    n = 100_000_000
+    a = torch.ones((n, 3), device="cuda:0")
+    b = torch.zeros((n, 3), device="cuda:0")
+    want = B.msd(a[:1000], b[:1000], 1000)
+    B.msd(a, b, n)
+    torch.cuda.synchronize()
+    rt = C.CDLL("libcudart.so.12")
+    p = C.c_void_p()
+    assert rt.cudaMalloc(C.byref(p), C.c_size_t(1 << 60)) != 0
+    try:
+        with pytest.raises(B.BDError):
+            B.msd(a, b, n)  # about 0.4 ms of work
+        idle = torch.cuda.default_stream().query()
+    finally:
+        rt.cudaGetLastError()
+    assert idle
+    assert B.msd(a[:1000], b[:1000], 1000) == want
+
+
 def test_invalid_species_rejected():
     p = B.setup_params(10.0, 10, 10, 1.5, 1.1)
     with pytest.raises(B.BDError):
