@@ -200,7 +200,10 @@ __global__ void k_cell_sort_long(const int *nocup, int *cell_vec, int nc3, int n
 // position, which a thread per particle walks 27 or 125 times with 110 threads
 // on an SM (16384 particles).  A warp per particle walks it once or four times
 // and fills the chip; with more particles fewer lanes each, and so fewer
-// instructions, win (launch_forces).
+// instructions, win (launch_forces).  12 blocks an SM (40 registers): a thread
+// per particle over 1.5 million waits for memory, 719 us with 48 warps on an SM,
+// 799 with the 40 that 46 registers allow.
+constexpr int kForceThreads = 128;
 template <int G>  // the aligned group of G lanes that `lane` belongs to
 __host__ __device__ constexpr unsigned lanes_of_group(int lane) {
     return (unsigned)(((1ull << G) - 1ull) << (lane & ~(G - 1)));
@@ -209,7 +212,7 @@ static_assert(lanes_of_group<32>(5) == 0xffffffffu && lanes_of_group<8>(0) == 0x
                   lanes_of_group<8>(15) == 0xff00u && lanes_of_group<8>(31) == 0xff000000u,
               "a particle's lanes");
 template <bool SAME, int G, int W>
-__global__ void k_forces(const float *__restrict__ rr, float *ff, float *vir, float *pot,
+__global__ void __launch_bounds__(kForceThreads, 12) k_forces(const float *__restrict__ rr, float *ff, float *vir, float *pot,
                          const float *__restrict__ rr_o, const int *__restrict__ nocup,
                          const int *__restrict__ cell_vec, int n, int ncell, int ntags, int nrange, float csi,
                          float sigma, float side, const CallStatus st) {
@@ -230,19 +233,13 @@ __global__ void k_forces(const float *__restrict__ rr, float *ff, float *vir, fl
     }
     float fx = 0.f, fy = 0.f, fz = 0.f, v = 0.f, p = 0.f;
     if (G == 1) fx = ff[3 * (size_t)m], fy = ff[3 * (size_t)m + 1], fz = ff[3 * (size_t)m + 2], v = vir[m], p = pot[m];
-    const int w = W > 0 ? W : 2 * nrange + 1, cells = w * w * w, reach = W > 0 ? W / 2 : nrange;
+    const int w = W > 0 ? W : 2 * nrange + 1, reach = W > 0 ? W / 2 : nrange;
     auto wrap = [&](int k) {
         while (k < 0) k += ncell;
         while (k >= ncell) k -= ncell;
         return k;
     };
-    for (int t0 = sub; t0 < cells; t0 += G) {
-        // consecutive lanes take cells that follow one another in memory (x runs
-        // fastest there); a single thread keeps the reference's order of sums
-        const int slow = t0 / (w * w) - reach, fast = t0 % w - reach;
-        const int ip = wrap(ii + (G == 1 ? slow : fast)), jp = wrap(jj + t0 / w % w - reach),
-                  kp = wrap(kk + (G == 1 ? fast : slow));
-        int c = ip + ncell * (jp + ncell * kp);
+    auto visit = [&](int c) {
         int occ = min(nocup[c], ntags);
         const int *cv = cell_vec + (long)c * ntags;
 #pragma unroll 2
@@ -262,6 +259,19 @@ __global__ void k_forces(const float *__restrict__ rr, float *ff, float *vir, fl
                 v += o.vir;
             }
         }
+    };
+    if (G == 1) {  // the reference's order of sums
+        for (int di = -reach; di <= reach; di++) {
+            const int ip = wrap(ii + di);
+            for (int dj = -reach; dj <= reach; dj++) {
+                const int jp = wrap(jj + dj);
+                for (int dk = -reach; dk <= reach; dk++) visit(ip + ncell * (jp + ncell * wrap(kk + dk)));
+            }
+        }
+    } else {  // consecutive lanes take cells that follow one another in memory (x runs fastest)
+        for (int t0 = sub; t0 < w * w * w; t0 += G)
+            visit(wrap(ii + t0 % w - reach) +
+                  ncell * (wrap(jj + t0 / w % w - reach) + ncell * wrap(kk + t0 / (w * w) - reach)));
     }
     if (G > 1) {
         // this particle's lanes: they left together at m >= n, and the loop has not
@@ -297,11 +307,12 @@ static int launch_forces(const float *rr, float *ff, float *vir, float *pot, con
     // lanes per particle.  A call's time (us) with 32, 8 and 1 lanes over 27
     // cells: 20, 24, 68 at 6000 particles; 30, 27, 74 at 16384; 64, 49, 76 at
     // 60000; 255, 163, 159 at 300000; over 125 cells: 26, 41, 193 at 6000; 45,
-    // 46, 220 at 16384; 112, 106, 226 at 60000; 487, 402, 494 at 300000.
-    const int lanes = nrange > 1 ? (n <= 32768 ? 32 : 8) : n <= 8192 ? 32 : n <= 131072 ? 8 : 1;
+    // 46, 220 at 16384; 112, 106, 226 at 60000; 487, 402, 494 at 300000; with 8
+    // and 1 lanes 546, 585 at 500000; 950, 893 at 800000; 2125, 1985 at 1.5 million.
+    const int lanes = nrange > 1 ? (n <= 32768 ? 32 : n <= 655360 ? 8 : 1) : n <= 8192 ? 32 : n <= 131072 ? 8 : 1;
     auto kern = lanes == 32 ? forces_kernel<SAME, 32>(nrange) : lanes == 8 ? forces_kernel<SAME, 8>(nrange)
                                                                           : forces_kernel<SAME, 1>(nrange);
-    kern<<<div_up((long)n * lanes, 128), 128, 0, s>>>(rr, ff, vir, pot, rr_o, nocup, cell_vec, n, ncell, ntags, nrange, csi,
+    kern<<<div_up((long)n * lanes, kForceThreads), kForceThreads, 0, s>>>(rr, ff, vir, pot, rr_o, nocup, cell_vec, n, ncell, ntags, nrange, csi,
                                                       sigma, side, w.status());
     BD_LAUNCH_CHECK();
     return read_status(w);

@@ -93,6 +93,19 @@ def test_cell_sort_and_force_paths_match_the_oracle(nb, ns, ntags):
         np.testing.assert_allclose(v, ref[k], rtol=2e-5, atol=2e-5 * np.abs(ref[k]).max(), err_msg=k)
 
 
+def test_a_thread_per_particle_over_125_cells_matches_the_oracle():
+    """The first size at which the calls over 125 cells take a thread per particle."""
+    nb, ns = 655361, 4000
+    side = CF.side_from_phi(nb, ns, 0.3)
+    pos = CF.lattice_config(nb, ns, side, 29)
+    p = O.setup_params(side, nb, ns, float(CF.SIGMA_BIG), float(CF.SIGMA_SML), ntags=(16, 16))
+    pp = B.Parametros.from_buffer_copy(bytes(p))
+    assert pp.nrange_bs == 2
+    out, ref = forces_four_calls(pp, pos[:nb], pos[nb:]), O.ref_forces(p, pos[:nb].copy(), pos[nb:].copy())
+    for k, v in out.items():
+        np.testing.assert_allclose(v, ref[k], rtol=2e-5, atol=2e-5 * np.abs(ref[k]).max(), err_msg=k)
+
+
 @pytest.mark.parametrize("per_side,ntags", [(40, 16), (41, 16), (32, 17), (33, 17), (32, 32), (33, 32)])
 def test_cell_lists_on_both_sides_of_the_lane_limit(per_side, ntags):
     """2^20 lanes in all (16 per cell, or 32 with more slots): cells sorted by
