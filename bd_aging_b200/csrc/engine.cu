@@ -322,8 +322,11 @@ int launch_list_grid(bd_engine *e, int cur, int nsteps) {
     BD_LAUNCH_CHECK();
     return BD_OK;
 }
-// launches of a whole batch of steps
-bool list_batched(const bd_engine *e) { return list_per_replica(e) || list_cluster(e) || list_grid(e); }
+// launches of a whole batch of `nsteps` steps
+bool list_batched(const bd_engine *e, int nsteps) {
+    if (e->lvar == 0 && e->lrep_default && nsteps <= e->lrep_short) return false;
+    return list_per_replica(e) || list_cluster(e) || list_grid(e);
+}
 int list_batch_steps(bd_engine *e, int cur, int nsteps) {
     if (nsteps > e->graph_steps) return BD_ERR_ARG;  // the amplitude table holds one batch
     if (list_cluster(e)) return launch_list_cluster(e, cur, nsteps);
@@ -384,7 +387,7 @@ int direct_steps(bd_engine *e, int k) {
     if (e->list) {
         if (k > e->graph_steps) return BD_ERR_ARG;  // the amplitude table holds one batch
         if (int rc = list_amplitudes(e, k)) return rc;
-        if (list_batched(e)) {
+        if (list_batched(e, k)) {
             if (int rc = list_batch_steps(e, e->cur, k)) return rc;
         } else {
             for (int i = 0; i < k; i++) {
@@ -417,7 +420,7 @@ int build_graph(bd_engine *e) {
     int rc = BD_OK;
     if (e->list) {
         rc = list_amplitudes(e, e->graph_steps);
-        if (rc == BD_OK && list_batched(e)) rc = list_batch_steps(e, e->cur, e->graph_steps);
+        if (rc == BD_OK && list_batched(e, e->graph_steps)) rc = list_batch_steps(e, e->cur, e->graph_steps);
         else
             for (int j = 0; j < e->graph_steps && rc == BD_OK; j++) rc = list_step(e, e->cur + j, j);
     } else if (e->mode == BD_MODE_PERSISTENT) {
@@ -629,6 +632,13 @@ void choose_resident(bd_engine *e) {
     const double replica_us = replica_step_us(e, sms);
     const bool cluster = cluster_us <= std::min(other, replica_us);
     e->lrep_default = !cluster && replica_us < other;
+    // A short launch is as long as the slowest replica's rebuild, which the
+    // others' steps hide in a long one and the per-step kernels spread over the
+    // chip.  us a call of 1, 2, 3, 5 steps, per step / per replica: 256 x 1000 69,
+    // 129, 190, 301 / 77, 103, 116, 137; 200 x 2000 80, 138, 197, 313 / 119, 148,
+    // 176, 216; 250 x 4000 110, 200, 294, 473 / 217, 287, 333, 414; 148 x 6000
+    // 96, 174, 252, 411 / 232, 310, 359, 432.
+    e->lrep_short = std::max(1, nmax / 1000);
     if (!cluster) e->lcl_ctas = 0;
     if (cluster || e->lrep_default) e->lgr_blocks = 0;
 }
@@ -1034,7 +1044,7 @@ namespace {
 // Steps issued directly (no graph): one persistent launch, or k plain launches.
 int run_direct(bd_engine *e, int k) {
     if (k <= 0) return BD_OK;
-    if (e->mode == BD_MODE_PERSISTENT || list_batched(e)) return direct_steps(e, k);
+    if (e->mode == BD_MODE_PERSISTENT || list_batched(e, k)) return direct_steps(e, k);
     for (int i = 0; i < k; i++) {
         int rc = direct_steps(e, 1);
         if (rc) return rc;

@@ -85,6 +85,7 @@ struct bd_engine {
     int *d_rep_order = nullptr;     // per-replica launch (variants 3-5): replica of each block
     bool lrep_resident = false;     // variant 5: positions resident in shared memory
     bool lrep_default = false;      // variant 0 takes variant 5's launch
+    int lrep_short = 0;             //   but for launches of up to this many steps
     size_t lrep_smem = 0;           // variant 5: dynamic shared memory (resident positions, in-block rebuilds)
     // variant 0 in clusters (0 CTAs: the per-step kernels): CTAs per replica, the particles each owns at
     // most, their shared memory, the largest replica's particles and cells

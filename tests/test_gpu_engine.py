@@ -370,6 +370,30 @@ def test_clusters_in_several_rounds_match_the_per_step_kernels(sizes):
         np.testing.assert_array_equal(a, b)
 
 
+def test_short_runs_between_block_per_replica_launches():
+    """Batches whose default is a block per replica take runs of up to one step
+    per 1000 particles of the largest replica step by step: any mix of run
+    lengths gives the bits, rebuilds and lists of either launch alone."""
+    systems, poss = [], []
+    for k in range(76):
+        s, p = system(1000 + k, 1101, 0.4, 51 + k, T0=3.0, force_cap=100.0)
+        systems.append(s)
+        poss.append(p)
+    pos = np.concatenate(poss)
+    out = []
+    for v in (1, 5, None):
+        e = B.Engine(list(systems), list_variant=v)
+        e.set_positions(pos)
+        for k in (1, 2, 3, 1, 99, 98, 2, 4, 1):
+            e.run(k)
+        info = e.info()
+        out.append((*e.get_positions(), *e.census(), np.array([info.list_builds, info.list_rebuild_steps])))
+        e.close()
+    for got in out[1:]:
+        for a, b in zip(out[0], got):
+            np.testing.assert_array_equal(a, b)
+
+
 def test_first_step_temperature_carried_over():
     """A replica given T_first takes its first update at that temperature and
     then follows its protocol (the drop-in executable uses this for
