@@ -302,7 +302,7 @@ int launch_list_cluster(bd_engine *e, int cur, int nsteps) {
 }
 // Variant 0 of mid-size batches: the whole grid runs `nsteps` steps.
 bool list_grid(const bd_engine *e) { return e->list && e->lvar == 0 && e->lgr_blocks > 0 && e->rng == BD_RNG_PHILOX; }
-int launch_list_grid(bd_engine *e, int cur, int nsteps) {
+int launch_list_grid(bd_engine *e, int cur, int nsteps, GridWait limit = GridWait()) {
     const ListPersist lp{{e->lpos[0], e->lpos[1]}, cur & 1, e->cnt[0], e->pos[0], e->cap, e->nbr, e->nnb,
                          e->pbuild, e->d_rep_order, e->d_builds, e->d_step_rebuilt, 0, 0};
     cudaLaunchConfig_t cfg;
@@ -317,7 +317,7 @@ int launch_list_grid(bd_engine *e, int cur, int nsteps) {
     cfg.attrs = at;
     cfg.numAttrs = 1;
     BD_CUDA_TRY(cudaLaunchKernelEx(&cfg, grid_kernel(e), make_largs(e, cur), lp, (const long long *)e->d_ni, nsteps,
-                                   grid_word(e)));
+                                   grid_word(e), limit));
     k_list_replica_done<<<1, 256, 0, e->stream>>>(e->lflag, e->R, e->d_step_rebuilt, nsteps, e->d_builds, grid_word(e));
     BD_LAUNCH_CHECK();
     return BD_OK;
@@ -1228,6 +1228,21 @@ int bd_engine_run(bd_engine *e, long long nsteps) {
             nsteps = 0;
         }
     }
+    return engine_status(e);
+}
+
+// For the test of the grid barrier's limit: one step whose first barrier waits
+// `polls` polls for an arrival that no block makes (BD_ERR_TIMEOUT; the state is
+// void until the next bd_engine_set_positions).  BD_ERR_ARG where the engine
+// does not take the whole-grid launch.
+int bd_engine_grid_barrier_timeout(bd_engine *e, unsigned polls) {
+    if (!e || !polls || polls > 1u << 21 || !list_grid(e)) return BD_ERR_ARG;
+    if (!e->loaded) return BD_ERR_STATE;
+    if (int rc = list_amplitudes(e, 1)) return rc;
+    GridWait limit;
+    limit.polls = polls;
+    limit.extra = 1;
+    if (int rc = launch_list_grid(e, e->cur, 1, limit)) return rc;
     return engine_status(e);
 }
 

@@ -1,6 +1,8 @@
 """GPU parity of the batched replica engine against the oracle: neighbour
 sets (exact), one step with injected noise, observables, g(r) counts (exact),
 batched == plain bit identity, error paths."""
+import ctypes as C
+
 import numpy as np
 import pytest
 
@@ -392,6 +394,32 @@ def test_short_runs_between_block_per_replica_launches():
     for got in out[1:]:
         for a, b in zip(out[0], got):
             np.testing.assert_array_equal(a, b)
+
+
+@pytest.mark.parametrize("n", [(1500, 1600), (20000, 20000)])
+def test_grid_barrier_gives_up_with_a_status(n):
+    """With helper threads and without: a barrier that waits for an arrival that
+    does not come ends the launch and the call returns BD_ERR_TIMEOUT; loading
+    positions starts the engine anew, with the usual bits."""
+    s, pos = system(*n, 0.45, 6, T0=1.0, force_cap=100.0)
+    out = []
+    for give_up in (False, True):
+        e = B.Engine([s])
+        e.set_positions(pos)
+        if give_up:
+            assert B.lib().bd_engine_grid_barrier_timeout(e._h, C.c_uint(0)) == B.BD_ERR_ARG
+            assert B.lib().bd_engine_grid_barrier_timeout(e._h, C.c_uint(2000)) == 6
+            e.set_positions(pos)
+        e.run(103)
+        out.append((*e.get_positions(), *e.census()))
+        e.close()
+    for a, b in zip(*out):
+        np.testing.assert_array_equal(a, b)
+    small, p = system(300, 300, 0.45, 6)
+    e = B.Engine([small])  # a cluster launch
+    e.set_positions(p)
+    assert B.lib().bd_engine_grid_barrier_timeout(e._h, C.c_uint(2000)) == B.BD_ERR_ARG
+    e.close()
 
 
 def test_first_step_temperature_carried_over():
