@@ -724,11 +724,14 @@ int bd_surrogate_train(bd_surrogate *s, int steps, float lr, float *last_loss) {
     return rc;
 }
 
-// Gradients of the mean loss over one batch (x [batch][n_in], y
-// [batch][n_out], host) without an update, flat like bd_surrogate_get_params;
-// loss = (1 / (batch n_out)) sum w (y_pred - y)^2.
-int bd_surrogate_gradients(bd_surrogate *s, const float *x, const float *y, float *grad, float *loss) {
-    if (!s || !x || !y || !grad) return BD_ERR_ARG;
+}  // extern "C"
+
+namespace {
+
+// the work of bd_surrogate_gradients and bd_surrogate_predict, which wait for
+// the stream also where it fails: copies from and to the caller's arrays may be
+// in flight
+int gradients_of(bd_surrogate *s, const float *x, const float *y, float *grad, double *sum) {
     const int B = s->batch;
     int rc = io_rows(s, B);
     if (rc) return rc;
@@ -741,16 +744,9 @@ int bd_surrogate_gradients(bd_surrogate *s, const float *x, const float *y, floa
     k_bias_grads<<<div_up(a.first[s->L], kBiasRows), kBiasRows * 32, 0, s->stream>>>(a);
     BD_LAUNCH_CHECK();
     rc = flatten(s, true, grad);
-    if (rc) return rc;
-    double sum = 0;
-    rc = sg_finish(s, &sum);
-    if (loss) *loss = (float)(sum / ((double)B * s->n_out));
-    return rc;
+    return rc ? rc : sg_finish(s, sum);
 }
-
-// Network outputs for n inputs (host x [n][n_in] -> y [n][n_out]).
-int bd_surrogate_predict(bd_surrogate *s, const float *x, int n, float *y) {
-    if (!s || !x || !y || n < 0) return BD_ERR_ARG;
+int predict_rows(bd_surrogate *s, const float *x, int n, float *y) {
     int rc = io_rows(s, std::min(n, kPredictRows));
     for (int r0 = 0; r0 < n && !rc; r0 += kPredictRows) {
         const int cnt = std::min(kPredictRows, n - r0);
@@ -761,8 +757,31 @@ int bd_surrogate_predict(bd_surrogate *s, const float *x, int n, float *y) {
             BD_CUDA_TRY(cudaMemcpyAsync(y + (size_t)r0 * s->n_out, s->py, (size_t)cnt * s->n_out * 4,
                                         cudaMemcpyDeviceToHost, s->stream));
     }
-    if (rc) return rc;
-    return sg_finish(s, nullptr);
+    return rc ? rc : sg_finish(s, nullptr);
+}
+
+}  // namespace
+
+extern "C" {
+
+// Gradients of the mean loss over one batch (x [batch][n_in], y
+// [batch][n_out], host) without an update, flat like bd_surrogate_get_params;
+// loss = (1 / (batch n_out)) sum w (y_pred - y)^2.
+int bd_surrogate_gradients(bd_surrogate *s, const float *x, const float *y, float *grad, float *loss) {
+    if (!s || !x || !y || !grad) return BD_ERR_ARG;
+    double sum = 0;
+    const int rc = gradients_of(s, x, y, grad, &sum);
+    if (rc) cudaStreamSynchronize(s->stream);
+    if (loss && (!rc || rc == BD_ERR_TIMEOUT)) *loss = (float)(sum / ((double)s->batch * s->n_out));
+    return rc;
+}
+
+// Network outputs for n inputs (host x [n][n_in] -> y [n][n_out]).
+int bd_surrogate_predict(bd_surrogate *s, const float *x, int n, float *y) {
+    if (!s || !x || !y || n < 0) return BD_ERR_ARG;
+    const int rc = predict_rows(s, x, n, y);
+    if (rc) cudaStreamSynchronize(s->stream);
+    return rc;
 }
 
 // Plain GEMM through the same kernel, for tests and measurement:

@@ -151,3 +151,31 @@ def test_network_shapes_match_oracle(width, depth, batch, n_in, n_out):
     # |g| >> eps there; the FP32 parameters (below 8 in size) round the sum
     assert np.all(np.abs(moved + 1e-3 * np.sign(go))[big] <= 1e-3 * 1e-3 + 2.0 ** -21)
     s.close()
+
+
+def test_a_call_that_fails_waits_for_its_copies():
+    """An error left pending by the caller makes predict and gradients return
+    after their first launch; the caller's arrays are no longer read or written
+    then, and the next call is unharmed."""
+    import ctypes as C
+
+    import torch
+    n, b = 32768, 32768
+    net = B.Surrogate(width=256, depth=8, batch=b, seed=4)
+    g = np.random.default_rng(1)
+    x, y = g.uniform(-1, 1, (n, 5)).astype(np.float32), g.normal(size=(n, 34)).astype(np.float32)
+    want = net.predict(x)
+    net.gradients(x, y)
+    stream = torch.cuda.ExternalStream(net.stream_handle())
+    rt = C.CDLL("libcudart.so.12")
+    p = C.c_void_p()
+    for call in (lambda: net.predict(x), lambda: net.gradients(x, y)):
+        assert rt.cudaMalloc(C.byref(p), C.c_size_t(1 << 60)) != 0
+        try:
+            with pytest.raises(B.BDError):
+                call()
+            idle = stream.query()
+        finally:
+            rt.cudaGetLastError()
+        assert idle
+    np.testing.assert_array_equal(net.predict(x), want)
