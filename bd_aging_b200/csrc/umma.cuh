@@ -234,6 +234,9 @@ __global__ void __launch_bounds__(kThreads, 1) k_umma_gemm(const __grid_constant
             for (int kk = 0; kk < kBK / 16; kk++)  // 16 bf16 = 32 bytes = 2 descriptor units
                 umma_bf16(lead, tmem, ad + 2 * kk, bd + 2 * kk, idesc, (c | kk) ? 1u : 0u);
         }
+        // after a load that did not come, this CTA's other copies before its memory goes away
+        if (!ok)
+            for (int c = 0; c < nk; c++) mbar_wait(&full[c], 0, t.err, 4u);
         umma_commit(lead, done);  // arrives once every issued MMA has completed
     }
     __syncwarp();
