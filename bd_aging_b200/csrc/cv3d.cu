@@ -6,9 +6,10 @@
 // sum, Contracting_Vector3D.cu:101-105), then per Cartesian component c the
 // normal equations A^T A_c += h_c h_c^T and A^T b_c += h_c f_c.
 //   k_cv_hits: 32 particles per block, a lane each; its warps share the
-//     partners.  Up to kCvFused bins the block adds its rows' products H_c^T H_c
-//     and H_c^T f_c (FP64; the reference accumulates in float) to the sums;
-//   with more bins H[c][m][b] (float, like the reference's hit_vec) goes to
+//     partners.  Up to kCvFused bins, with enough particles for them, the block
+//     adds its rows' products H_c^T H_c and H_c^T f_c (FP64; the reference
+//     accumulates in float) to the sums;
+//   otherwise H[c][m][b] (float, like the reference's hit_vec) goes to
 //     memory, k_cv_normal multiplies it, tiled over the bins and split over m
 //     so that every SM has a block, and k_cv_reduce adds the splits in order.
 // k_cv_hits is bound by issue: all but about 2% of the pairs are out of range.
@@ -18,8 +19,8 @@
 // mask per 32 (no branch in that loop), and the reference's arithmetic decides
 // on those, eight masks at a time.  Where that test could miss a pair (range
 // beyond 0.49 side, a coordinate far outside the box) every pair is noted.  A
-// lane adds to a row of its own (a copy per warp, summed
-// at the end), so it needs no atomics; with H in memory it adds there.
+// lane adds to a row of its own (a copy per warp, summed at the end), so it
+// needs no atomics; with H in memory it adds there.
 // Measured, 4000 particles, 24 bins to 3.5: 38 us a configuration (84 + 259 for
 // a warp per particle with a double-precision floor per component of every
 // pair, and a product kernel of 12 blocks).
@@ -41,7 +42,14 @@ constexpr int kCvNeighsMax = 10000;  // Contracting_Vector3D.cuh:36
 constexpr int kCvBlock = 32;   // particles per block
 constexpr int kCvTile = 1024;  // partners staged at a time
 constexpr int kCvMasks = 8;    // masks of 32 partners a lane notes before they are settled
-constexpr int kCvFused = 64;
+// Products in k_cv_hits: us a call, in it / by k_cv_normal from H in memory, at
+// 60 particles 30 / 32 with 24 bins, 38 / 32 with 40, 52 / 32 with 60; at 1000
+// 26 / 33, 36 / 37, 50 / 42; at 4000 38 / 57, 50 (34 bins) / 71, 68 / 89.  A block's products
+// take 3 bins^2 sums of 32 terms however few blocks there are, so that with
+// more than 24 bins some 40 particles a bin have to be there; beyond 60 bins its
+// 8 warps' rows don't fit (4 warps: 79 / 34 at 300 particles, 105 / 88 at 4000).
+constexpr int kCvFused = 60;
+inline bool cv_fused(int n, int bins) { return bins <= kCvFused && n >= 40 * (bins - 24); }
 constexpr size_t kCvSmemMost = (size_t)227 * 1024 - 256;  // beside the static shared memory
 struct CvHits {
     const float *rr, *xx;
@@ -359,7 +367,7 @@ int bd_cv3d_add_statistics(bd_cv3d *cv, const float *rr, const float *xx, int n,
     if (!cv || n <= 0 || !rr || !xx) return BD_ERR_ARG;  // DEBUG_ASSERT(nparticles > 0) in the reference
     cudaStream_t s = as_stream(stream);
     const int bins = cv->bins, tiles = div_up(bins, 16);
-    const bool fused = bins <= kCvFused;
+    const bool fused = cv_fused(n, bins);
     // splits over the particles until about two blocks per SM, each with a tile
     // of rows at least
     const int splits = std::max(1, std::min(div_up(n, kCvRows), 148 * 2 / (3 * tiles * tiles)));
@@ -376,9 +384,8 @@ int bd_cv3d_add_statistics(bd_cv3d *cv, const float *rr, const float *xx, int n,
     double *d_part = static_cast<double *>(cv->d_work);
     float *d_H = fused ? nullptr : reinterpret_cast<float *>(static_cast<unsigned char *>(cv->d_work) + part);
     // 16 warps a block where their copies of the rows fit beside the static
-    // shared memory (33 bins), else 8 (60 bins), else 4 (148 KB at kCvFused bins)
-    int warps = 16;
-    while (warps > 4 && cv_hits_smem(bins, fused, warps) > kCvSmemMost) warps /= 2;
+    // shared memory (33 bins), else 8 (60 bins)
+    const int warps = cv_hits_smem(bins, fused, 16) <= kCvSmemMost ? 16 : 8;
     const size_t sm = cv_hits_smem(bins, fused, warps);
     CallSlot w(s);
     if (!w.ok()) return BD_ERR_NOMEM;

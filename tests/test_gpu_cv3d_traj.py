@@ -102,6 +102,13 @@ def test_cv3d_block_widths(n, bins):
     assert np.linalg.norm(got - ref) <= bound
 
 
+@pytest.mark.parametrize("n,bins", [(399, 34), (400, 34), (1439, 60), (1440, 60), (40, 25), (39, 25), (30, 60)])
+def test_cv3d_product_rule(n, bins):
+    """Particle counts on both sides of where the products move into the pair
+    kernel (40 a bin beyond 24 bins), with the bound of the edge cases above."""
+    test_cv3d_block_widths(n, bins)
+
+
 def test_cv3d_state_errors_replace_reference_throws():
     cv = B.Contracting_Vector3D(8, 2.0)
     with pytest.raises(B.BDError) as e1:
