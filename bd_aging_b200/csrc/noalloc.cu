@@ -1,7 +1,7 @@
 // noalloc.cu -- F_s(q) reduction that allocates nothing on the device.
 //
-// bd_fself_isotropic (mirror.cu) keeps its FP64 partial sums in a per-device
-// workspace that is cudaMalloc'd on first use.  Some callers cannot allocate
+// bd_fself_isotropic (mirror.cu) keeps its FP64 partial sums in a workspace of
+// its context that is cudaMalloc'd on first use.  Some callers cannot allocate
 // device memory at the moment they sample F_s: real-time sampling loops whose
 // rules forbid allocation after start-up, and host programs whose device
 // memory is fully reserved up front by another allocator (a pool that owns

@@ -17,7 +17,7 @@
  *     (big particles first, main.cu:377-394).
  *
  * All functions are thread-compatible (no hidden global state apart from
- * per-device kernel attributes and a fixed set of per-device workspaces, one
+ * per-device kernel attributes and a fixed set of workspaces of each context, one
  * held by each synchronous call at a time); handles are not shared across
  * threads.
  */
