@@ -38,8 +38,9 @@
 // Warps: 16 for the epilogues, one that issues the MMAs, one that loads.
 // Every mbarrier wait is bounded: on expiry the error flag is recorded, the
 // remaining MMAs, loads and epilogues are skipped while every barrier is still
-// passed, and where the MMA warp gave up the loading warp waits (bounded) for
-// its own copies before the CTA ends.
+// passed, and the loading warp waits (bounded) for its own copies, which nobody
+// else does where the MMA warp gave up (always, in its own time: a word that
+// told it to, read after the block's last barrier, took 1.2 us of a step).
 #pragma once
 #include "umma.cuh"
 
@@ -195,7 +196,6 @@ __global__ void __launch_bounds__(kChainThreads, 1)
     uint64_t *bar_d = empty + kChainStages;   // [2]: MMAs of tile 0, 1 of the current GEMM completed
     uint64_t *bar_e = bar_d + 2;              // [2]: columns 0 .. 127, 128 .. 255 of the next operand written
     uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(bar_e + 2);
-    uint32_t *gave_up = tmem_slot + 1;        // the MMA warp has: copies may be in flight
     __shared__ float red[kChainWarps];
     __shared__ int s_src[kChainRows];         // data row of each row, -1: none
 
@@ -209,7 +209,6 @@ __global__ void __launch_bounds__(kChainThreads, 1)
     const uint32_t tmem_cols = n_keep == 0 ? 64u : n_keep == 1 ? 128u : n_keep <= 3 ? 256u : 512u;
 
     if (tid == 0) {
-        *gave_up = 0;
         for (int i = 0; i < 2 * kChainStages + 2; i++) mbar_init(&full[i], 1);
         mbar_init(&bar_e[0], kChainWarps);
         mbar_init(&bar_e[1], kChainWarps);
@@ -232,7 +231,6 @@ __global__ void __launch_bounds__(kChainThreads, 1)
     const uint32_t tmem = *tmem_slot;
 
     float loss = 0.f;
-    int issued = 0;  // loads of the loading warp
     if (warp == kChainWarps + 1) {  // the loading warp
         const uint32_t lead = elect_one();
         int idx = 0;
@@ -254,7 +252,9 @@ __global__ void __launch_bounds__(kChainThreads, 1)
                 tma_load_2d(lead, smem_u32(sW + s * kChainStage), map, smem_u32(&full[s]), k * kBK, t * kBM);
             }
         }
-        issued = idx;
+        // the CTA's copies, before its memory goes away
+        for (int i = max(0, idx - kChainStages); i < idx; i++)
+            mbar_wait(&full[i % kChainStages], (uint32_t)((i / kChainStages) & 1), g.err, 4u);
     } else if (warp == kChainWarps) {  // the MMA warp
         const uint32_t lead = elect_one(), idesc = umma_idesc(kChainRows);
         int idx = 0;
@@ -293,7 +293,6 @@ __global__ void __launch_bounds__(kChainThreads, 1)
                 umma_commit(lead, &bar_d[t]);
             }
         }
-        if (!ok && lead) *gave_up = 1;
     } else {  // the epilogue warps
         const int quad = warp & 3, group = warp >> 2;
         const uint32_t quad_row = (uint32_t)(quad * 32) << 16;
@@ -412,10 +411,6 @@ __global__ void __launch_bounds__(kChainThreads, 1)
     __syncwarp();
     tc_fence_before();
     __syncthreads();
-    // otherwise the MMAs have waited for every load
-    if (warp == kChainWarps + 1 && *gave_up)
-        for (int i = max(0, issued - kChainStages); i < issued; i++)
-            mbar_wait(&full[i % kChainStages], (uint32_t)((i / kChainStages) & 1), g.err, 4u);
     if (train && tid == 0) {
         float t = 0.f;
 #pragma unroll
