@@ -302,7 +302,7 @@ int launch_list_cluster(bd_engine *e, int cur, int nsteps) {
 }
 // Variant 0 of mid-size batches: the whole grid runs `nsteps` steps.
 bool list_grid(const bd_engine *e) { return e->list && e->lvar == 0 && e->lgr_blocks > 0 && e->rng == BD_RNG_PHILOX; }
-int launch_list_grid(bd_engine *e, int cur, int nsteps, GridWait limit = GridWait()) {
+int launch_list_grid(bd_engine *e, int cur, int nsteps) {
     const ListPersist lp{{e->lpos[0], e->lpos[1]}, cur & 1, e->cnt[0], e->pos[0], e->cap, e->nbr, e->nnb,
                          e->pbuild, e->d_rep_order, e->d_builds, e->d_step_rebuilt, 0, 0};
     cudaLaunchConfig_t cfg;
@@ -317,7 +317,7 @@ int launch_list_grid(bd_engine *e, int cur, int nsteps, GridWait limit = GridWai
     cfg.attrs = at;
     cfg.numAttrs = 1;
     BD_CUDA_TRY(cudaLaunchKernelEx(&cfg, grid_kernel(e), make_largs(e, cur), lp, (const long long *)e->d_ni, nsteps,
-                                   grid_word(e), limit));
+                                   grid_word(e)));
     k_list_replica_done<<<1, 256, 0, e->stream>>>(e->lflag, e->R, e->d_step_rebuilt, nsteps, e->d_builds, grid_word(e));
     BD_LAUNCH_CHECK();
     return BD_OK;
@@ -1231,18 +1231,19 @@ int bd_engine_run(bd_engine *e, long long nsteps) {
     return engine_status(e);
 }
 
-// For the test of the grid barrier's limit: one step whose first barrier waits
-// `polls` polls for an arrival that no block makes (BD_ERR_TIMEOUT; the state is
-// void until the next bd_engine_set_positions).  BD_ERR_ARG where the engine
-// does not take the whole-grid launch.
-int bd_engine_grid_barrier_timeout(bd_engine *e, unsigned polls) {
-    if (!e || !polls || polls > 1u << 21 || !list_grid(e)) return BD_ERR_ARG;
+// For the test of the grid barrier's limit: one step whose first barrier counts
+// its arrivals from -missing, as if that many blocks did not come, and so waits
+// until its limit (BD_ERR_TIMEOUT after a second or so; the state is void until
+// the next bd_engine_set_positions).  BD_ERR_ARG where the engine does not take
+// the whole-grid launch.
+int bd_engine_grid_barrier_timeout(bd_engine *e, unsigned missing) {
+    if (!e || !missing || missing > 1u << 21 || !list_grid(e)) return BD_ERR_ARG;
     if (!e->loaded) return BD_ERR_STATE;
     if (int rc = list_amplitudes(e, 1)) return rc;
-    GridWait limit;
-    limit.polls = polls;
-    limit.extra = 1;
-    if (int rc = launch_list_grid(e, e->cur, 1, limit)) return rc;
+    const unsigned long long first = 0u - missing;  // the high half, the askers, stays zero
+    BD_CUDA_TRY(cudaMemcpyAsync(grid_word(e), &first, sizeof(first), cudaMemcpyHostToDevice, e->stream));
+    BD_CUDA_TRY(cudaStreamSynchronize(e->stream));
+    if (int rc = launch_list_grid(e, e->cur, 1)) return rc;
     return engine_status(e);
 }
 

@@ -27,11 +27,9 @@
 namespace bd {
 
 constexpr int kGridMaxOwners = 512;            // particles per block; threads per block (128 registers each)
-// polls of a barrier before it gives up (a second or so), and arrivals it waits
-// for beyond the grid's (none, but in the test of giving up)
-struct GridWait {
-    unsigned polls = 1u << 21, extra = 0;
-};
+// polls of a barrier (a second or so).  A constant: as a launch argument it made
+// 192 steps of 4000 particles 587 us instead of 567
+constexpr unsigned kGridSpinLimit = 1u << 21;
 
 __host__ __device__ inline size_t grid_smem_bytes(int owners) { return (size_t)(kMaxNbr * 4 + 24) * owners; }
 
@@ -61,9 +59,8 @@ struct ListGrid {  // lists in shared memory, positions in global memory; entrie
 // word and waits there, so a slow block reads exactly this barrier's askers.
 struct GridBarrier {
     unsigned long long *word;
-    GridWait limit;
     unsigned phase = 0, rounds = 0;  // word of the next barrier, barriers it has completed
-    __device__ __forceinline__ GridBarrier(unsigned long long *w, GridWait l) : word(w), limit(l) {}
+    __device__ __forceinline__ explicit GridBarrier(unsigned long long *w) : word(w) {}
     // by one thread of the block, after a block barrier
     __device__ __forceinline__ void arrive(bool ask) {
         __threadfence();
@@ -71,10 +68,10 @@ struct GridBarrier {
     }
     // by the same thread: false when the limit is reached
     __device__ __forceinline__ bool wait(unsigned long long &v) const {
-        const unsigned target = (rounds + 1u) * gridDim.x + limit.extra;
-        for (unsigned k = 0; k < limit.polls; k++) {
+        const int target = (int)((rounds + 1u) * gridDim.x);
+        for (unsigned k = 0; k < kGridSpinLimit; k++) {
             asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(word + phase) : "memory");
-            if ((unsigned)v >= target) return true;
+            if ((int)(unsigned)v >= target) return true;
         }
         return false;
     }
@@ -149,8 +146,7 @@ __device__ __forceinline__ int bucket_partners(const SysDev &S, float4 v, const 
 // other T draw the noise of the step after theirs.
 template <bool EXTRA, bool HELP>
 __global__ void __launch_bounds__(kGridMaxOwners, 1)
-    k_list_grid(ListArgs a, ListPersist lp, const long long *ni_base, int nsteps, unsigned long long *bar_word,
-                GridWait limit) {
+    k_list_grid(ListArgs a, ListPersist lp, const long long *ni_base, int nsteps, unsigned long long *bar_word) {
     extern __shared__ __align__(16) unsigned char dsm[];
     __shared__ unsigned long long s_word;
     __shared__ int s_ok;
@@ -202,7 +198,7 @@ __global__ void __launch_bounds__(kGridMaxOwners, 1)
     const float c0 = tm ? S.cut2[1] : S.cut2[0], c1 = tm ? S.cut2[2] : S.cut2[1];
     const bool general = (EXTRA && S.pot != kPotWcaModified) || S.fcap > 0.f;
     const float skin_half2 = S.skin_half2;
-    GridBarrier bar(bar_word, limit);
+    GridBarrier bar(bar_word);
     unsigned asked0 = 0, asked1 = 0;  // askers so far on either word
     // the whole grid waits; true (and the word) unless the limit was reached
     auto grid_wait = [&]() {
