@@ -31,16 +31,16 @@ __device__ __forceinline__ void set_status(unsigned *st, unsigned bits) {
     if (st) atomicOr(st, bits);
 }
 // Status of a call whose word lies in host memory, where an atomic costs 30 ns
-// and a million failing threads took 60 ms: the first thread with a bit, told
-// by a device word per bit that then holds the call's number, sets it there.
+// and a million failing threads took 60 ms: the first thread with a bit, told by
+// a device word per bit, sets it there.  In device memory, so that a kernel takes
+// one pointer (handed over by value it cost every call half a microsecond).
 struct CallStatus {
-    unsigned *word;  // host word
-    unsigned *seen;  // [32] device words
-    unsigned call;
+    unsigned *word;     // host word
+    unsigned seen[30];  // zero between calls
 };
-__device__ __forceinline__ void set_status(const CallStatus &st, unsigned bit) {
-    unsigned *seen = st.seen + (__ffs(bit) - 1);
-    if (*(volatile unsigned *)seen != st.call && atomicExch(seen, st.call) != st.call) atomicOr(st.word, bit);
+__device__ __forceinline__ void set_status(CallStatus *st, unsigned bit) {
+    unsigned *seen = st->seen + (__ffs(bit) - 1);
+    if (*(volatile unsigned *)seen == 0u && atomicExch(seen, 1u) == 0u) atomicOr(st->word, bit);
 }
 
 

@@ -58,7 +58,7 @@ struct CvHits {
     int bins;
     float *H;            // [3][n][bins] (zero), or null: the block adds to ata and atb
     double *ata, *atb;
-    CallStatus st;
+    CallStatus *st;
 };
 // shared memory: tile [3][kCvTile] and masks [warps][kCvMasks][32] (later the
 // rows in FP64, [32][3 bins | 1]), bin sums [warps][32][3 bins | 1] (an odd row
@@ -391,7 +391,7 @@ int bd_cv3d_add_statistics(bd_cv3d *cv, const float *rr, const float *xx, int n,
     if (!w.ok()) return BD_ERR_NOMEM;
     if (!fused) BD_CUDA_TRY(cudaMemsetAsync(d_H, 0, sizeof(float) * 3 * (size_t)n * bins, s));
     k_cv_hits<<<div_up(n, kCvBlock), warps * 32, sm, s>>>({rr, xx, n, side, cv->range, bins, d_H, cv->d_ata, cv->d_atb,
-                                                           w.status()});
+                                                           w.status});
     BD_LAUNCH_CHECK();
     if (!fused) {
         k_cv_normal<<<dim3(tiles, tiles, 3 * splits), dim3(16, 16), 0, s>>>(d_H, xx, n, bins, splits, d_part, cv->d_ata,

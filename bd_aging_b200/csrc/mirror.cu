@@ -54,17 +54,29 @@ namespace {
 constexpr int kSlots = 32;
 struct SlotState {
     std::atomic_flag busy = ATOMIC_FLAG_INIT;
-    unsigned calls = 0;
 };
+struct SlotWords {  // on the device
+    unsigned counter, pad[31];
+    CallStatus status;
+};
+static_assert(sizeof(SlotWords) == 256, "on their own lines");
 struct ContextSlots {
     HostWords *host = nullptr, *dev = nullptr;  // [kSlots] words, 128 bytes apart
-    double *accum = nullptr;                    // [kSlots][kWorkAccum], then the counters
+    double *accum = nullptr;                    // [kSlots][kWorkAccum], then SlotWords [kSlots]
     unsigned long long ctx = 0;                 // context the pointers belong to
     SlotState slot[kSlots];
     ContextSlots *next = nullptr;
 };
 constexpr size_t kWordStride = 128 / sizeof(HostWords);
 static_assert(128 % sizeof(HostWords) == 0, "slots on their own lines");
+
+bool init_slots(void *acc, size_t sums, HostWords *dev) {
+    SlotWords w[kSlots];
+    std::memset(w, 0, sizeof(w));
+    for (int k = 0; k < kSlots; k++) w[k].status.word = &dev[k * kWordStride].status;
+    return cudaMemset(acc, 0, sums) == cudaSuccess &&
+           cudaMemcpy(static_cast<char *>(acc) + sums, w, sizeof(w), cudaMemcpyHostToDevice) == cudaSuccess;
+}
 
 // The current context's slots, made on first use and never changed after: a
 // context's id is its own for the life of the process, so one that was destroyed
@@ -80,10 +92,10 @@ ContextSlots *context_slots() {
     ContextSlots *d = new (std::nothrow) ContextSlots();
     if (!d) return nullptr;
     void *h = nullptr, *p = nullptr, *acc = nullptr;
-    const size_t sums = sizeof(double) * kWorkAccum * kSlots, bytes = sums + 256 * kSlots;
+    const size_t sums = sizeof(double) * kWorkAccum * kSlots, bytes = sums + sizeof(SlotWords) * kSlots;
     if (cudaHostAlloc(&h, 128 * kSlots, cudaHostAllocMapped) != cudaSuccess ||
         cudaHostGetDevicePointer(&p, h, 0) != cudaSuccess || cudaMalloc(&acc, bytes) != cudaSuccess ||
-        cudaMemset(acc, 0, bytes) != cudaSuccess || cudaDeviceSynchronize() != cudaSuccess) {
+        !init_slots(acc, sums, static_cast<HostWords *>(p)) || cudaDeviceSynchronize() != cudaSuccess) {
         if (h) cudaFreeHost(h);
         if (acc) cudaFree(acc);
         delete d;
@@ -113,9 +125,9 @@ CallSlot::CallSlot(cudaStream_t s) : stream(s) {
     host = d->host + k * kWordStride;
     dev = d->dev + k * kWordStride;
     accum = d->accum + (size_t)k * kWorkAccum;
-    counter = reinterpret_cast<unsigned *>(d->accum + (size_t)kSlots * kWorkAccum) + 64 * k;
-    seen = counter + 32;
-    call = ++d->slot[k].calls;
+    SlotWords *w = reinterpret_cast<SlotWords *>(d->accum + (size_t)kSlots * kWorkAccum) + k;
+    counter = &w->counter;
+    status = &w->status;
     host->status = 0;
 }
 cudaError_t CallSlot::wait() {
@@ -125,6 +137,10 @@ cudaError_t CallSlot::wait() {
 CallSlot::~CallSlot() {
     if (!state) return;
     if (!waited) cudaStreamSynchronize(stream);
+    if (*static_cast<volatile unsigned *>(&host->status)) {
+        cudaMemsetAsync(status->seen, 0, sizeof(status->seen), stream);
+        cudaStreamSynchronize(stream);
+    }
     static_cast<SlotState *>(state)->busy.clear(std::memory_order_release);
 }
 
@@ -139,7 +155,7 @@ static int read_status(CallSlot &w) {
 // with the inverse side a double division narrowed to float, ==ncell clamp,
 // linear index i + n(j + n k), slot by atomic increment of nocup.
 __global__ void k_cell_bin(const float *__restrict__ rr, int n, float csi, int ncell, int ntags, int *nocup,
-                           int *cell_vec, const CallStatus st) {
+                           int *cell_vec, CallStatus *st) {
     int m = blockIdx.x * blockDim.x + threadIdx.x;
     if (m >= n) return;
     float x = rr[3 * m], y = rr[3 * m + 1], z = rr[3 * m + 2];
@@ -215,7 +231,7 @@ template <bool SAME, int G, int W>
 __global__ void __launch_bounds__(kForceThreads, 12) k_forces(const float *__restrict__ rr, float *ff, float *vir, float *pot,
                          const float *__restrict__ rr_o, const int *__restrict__ nocup,
                          const int *__restrict__ cell_vec, int n, int ncell, int ntags, int nrange, float csi,
-                         float sigma, float side, const CallStatus st) {
+                         float sigma, float side, CallStatus *st) {
     const int m = (int)(((size_t)blockIdx.x * blockDim.x + threadIdx.x) / G), sub = threadIdx.x % G;
     if (m >= n) return;  // the lanes of a particle leave together
     const float side_inv = __fdiv_rn(1.0f, side);
@@ -313,7 +329,7 @@ static int launch_forces(const float *rr, float *ff, float *vir, float *pot, con
     auto kern = lanes == 32 ? forces_kernel<SAME, 32>(nrange) : lanes == 8 ? forces_kernel<SAME, 8>(nrange)
                                                                           : forces_kernel<SAME, 1>(nrange);
     kern<<<div_up((long)n * lanes, kForceThreads), kForceThreads, 0, s>>>(rr, ff, vir, pot, rr_o, nocup, cell_vec, n, ncell, ntags, nrange, csi,
-                                                      sigma, side, w.status());
+                                                      sigma, side, w.status);
     BD_LAUNCH_CHECK();
     return read_status(w);
 }
@@ -745,7 +761,7 @@ int bd_cell_locate(char type, const float *rr, int *nocup, int *cell_vec, const 
     const bool by_lanes = ntags <= 32 && (long long)nc3 * lanes <= 1 << 20;
     if (!by_lanes) BD_CUDA_TRY(cudaMemsetAsync(cell_vec, 0xff, sizeof(int) * (size_t)nc3 * ntags, s));
     if (n > 0) {
-        k_cell_bin<<<div_up(n, 256), 256, 0, s>>>(rr, n, csi, ncell, ntags, nocup, cell_vec, w.status());
+        k_cell_bin<<<div_up(n, 256), 256, 0, s>>>(rr, n, csi, ncell, ntags, nocup, cell_vec, w.status);
         BD_LAUNCH_CHECK();
     }
     if (by_lanes && lanes == 16) k_cell_sort<16><<<div_up((long)nc3 * 16, 256), 256, 0, s>>>(nocup, cell_vec, nc3, ntags);

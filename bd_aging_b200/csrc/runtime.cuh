@@ -35,8 +35,7 @@ struct CallSlot {
     HostWords *dev = nullptr;      // the same words as kernels see them
     double *accum = nullptr;       // kWorkAccum FP64 partial sums
     unsigned *counter = nullptr;   // finished blocks of a reduction, zero between calls
-    unsigned *seen = nullptr;      // status bits already passed on (CallStatus)
-    unsigned call = 0;             // number of this call among the slot's
+    CallStatus *status = nullptr;  // for the kernels, on the device
     void *state = nullptr;
     cudaStream_t stream;           // of the call's kernels
     bool waited = false;
@@ -46,7 +45,6 @@ struct CallSlot {
     CallSlot(const CallSlot &) = delete;
     CallSlot &operator=(const CallSlot &) = delete;
     bool ok() const { return host != nullptr; }  // false: allocation failed
-    CallStatus status() const { return {&dev->status, seen, call}; }
 };
 
 // Map the device status word to a BD_* code.  A non-finite position also
